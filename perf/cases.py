@@ -130,7 +130,8 @@ def _block(dtype):
     return _blocks[dtype]
 
 
-def prepare(case: dict, seed: int) -> dict:
+def _inputs(case: dict, seed: int) -> dict:
+    """The tensors of a case, from the seed alone."""
     dt = DTYPES[case["dtype"]]
     gen = torch.Generator(device="cuda").manual_seed(seed)
 
@@ -142,15 +143,28 @@ def prepare(case: dict, seed: int) -> dict:
         tokens = case["batch"] * case["seq"]
         resid = normal(tokens, BLOCK[0])
         x = resid.float()
-        return {"kind": kind, "block": _block(dt), "batch": case["batch"], "seq": case["seq"], "resid": resid,
-                "h": (x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + EPS)).to(dt)}
+        return {"resid": resid, "h": (x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + EPS)).to(dt)}
     m, n = case["m"], case["n"]
     if kind == "rmsnorm":
-        return {"kind": kind, "x": normal(m, n), "w": (1 + 0.1 * torch.randn(n, device="cuda", generator=gen)).to(dt)}
+        return {"x": normal(m, n), "w": (1 + 0.1 * torch.randn(n, device="cuda", generator=gen)).to(dt)}
     k = case["k"]
     x = normal(m, k)
     w = normal(n, k, scale=k ** -0.5)
-    g = (1 + 0.1 * torch.randn(n, device="cuda", generator=gen)).to(dt)
+    return {"x": x, "w": w, "g": (1 + 0.1 * torch.randn(n, device="cuda", generator=gen)).to(dt)}
+
+
+def prepare(case: dict, seed: int) -> dict:
+    dt = DTYPES[case["dtype"]]
+    kind = case["kind"]
+    t = _inputs(case, seed)
+    if kind == "block":
+        return {"kind": kind, "block": _block(dt), "batch": case["batch"], "seq": case["seq"], "resid": t["resid"],
+                "h": t["h"]}
+    m, n = case["m"], case["n"]
+    if kind == "rmsnorm":
+        return {"kind": kind, "x": t["x"], "w": t["w"]}
+    k = case["k"]
+    x, w, g = t["x"], t["w"], t["g"]
     if kind in ("all_reduce", "reduce_scatter"):
         layer = FusedRowParallelLinear(_shared_impl(), k, n, comm_op=kind, norm=case["norm"], eps=EPS,
                                        algo=case["algo"], dtype=dt)
@@ -192,6 +206,37 @@ def run(s: dict):
     if kind == "gemm":
         return ops.gemm(s["impl"], s["x"], s["w"], s["algo"])
     return s["block"](s["h"], s["resid"], s["batch"], s["seq"])
+
+
+def _norm64(x, w):
+    return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + EPS) * w.double()
+
+
+def exact(case: dict, seed: int):
+    """What ``run`` returns, in 64 bits with torch's own operations."""
+    t = _inputs(case, seed)
+    kind = case["kind"]
+    if kind == "rmsnorm":
+        return _norm64(t["x"].double(), t["w"])
+    if kind != "block":
+        y = t["x"].double() @ t["w"].double().t()
+        return _norm64(y, t["g"]) if case["norm"] else y
+    hidden, ffn, heads, kv = BLOCK
+    batch, seq, hd = case["batch"], case["seq"], hidden // heads
+    p = _block(DTYPES[case["dtype"]])  # for its weights
+    qkv = t["h"].double() @ p.w_qkv.double().t()
+    q, k, v = (z.reshape(batch, seq, -1, hd) for z in qkv.split([hidden, kv * hd, kv * hd], dim=-1))
+    hide = torch.ones(seq, seq, dtype=torch.bool, device="cuda").triu(1)
+    attn = torch.empty(batch, seq, heads, hd, dtype=torch.float64, device="cuda")
+    for b in range(batch):
+        for h in range(heads):
+            kh, vh = k[b, :, h * kv // heads], v[b, :, h * kv // heads]
+            scores = (q[b, :, h] @ kh.t() / math.sqrt(hd)).masked_fill(hide, -math.inf)
+            attn[b, :, h] = scores.softmax(-1) @ vh
+    h2 = t["resid"].double() + attn.reshape(batch * seq, hidden) @ p.w_o.double().t()
+    gate, up = (_norm64(h2, p.norm_attn) @ p.w_gate_up.double().t()).chunk(2, dim=-1)
+    h3 = h2 + (torch.nn.functional.silu(gate) * up) @ p.w_down.double().t()
+    return _norm64(h3, p.norm_next) @ p.w_qkv_next.double().t(), h3
 
 
 def work(case: dict) -> dict:
