@@ -98,7 +98,8 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
     return cudaErrorInvalidValue;
   }
   // every CTA stages 128 rows of A and (for a CTA pair) half of the B tile, 64 K-values per box
-  if (!make_tensor_map(&p.tmA, g.A, g.M, g.K, 128, g.dtype) ||
+  const int a_rows = g.a_rows > 0 && g.a_rows < g.M ? g.a_rows : g.M;  // the copy engine fills the rows after them with zero
+  if (!make_tensor_map(&p.tmA, g.A, a_rows, g.K, 128, g.dtype) ||
       !make_tensor_map(&p.tmB, g.B, g.N, g.K, tc.bn / tc.ctas, g.dtype)) {
     *why = "cuTensorMapEncodeTiled failed";
     return cudaErrorInvalidValue;

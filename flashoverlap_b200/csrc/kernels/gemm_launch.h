@@ -33,6 +33,9 @@ struct GemmOperands {
   // ([own_rows, K] row-major, 16-byte aligned) instead of from A.
   const void* A_own;
   int own_begin, own_rows;
+  // Rows that A really holds when that is less than M (M is a multiple of the
+  // tile height); the rows after them read as zero.  0 = A holds M rows.
+  int a_rows;
 };
 
 // Fills p.tmA / p.tmB / shape fields from `g`, validates shapes, launches.

@@ -496,11 +496,15 @@ void FusedEngine::a2a_gemm(const void* A_send, const void* B, void* C, const int
     if (mlen[i] < 0) throw std::runtime_error("a2a_gemm: negative row count");
   }
   const int m_pad = a2a_padded_rows(mlen, algo);  // the same on every rank
-  if (world_ == 1 && mlen[0] == m_pad && reinterpret_cast<uintptr_t>(A_send) % 16 == 0) {  // one rank, whole tiles: in place
+  // One rank: the GEMM reads the caller's rows where they are, also when they do not fill the last tile (its
+  // missing rows read as zero, and the scratch rows of C become zero).  Copying them through the gathered
+  // buffer costs a pass over A that the first tiles wait for.
+  if (world_ == 1 && mlen[0] > 0 && reinterpret_cast<uintptr_t>(A_send) % 16 == 0) {
     GemmOperands g{};
     g.A = A_send;
     g.B = B;
     g.M = m_pad;
+    g.a_rows = mlen[0];
     g.N = N;
     g.K = K;
     g.dtype = dtype;

@@ -295,6 +295,24 @@ def test_a2a_dispatch_gemm_world1():
     assert (C.float() - ref2).abs().max().item() <= 1e-2 * ref2.abs().max().item()
 
 
+@pytest.mark.parametrize("rows", [1, 127, 129, 255, 257])
+@pytest.mark.parametrize("algo", [0, 8])
+def test_a2a_dispatch_gemm_ragged_rows_in_place(rows, algo):
+    # rows that end inside the last tile: read where they are, the rest of the tile counts as zero
+    K, N = 136, 512
+    impl = make_impl()
+    mlen = torch.tensor([[rows]], dtype=torch.int32)
+    A, B, _ = make_inputs(rows, N, K, torch.float16, seed=rows)
+    C = torch.full((impl.a2a_padded_rows(mlen, algo), N), float("nan"), device="cuda", dtype=torch.float16)
+    impl.a2a_dispatch_gemm(A, B, C, mlen, algo)
+    torch.cuda.synchronize()
+    impl.check_status()
+    ref = A.double() @ B.double().t()
+    # one rounding to 11 bits and fp32 sums of 136 products
+    assert (C[:rows].double() - ref).abs().max().item() <= 2 ** -10 * ref.abs().max().item()
+    assert bool((C[rows:] == 0).all())
+
+
 def test_host_feeder_double_buffers_inputs():
     from flashoverlap_b200.utils.pipeline import HostFeeder
 
