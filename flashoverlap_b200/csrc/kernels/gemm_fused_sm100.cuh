@@ -838,6 +838,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       ptx::tc_fence_after_sync();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
       const int row0 = m_blk * TILE_M + static_cast<int>(cta_rank) * BM + q * 32;  // first global row of this warp's slab
+      const int chunk = lane & 7;  // of a 128-byte row segment; eight lanes write one
+      // A slab that stays on this GPU is a plain pitched block, in the natural layout and in the tiled one
+      // (its 32 rows lie in one tile row, its 64 columns in one tile): the address is found once per step at most.
+      const bool local = p.own_mode == OWN_SINGLE || p.nvls;
+      const OutLayout& L = p.epi_layout;
+      const bool pitched = local && (!L.tiled || (L.row_map == nullptr && L.bm % 32 == 0 && L.bn % 64 == 0));
+      const long long pitch = L.tiled ? static_cast<long long>(L.rldn) * L.bn : L.ld;
+      uint16_t* slab_dst = nullptr;
+      if (pitched) {
+        slab_dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(L, row0, n_blk * BN) +
+                   (lane >> 3) * pitch + chunk * 8;
+      }
 
 #pragma unroll 1
       for (int cc = 0; cc < BN / 64; ++cc) {
@@ -875,16 +887,24 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         }
         __syncwarp();
         // smem slab -> global: 8 lanes cover one 128-byte row segment
-        const int chunk = lane & 7;
         const int col = n_blk * BN + cc * 64 + chunk * 8;
+        uint16_t* step_dst = slab_dst + cc * 64;
+        if (pitched && L.tiled) {
+          step_dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(L, row0, col - chunk * 8) +
+                     (lane >> 3) * pitch + chunk * 8;
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int r = i * 4 + (lane >> 3);
           const uint4 v = ptx::ld_shared_v4(slab + r * 128 + ((chunk ^ (r & 7)) << 4));
+          if (pitched) {
+            ptx::st_v4(step_dst + i * 4 * pitch, v);
+            continue;
+          }
           const int g = row0 + r;
           uint16_t* dst;
-          if (p.own_mode == OWN_SINGLE || p.nvls) {
-            dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(p.epi_layout, g, col);
+          if (local) {
+            dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(L, g, col);
           } else if (p.own_mode == OWN_BLOCK) {
             const int o = g / p.rows_per_owner;
             const int lr = g - o * p.rows_per_owner;

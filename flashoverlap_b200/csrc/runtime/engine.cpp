@@ -230,6 +230,18 @@ void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* ou
   check_launch(launch_fused(g, p, stream, &why), why, "gemm_rmsnorm");
 }
 
+namespace {
+// Does the result at `out` share memory with an operand that the GEMM still reads while it writes tiles?
+bool overlaps_operand(const GemmOperands& g, const void* out) {
+  auto meets = [](const void* a, size_t na, const void* b, size_t nb) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb && y < x + na;
+  };
+  const size_t n = static_cast<size_t>(g.M) * g.N * 2, k = static_cast<size_t>(g.K) * 2;
+  return meets(out, n, g.A, k * g.M) || meets(out, n, g.B, k * g.N);
+}
+}  // namespace
+
 void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, const NormArgs& norm,
                                   const OutLayout* out_layout, const SignalArgs* sig, cudaStream_t stream) {
   NvtxRange range("flashoverlap::gemm_allreduce");
@@ -243,11 +255,11 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
   ensure_workspace(g.M, g.N);
   const int set = static_cast<int>(calls_ & 1ull);
   check(cudaMemsetAsync(flag_ptr(rank_, set ^ 1), 0, kFlagWords * 4, stream), "cudaMemsetAsync(counters)");
-  if (world_ == 1 && norm.gamma == nullptr && sig == nullptr && out_layout == nullptr) {
-    // One rank and no RMSNorm: nothing to sum or scale, the GEMM writes the result itself.  The buffer
-    // sets still alternate (and the other set's counters are cleared above) like after any fused call.
+  if (world_ == 1 && norm.gamma == nullptr && !(out_user != nullptr && overlaps_operand(g, out_user))) {
+    // One rank and no RMSNorm: nothing to sum or scale, the GEMM writes the result itself, in either layout.
+    // The buffer sets still alternate (and the other set's counters are cleared above) like after any fused call.
     void* result = out_user != nullptr ? out_user : heap_.local(ws_.result[set]);
-    gemm(g, result, nullptr, nullptr, stream);
+    gemm(g, result, out_layout, sig, stream);
     ++calls_;
     return result;
   }
@@ -319,8 +331,8 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
   ensure_workspace(g.M, g.N);
   const int set = static_cast<int>(calls_ & 1ull);
   check(cudaMemsetAsync(flag_ptr(rank_, set ^ 1), 0, kFlagWords * 4, stream), "cudaMemsetAsync(counters)");
-  if (world_ == 1 && norm.gamma == nullptr && sig == nullptr && out_layout == nullptr) {
-    gemm(g, D, nullptr, nullptr, stream);  // one rank, no RMSNorm: the GEMM writes the rows where they belong
+  if (world_ == 1 && norm.gamma == nullptr) {
+    gemm(g, D, out_layout, sig, stream);  // one rank, no RMSNorm: the GEMM writes the rows where they belong
     ++calls_;
     return;
   }

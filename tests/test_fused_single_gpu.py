@@ -188,6 +188,34 @@ def test_compat_overlap_api_reordered_layout_and_trace():
     assert (out.float() - want).abs().max().item() <= 1e-2 * want.abs().max().item()
 
 
+@pytest.mark.parametrize("algo,rldn", [(2, 1), (4, 2), (8, 1), (9, 4)])
+@pytest.mark.parametrize("monitor", [False, True])
+def test_compat_overlap_writes_tile_order_in_place(algo, rldn, monitor):
+    # one rank: the epilogue stores the tile-ordered result itself; tiles of every width, wide view rows, and a result
+    # that takes the place of an operand (which then goes through the staging buffer)
+    impl = make_impl()
+    bm, bn, _ = impl.algo_tile(algo)
+    M, N, K = 4 * bm, 8 * bn, 8 * bn
+    A, B, _ = make_inputs(M, N, K, torch.bfloat16, seed=algo)
+    RA = reorder_indices(32, [(11 * i + 5) % 32 for i in range(32)], device="cuda").reshape(4, 8)
+    cseg = torch.tensor([20, 12], dtype=torch.int32)
+    MM = torch.zeros((5, 8), dtype=torch.int32, device="cuda")
+    C = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    impl.gemm_allreduce_overlap(A, B, C, MM, RA, rldn, cseg, cseg.cuda(), algo, monitor)
+    ref = A.double() @ B.double().t()
+    want = to_tile_order(ref.to(torch.bfloat16), bm, bn, RA, rldn)
+    torch.cuda.synchronize()
+    impl.check_status()
+    # one rounding to 8 bits
+    assert (C.double() - want.double()).abs().max().item() <= 2 ** -7 * ref.abs().max().item()
+    A2 = A.clone()
+    MM.zero_()
+    impl.gemm_allreduce_overlap(A2, B, A2, MM, RA, rldn, cseg, cseg.cuda(), algo, False)
+    torch.cuda.synchronize()
+    impl.check_status()
+    assert torch.equal(A2, C)
+
+
 def test_index_arrays_are_checked_on_the_host_before_any_launch():
     M, N, K, algo = 256, 512, 64, 0
     A, B, W = make_inputs(M, N, K, torch.float16)
