@@ -1,11 +1,10 @@
 // RMSNorm and reorder+RMSNorm for 16-bit rows with fp32 statistics.
 //
-// One CTA of 256 threads per row; each thread owns 16-byte chunks
-// (8 values) at stride 256 chunks.  Rows of up to 16384 values are held in
-// registers between the statistics pass and the scaling pass; longer rows are
-// read twice.  Unlike the reference kernels (reference: src/rmsnorm/rmsnorm.cuh:12-115,
-// block size dim/16, eps fixed to 1e-5, default stream) any dim % 8 == 0 works,
-// eps is an argument and the launch goes to the caller's stream.
+// One CTA works on one row at a time and walks several rows; a thread owns the same one, two or four 16-byte chunks
+// (8 values each) of every row, so that the weights can stay in registers, and the next row is on its way from memory
+// while the current one is reduced, scaled and stored (one barrier per row).  Rows of more than 32768 values are read
+// twice.  Unlike the reference kernels (reference: src/rmsnorm/rmsnorm.cuh:12-115, block size dim/16, eps fixed to
+// 1e-5, default stream) any dim % 8 == 0 works, eps is an argument and the launch goes to the caller's stream.
 #include "rmsnorm.h"
 
 #include "gemm_fused_sm100.cuh"
@@ -14,95 +13,131 @@ namespace fo {
 
 namespace {
 
-constexpr int kNormThreads = 256;
-constexpr int kNormRegChunks = 8;
+constexpr int kMaxNormThreads = 1024;
 
-template <bool BF16, bool REORDER>
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const uint16_t* __restrict__ x,
-                                                               uint16_t* __restrict__ out,
-                                                               const uint16_t* __restrict__ w, int rows, int dim,
-                                                               float eps, OutLayout L) {
-  __shared__ float red[kNormThreads / 32];
-  const int row = blockIdx.x;
-  if (row >= rows) return;
+template <bool BF16, bool REORDER, int CPT>
+__global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t* x, uint16_t* out,
+                                                                  const uint16_t* __restrict__ w, int rows, int dim,
+                                                                  float eps, OutLayout L) {
+  __shared__ float red[2][kMaxNormThreads / 32];
   const int n_chunks = dim >> 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool in_regs = n_chunks <= kNormRegChunks * kNormThreads;
+  const int warps = blockDim.x >> 5;
 
-  auto src_ptr = [&](int c) -> const uint16_t* {
-    if constexpr (REORDER) return x + layout_offset(L, row, c * 8);
-    else return x + static_cast<long long>(row) * dim + c * 8;
+  auto load = [&](int row, uint4 (&v)[CPT]) {
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      // a chunk past the end of the row is clamped and its value dropped: the loads stay unconditional and go out together
+      const int c = min(static_cast<int>(threadIdx.x + k * blockDim.x), n_chunks - 1);
+      const uint16_t* src;
+      if constexpr (REORDER) src = x + layout_offset(L, row, c * 8);
+      else src = x + static_cast<long long>(row) * dim + c * 8;
+      v[k] = *reinterpret_cast<const uint4*>(src);
+    }
   };
 
-  uint4 v[kNormRegChunks];
-  float ssq = 0.f;
-  if (in_regs) {
+  constexpr bool KEEP = CPT <= 2;  // room for the weights beside two rows; four chunks read them from L1 for each row
+  const uint4* weights = reinterpret_cast<const uint4*>(w);
+  uint4 v[CPT], g[KEEP ? CPT : 1];
+  int row = blockIdx.x;
+  load(row, v);
+  if constexpr (KEEP) {
 #pragma unroll
-    for (int k = 0; k < kNormRegChunks; ++k) {
-      const int c = threadIdx.x + k * kNormThreads;
-      if (c < n_chunks) v[k] = *reinterpret_cast<const uint4*>(src_ptr(c));
-    }
-#pragma unroll
-    for (int k = 0; k < kNormRegChunks; ++k) {
-      const int c = threadIdx.x + k * kNormThreads;
-      if (c < n_chunks) {
-        float2 f;
-        f = unpack2<BF16>(v[k].x); ssq += f.x * f.x + f.y * f.y;
-        f = unpack2<BF16>(v[k].y); ssq += f.x * f.x + f.y * f.y;
-        f = unpack2<BF16>(v[k].z); ssq += f.x * f.x + f.y * f.y;
-        f = unpack2<BF16>(v[k].w); ssq += f.x * f.x + f.y * f.y;
-      }
-    }
-  } else {
-    for (int c = threadIdx.x; c < n_chunks; c += kNormThreads) {
-      const uint4 u = *reinterpret_cast<const uint4*>(src_ptr(c));
-      float2 f;
-      f = unpack2<BF16>(u.x); ssq += f.x * f.x + f.y * f.y;
-      f = unpack2<BF16>(u.y); ssq += f.x * f.x + f.y * f.y;
-      f = unpack2<BF16>(u.z); ssq += f.x * f.x + f.y * f.y;
-      f = unpack2<BF16>(u.w); ssq += f.x * f.x + f.y * f.y;
-    }
+    for (int k = 0; k < CPT; ++k) g[k] = __ldg(weights + min(static_cast<int>(threadIdx.x + k * blockDim.x), n_chunks - 1));
   }
+  for (int par = 0; row < rows; par ^= 1) {
+    float ssq = 0.f;
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      ssq += static_cast<int>(threadIdx.x + k * blockDim.x) < n_chunks ? sum_squares<BF16>(v[k]) : 0.f;
+    }
+    const int next = row + gridDim.x;
+    uint4 nv[CPT];
+    if (next < rows) load(next, nv);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+    if (warps > 1) {
+      if (lane == 0) red[par][warp] = ssq;  // two sets alternate: one barrier per row is enough
+      __syncthreads();
+      ssq = lane < warps ? red[par][lane] : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+    }
+    const float rstd = rsqrtf(ssq / static_cast<float>(dim) + eps);
+    uint4* dst = reinterpret_cast<uint4*>(out + static_cast<long long>(row) * dim);
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      const int c = threadIdx.x + k * blockDim.x;
+      if (c < n_chunks) dst[c] = scale_chunk<BF16>(v[k], rstd, KEEP ? g[KEEP ? k : 0] : __ldg(weights + c));
+    }
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) v[k] = nv[k];
+    row = next;
+  }
+}
+
+// Rows wider than the registers of a CTA hold: one CTA per row, read twice.
+template <bool BF16, bool REORDER>
+__global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_wide_kernel(const uint16_t* x, uint16_t* out,
+                                                                       const uint16_t* __restrict__ w, int dim,
+                                                                       float eps, OutLayout L) {
+  __shared__ float red[kMaxNormThreads / 32];
+  const int row = blockIdx.x;
+  const int n_chunks = dim >> 3;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long row_off = static_cast<long long>(row) * dim;
+  auto src_ptr = [&](int c) -> const uint4* {
+    if constexpr (REORDER) return reinterpret_cast<const uint4*>(x + layout_offset(L, row, c * 8));
+    else return reinterpret_cast<const uint4*>(x + row_off) + c;
+  };
+  float ssq = 0.f;
+  for (int c = threadIdx.x; c < n_chunks; c += kMaxNormThreads) ssq += sum_squares<BF16>(*src_ptr(c));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
   if (lane == 0) red[warp] = ssq;
   __syncthreads();
-  float tot = 0.f;
+  ssq = red[lane];
 #pragma unroll
-  for (int i = 0; i < kNormThreads / 32; ++i) tot += red[i];
-  const float rstd = rsqrtf(tot / static_cast<float>(dim) + eps);
-
-  auto emit = [&](int c, const uint4& u) {
-    const uint4 g = *reinterpret_cast<const uint4*>(w + c * 8);
-    float2 f;
-    uint4 o;
-    f = unpack2<BF16>(u.x); o.x = norm_pack2<BF16>(f.x, f.y, rstd, g.x);
-    f = unpack2<BF16>(u.y); o.y = norm_pack2<BF16>(f.x, f.y, rstd, g.y);
-    f = unpack2<BF16>(u.z); o.z = norm_pack2<BF16>(f.x, f.y, rstd, g.z);
-    f = unpack2<BF16>(u.w); o.w = norm_pack2<BF16>(f.x, f.y, rstd, g.w);
-    *reinterpret_cast<uint4*>(out + static_cast<long long>(row) * dim + c * 8) = o;
-  };
-  if (in_regs) {
-#pragma unroll
-    for (int k = 0; k < kNormRegChunks; ++k) {
-      const int c = threadIdx.x + k * kNormThreads;
-      if (c < n_chunks) emit(c, v[k]);
-    }
-  } else {
-    for (int c = threadIdx.x; c < n_chunks; c += kNormThreads) emit(c, *reinterpret_cast<const uint4*>(src_ptr(c)));
+  for (int o = 16; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+  const float rstd = rsqrtf(ssq / static_cast<float>(dim) + eps);
+  uint4* dst = reinterpret_cast<uint4*>(out + row_off);
+  for (int c = threadIdx.x; c < n_chunks; c += kMaxNormThreads) {
+    dst[c] = scale_chunk<BF16>(*src_ptr(c), rstd, __ldg(reinterpret_cast<const uint4*>(w) + c));
   }
+}
+
+template <bool BF16, bool REORDER>
+cudaError_t launch_typed(const uint16_t* x, uint16_t* out, const uint16_t* w, int rows, int dim, float eps,
+                         const OutLayout& L, cudaStream_t stream) {
+  const int n_chunks = dim >> 3;
+  if (n_chunks > 4 * kMaxNormThreads) {
+    rmsnorm_wide_kernel<BF16, REORDER><<<rows, kMaxNormThreads, 0, stream>>>(x, out, w, dim, eps, L);
+    return cudaGetLastError();
+  }
+  const int sms = device_sm_count();
+  // Few rows: as many threads per row as it has chunks, since only the latency of one row counts.  Many rows: two
+  // chunks per thread, which leaves fewer warps to wait at the row's barrier.
+  int cpt = rows <= 2 * sms || n_chunks <= 32 ? 1 : 2;
+  while (n_chunks > cpt * kMaxNormThreads) cpt *= 2;
+  const int threads = ((n_chunks + cpt - 1) / cpt + 31) / 32 * 32;
+  // 64 registers a thread: the CTAs that are resident together
+  int per_sm = kMaxNormThreads / threads;
+  if (per_sm > 32) per_sm = 32;
+  const int grid = rows < sms * per_sm ? rows : sms * per_sm;
+  auto kernel = cpt == 1   ? rmsnorm_kernel<BF16, REORDER, 1>
+                : cpt == 2 ? rmsnorm_kernel<BF16, REORDER, 2>
+                           : rmsnorm_kernel<BF16, REORDER, 4>;
+  kernel<<<grid, threads, 0, stream>>>(x, out, w, rows, dim, eps, L);
+  return cudaGetLastError();
 }
 
 template <bool REORDER>
 cudaError_t launch(const void* x, void* out, const void* w, int rows, int dim, float eps, const OutLayout& L, DType dt,
                    cudaStream_t stream) {
   if (rows <= 0 || dim <= 0 || dim % 8 != 0) return cudaErrorInvalidValue;
-  auto xs = reinterpret_cast<const uint16_t*>(x);
-  auto os = reinterpret_cast<uint16_t*>(out);
-  auto ws = reinterpret_cast<const uint16_t*>(w);
-  if (dt == DT_BF16) rmsnorm_kernel<true, REORDER><<<rows, kNormThreads, 0, stream>>>(xs, os, ws, rows, dim, eps, L);
-  else rmsnorm_kernel<false, REORDER><<<rows, kNormThreads, 0, stream>>>(xs, os, ws, rows, dim, eps, L);
-  return cudaGetLastError();
+  auto typed = dt == DT_BF16 ? launch_typed<true, REORDER> : launch_typed<false, REORDER>;
+  return typed(static_cast<const uint16_t*>(x), static_cast<uint16_t*>(out), static_cast<const uint16_t*>(w), rows, dim,
+               eps, L, stream);
 }
 
 }  // namespace

@@ -267,6 +267,23 @@ def test_rmsnorm_op(dtype, dim):
     assert (o.float() - want).abs().max().item() <= tol * want.abs().max().item()
 
 
+@pytest.mark.parametrize("rows", [1, 296, 297, 2500])
+@pytest.mark.parametrize("dim", [8, 256, 264, 8192, 8200, 16384, 16392, 32768, 32776])
+def test_rmsnorm_thread_shapes(rows, dim):
+    # one, two or four chunks per thread, a partly filled last warp, several rows per CTA, rows read twice; in place too
+    torch.manual_seed(dim + rows)
+    x = torch.randn(rows, dim, device="cuda", dtype=torch.float16)
+    w = (1 + 0.1 * torch.randn(dim, device="cuda")).half()
+    o = torch.full_like(x, float("nan"))
+    torch.ops.flashoverlap_op.rmsnorm(x, o, w, 1e-6)
+    xd = x.double()
+    want = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    # two roundings to 11 bits each
+    assert ((o.double() - want).abs() <= 2 ** -9.9 * want.abs() + 1e-7).all()
+    torch.ops.flashoverlap_op.rmsnorm(x, x, w, 1e-6)
+    assert torch.equal(x, o)
+
+
 def test_reorder_rmsnorm_rldn2():
     M, N, bm, bn = 512, 1024, 128, 256
     tm, tn = M // bm, N // bn
