@@ -147,6 +147,30 @@ __device__ __forceinline__ uint32_t norm_pack2(float a, float b, float rstd, uin
   }
 }
 
+// Sum of the squares of eight 16-bit values.
+template <bool BF16>
+__device__ __forceinline__ float sum_squares(const uint4& h) {
+  float2 f;
+  float r;
+  f = unpack2<BF16>(h.x); r = f.x * f.x + f.y * f.y;
+  f = unpack2<BF16>(h.y); r += f.x * f.x + f.y * f.y;
+  f = unpack2<BF16>(h.z); r += f.x * f.x + f.y * f.y;
+  f = unpack2<BF16>(h.w); r += f.x * f.x + f.y * f.y;
+  return r;
+}
+
+// Eight values scaled by rstd and the RMSNorm weights.
+template <bool BF16>
+__device__ __forceinline__ uint4 scale_chunk(const uint4& h, float rstd, const uint4& w) {
+  float2 f;
+  uint4 o;
+  f = unpack2<BF16>(h.x); o.x = norm_pack2<BF16>(f.x, f.y, rstd, w.x);
+  f = unpack2<BF16>(h.y); o.y = norm_pack2<BF16>(f.x, f.y, rstd, w.y);
+  f = unpack2<BF16>(h.z); o.z = norm_pack2<BF16>(f.x, f.y, rstd, w.z);
+  f = unpack2<BF16>(h.w); o.w = norm_pack2<BF16>(f.x, f.y, rstd, w.w);
+  return o;
+}
+
 // ---------------------------------------------------------------------------
 // reduce phase: groups of kGroupWarps warps, one owned row at a time
 // ---------------------------------------------------------------------------
@@ -246,24 +270,6 @@ __device__ __forceinline__ void comm_worker(const FusedParams& p, GroupScratch* 
       h.w = pack2<BF16>(a[6], a[7]);
       return h;
     }
-  };
-  auto sq = [&](const uint4& h) -> float {
-    float2 f;
-    float r;
-    f = unpack2<BF16>(h.x); r = f.x * f.x + f.y * f.y;
-    f = unpack2<BF16>(h.y); r += f.x * f.x + f.y * f.y;
-    f = unpack2<BF16>(h.z); r += f.x * f.x + f.y * f.y;
-    f = unpack2<BF16>(h.w); r += f.x * f.x + f.y * f.y;
-    return r;
-  };
-  auto scale = [&](const uint4& h, float rstd, const uint4& w) -> uint4 {
-    float2 f;
-    uint4 o;
-    f = unpack2<BF16>(h.x); o.x = norm_pack2<BF16>(f.x, f.y, rstd, w.x);
-    f = unpack2<BF16>(h.y); o.y = norm_pack2<BF16>(f.x, f.y, rstd, w.y);
-    f = unpack2<BF16>(h.z); o.z = norm_pack2<BF16>(f.x, f.y, rstd, w.z);
-    f = unpack2<BF16>(h.w); o.w = norm_pack2<BF16>(f.x, f.y, rstd, w.w);
-    return o;
   };
   // where owned row lr lives: global row, 128-row block, partial rows, output row
   auto global_row = [&](int lr) -> int {
@@ -378,7 +384,7 @@ __device__ __forceinline__ void comm_worker(const FusedParams& p, GroupScratch* 
           const int c = u * GT + tid;
           if (c < n_chunks) {
             h[u] = load_sum_generic(src0, c);
-            if (p.norm) ssq += sq(h[u]);
+            if (p.norm) ssq += sum_squares<BF16>(h[u]);
             else store_out(out_row, c, h[u]);
           }
         }
@@ -401,7 +407,7 @@ __device__ __forceinline__ void comm_worker(const FusedParams& p, GroupScratch* 
 #pragma unroll
         for (int u = 0; u < CPT; ++u) {
           const int c = u * GT + tid;
-          if (p.norm) ssq += c < n_chunks ? sq(h[u]) : 0.f;
+          if (p.norm) ssq += c < n_chunks ? sum_squares<BF16>(h[u]) : 0.f;
           else if (c < n_chunks) store_out(out_row, c, h[u]);
         }
       } else {
@@ -429,7 +435,7 @@ __device__ __forceinline__ void comm_worker(const FusedParams& p, GroupScratch* 
           for (int u = 0; u < BATCH; ++u) {
             const int c = (k * BATCH + u) * GT + tid;
             h[k * BATCH + u] = sum_sources(buf[k & 1][u]);
-            if (p.norm) ssq += c < n_chunks ? sq(h[k * BATCH + u]) : 0.f;
+            if (p.norm) ssq += c < n_chunks ? sum_squares<BF16>(h[k * BATCH + u]) : 0.f;
             else if (c < n_chunks) store_out(out_row, c, h[k * BATCH + u]);
           }
         }
@@ -446,7 +452,7 @@ __device__ __forceinline__ void comm_worker(const FusedParams& p, GroupScratch* 
           hv = sum_sources(v);
         }
         if (p.norm) {
-          ssq += sq(hv);
+          ssq += sum_squares<BF16>(hv);
           ptx::st_v4(park + layout_offset(p.out_layout, out_row, c * 8), hv);
         } else {
           store_out(out_row, c, hv);
@@ -498,14 +504,14 @@ __device__ __forceinline__ void comm_worker(const FusedParams& p, GroupScratch* 
         for (int u = 0; u < CPT; ++u) {
           const int c = u * GT + tid;
           if (c < n_chunks) {
-            store_out(out_row, c, scale(h[u], rstd, ptx::ld_shared_v4(gamma_smem + (static_cast<uint32_t>(c) << 4))));
+            store_out(out_row, c, scale_chunk<BF16>(h[u], rstd, ptx::ld_shared_v4(gamma_smem + (static_cast<uint32_t>(c) << 4))));
           }
         }
       } else {
         for (int c = tid; c < n_chunks; c += GT) {  // every thread re-reads exactly the chunks it wrote
           const uint4 hv = ptx::ld_cg_v4(park + layout_offset(p.out_layout, out_row, c * 8));
           const uint4 wv = __ldg(gamma + c);
-          store_out(out_row, c, scale(hv, rstd, wv));
+          store_out(out_row, c, scale_chunk<BF16>(hv, rstd, wv));
         }
       }
     }
