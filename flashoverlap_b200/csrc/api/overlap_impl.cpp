@@ -609,7 +609,8 @@ void OverlapImpl::GemmRmsNorm(at::Tensor A, at::Tensor B, at::Tensor C, at::Tens
   NormArgs norm;
   norm.gamma = weight.data_ptr();
   norm.eps = static_cast<float>(eps);
-  engine_.gemm_rmsnorm(g, C.data_ptr(), O.data_ptr(), norm, current_stream());
+  at::Tensor ssq = torch::empty({A.size(0) * (B.size(0) / 64)}, A.options().dtype(at::kFloat));
+  engine_.gemm_rmsnorm(g, C.data_ptr(), O.data_ptr(), ssq.data_ptr<float>(), norm, current_stream());
 }
 
 void OverlapImpl::AttachSymmetric(std::vector<int64_t> peer_ptrs, int64_t mc_ptr, int64_t nbytes) {

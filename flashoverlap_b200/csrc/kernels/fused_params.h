@@ -151,7 +151,13 @@ struct alignas(64) FusedParams {
 
   // ---- reduce phase ---------------------------------------------------------
   int reduce;                      // 0 = kernel ends after the GEMM
-  uint32_t* job_counter;           // next owned row to reduce (zero at launch); rows are claimed in order
+  uint32_t* job_counter;           // next owned row (or unit, see ssq) to reduce (zero at launch); claimed in order
+  // One rank and RMSNorm: sums of squares of the rounded values, one per tile column and row,
+  // [M / 128][TN][128], written by the epilogue.  The reduce phase then scales rows without a pass of its own
+  // over them (norm_stream).  Null = the row workers find the sums.
+  float* ssq;
+  // Counter set of the next call, zeroed by this launch (one rank: nobody else raises it).  Null = the host clears it.
+  uint32_t* clear_words;
   const void* stage;               // this GPU's staging: [ws][rows_per_owner][N]
   uint32_t flag_target;            // value every arrival counter must reach
   int norm;                        // apply RMSNorm after the sum

@@ -552,6 +552,129 @@ __device__ __forceinline__ void comm_worker(const FusedParams& p, GroupScratch* 
   }
 }
 
+// Reduce phase of one rank with RMSNorm.  Nothing has to be summed over ranks and the epilogue has left the sums of
+// squares (p.ssq), so a row needs no pass for its statistics: the rest is a copy that scales.  A unit is 8 rows x 512
+// columns; a row group claims one per warp, in the order in which tile rows complete, and one thread of it looks at the
+// arrival counter (every warp of every CTA polling the same few words held up the arrivals themselves: the last rows of a
+// 128-row call left 8 us after the last tile).  The 16 loads of a lane go out back to back, together with those of the row
+// statistics.
+template <bool BF16>
+__device__ __forceinline__ void norm_stream(const FusedParams& p, GroupScratch* gs, uint32_t gamma_smem, int group, int wg,
+                                            int lane, uint64_t deadline, volatile uint32_t* abort_flag) {
+  constexpr int ROWS = 8;
+  constexpr int CHUNKS = 64;      // 16-byte chunks per row of a unit, two per lane
+  constexpr int STATS = 16;       // statistics loads a lane has in flight
+  const int n_chunks = p.N >> 3;
+  const int col_units = (n_chunks + CHUNKS - 1) / CHUNKS;
+  const int units = p.M / ROWS * col_units;
+  const bool gamma_here = p.N <= kGammaSmemValues;
+  const uint4* gamma = reinterpret_cast<const uint4*>(p.gamma);
+  const uint32_t* my_flag = p.flag[0];
+  const bool leader = wg == 0 && lane == 0;
+  unsigned long long t_first = 0, t_last = 0;
+  uint32_t rows_done = 0;
+  int ready_rb = -1;  // leader: last 128-row block seen complete
+  uint32_t claimed = 0;
+  if (leader) claimed = atomicAdd(p.job_counter, static_cast<uint32_t>(kGroupWarps));
+  for (int it = 0;; ++it) {
+    unsigned long long t_claim = 0;
+    if (leader) {
+      t_claim = p.row_trace != nullptr ? ptx::globaltimer_ns() : 0ull;
+      uint32_t first = claimed;
+      if (first < static_cast<uint32_t>(units)) {
+        // the blocks of all claimed units
+        const int last = min(static_cast<int>(first) + kGroupWarps, units) - 1;
+        const int rb_last = last / col_units * ROWS / 128;
+        for (int rb = max(static_cast<int>(first) / col_units * ROWS / 128, ready_rb + 1); rb <= rb_last; ++rb) {
+          uint32_t seen = 0;
+          if (!ptx::wait_counter_relaxed_gpu(my_flag + rb, p.flag_target, deadline, &seen)) {
+            report_error(p, ST_TIMEOUT_FLAG, rb, seen, p.flag_target);
+            *abort_flag = 1;
+            first = static_cast<uint32_t>(units);  // nothing more to do for this group
+            break;
+          }
+          ready_rb = rb;
+        }
+        ptx::fence_acq_rel_gpu();  // the tiles behind the counters, before the group's loads
+      }
+      gs->job[it & 1] = first;
+    }
+    group_barrier(group);
+    const uint32_t base = gs->job[it & 1];
+    if (base >= static_cast<uint32_t>(units)) break;
+    if (leader) claimed = atomicAdd(p.job_counter, static_cast<uint32_t>(kGroupWarps));  // latency hides behind the unit
+    const int u = static_cast<int>(base) + wg;
+    if (u >= units) continue;
+    const int octet = u / col_units;
+    const int cu = u - octet * col_units;
+    const int r0 = octet * ROWS;
+    const bool timeline = p.row_trace != nullptr && cu == 0 && lane == 0;
+    const unsigned long long t_ready = timeline ? ptx::globaltimer_ns() : 0ull;
+    const long long row_off = static_cast<long long>(r0) * p.N;
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(p.stage) + row_off;
+    uint16_t* dst = reinterpret_cast<uint16_t*>(p.out[0]) + row_off;
+    uint4 v[2][ROWS];
+    int c[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      c[h] = cu * CHUNKS + h * 32 + lane;
+      const int cl = min(c[h], n_chunks - 1);  // loads past the row's end are clamped and their values dropped
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) v[h][i] = ptx::ld_cg_v4(src + static_cast<long long>(i) * p.N + cl * 8);
+    }
+    // four lanes share a row's statistics
+    float ssq = 0.f;
+    const float* part = p.ssq + static_cast<long long>(r0 / 128) * p.TN * 128 + (r0 & 127) + (lane >> 2);
+    for (int t0 = lane & 3; t0 < p.TN; t0 += 4 * STATS) {
+      float s[STATS];
+#pragma unroll
+      for (int k = 0; k < STATS; ++k) s[k] = __ldcg(part + min(t0 + 4 * k, p.TN - 1) * 128);
+#pragma unroll
+      for (int k = 0; k < STATS; ++k) ssq += t0 + 4 * k < p.TN ? s[k] : 0.f;
+    }
+    ssq += __shfl_xor_sync(0xffffffffu, ssq, 1);
+    ssq += __shfl_xor_sync(0xffffffffu, ssq, 2);
+    const float rstd = rsqrtf(ssq / static_cast<float>(p.N) + p.eps);
+    const unsigned long long t_sum = timeline ? ptx::globaltimer_ns() : 0ull;
+    float rs[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) rs[i] = __shfl_sync(0xffffffffu, rstd, i * 4);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (c[h] < n_chunks) {
+        const uint4 w = gamma_here ? ptx::ld_shared_v4(gamma_smem + (static_cast<uint32_t>(c[h]) << 4)) : __ldg(gamma + c[h]);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+          ptx::st_v4(dst + static_cast<long long>(i) * p.N + c[h] * 8, scale_chunk<BF16>(v[h][i], rs[i], w));
+        }
+      }
+    }
+    if (timeline) {
+      const long long m = p.M;
+      const unsigned long long t_end = ptx::globaltimer_ns();
+      for (int g = r0; g < r0 + ROWS; ++g) {
+        p.row_trace[g] = t_claim != 0 ? t_claim : t_ready;
+        p.row_trace[m + g] = t_end;
+        p.row_trace[2 * m + g] = static_cast<unsigned long long>(blockIdx.x) * 4ull + group;
+        p.row_trace[3 * m + g] = t_ready;
+        p.row_trace[4 * m + g] = t_sum;
+        p.row_trace[5 * m + g] = t_sum;
+      }
+    }
+    if (p.phase_trace != nullptr && cu == 0 && lane == 0) {
+      t_last = ptx::globaltimer_ns();
+      if (t_first == 0) t_first = t_last;
+      rows_done += ROWS;
+    }
+  }
+  if (p.phase_trace != nullptr && lane == 0 && rows_done != 0) {
+    unsigned long long* tr = p.phase_trace + static_cast<unsigned long long>(kTraceWords) * blockIdx.x;
+    atomicMax(tr + 2, t_last);
+    atomicMin(tr + 4, t_first);
+    atomicAdd(tr + 5, static_cast<unsigned long long>(rows_done));
+  }
+}
+
 template <bool BF16>
 __device__ __forceinline__ void comm_dispatch(const FusedParams& p, GroupScratch* gs, uint32_t gamma_smem, int group, int wg,
                                            int lane, uint64_t deadline, volatile uint32_t* abort_flag) {
@@ -653,6 +776,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
 
   const int num_tiles = p.TM * p.TN;
   const int num_kb = (p.K + BK - 1) / BK;  // a K tail is zero-filled by TMA
+  if (p.clear_words != nullptr && warp == 2 && blockIdx.x == 0) {
+    for (int i = lane; i < kFlagWords / 4; i += 32) {
+      reinterpret_cast<uint4*>(p.clear_words)[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
 
   if (warp == 0) {
     // ===================== TMA producer =====================
@@ -856,6 +984,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         slab_dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(L, row0, n_blk * BN) +
                    (lane >> 3) * pitch + chunk * 8;
       }
+      float ssq = 0.f;  // of this lane's row over the tile's columns, as rounded
 
 #pragma unroll 1
       for (int cc = 0; cc < BN / 64; ++cc) {
@@ -880,6 +1009,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
           v.y = pack2<BF16>(__uint_as_float(r0[8 * j + 2]), __uint_as_float(r0[8 * j + 3]));
           v.z = pack2<BF16>(__uint_as_float(r0[8 * j + 4]), __uint_as_float(r0[8 * j + 5]));
           v.w = pack2<BF16>(__uint_as_float(r0[8 * j + 6]), __uint_as_float(r0[8 * j + 7]));
+          if (p.ssq != nullptr) ssq += sum_squares<BF16>(v);
           ptx::st_shared_v4(slab + lane * 128 + ((j ^ (lane & 7)) << 4), v);
         }
 #pragma unroll
@@ -889,6 +1019,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
           v.y = pack2<BF16>(__uint_as_float(r1[8 * j + 2]), __uint_as_float(r1[8 * j + 3]));
           v.z = pack2<BF16>(__uint_as_float(r1[8 * j + 4]), __uint_as_float(r1[8 * j + 5]));
           v.w = pack2<BF16>(__uint_as_float(r1[8 * j + 6]), __uint_as_float(r1[8 * j + 7]));
+          if (p.ssq != nullptr) ssq += sum_squares<BF16>(v);
           ptx::st_shared_v4(slab + lane * 128 + (((j + 4) ^ (lane & 7)) << 4), v);
         }
         __syncwarp();
@@ -922,6 +1053,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
           }
           ptx::st_v4(dst, v);
         }
+        __syncwarp();
+      }
+      if (p.ssq != nullptr) {
+        p.ssq[(static_cast<long long>(row0 / BM) * p.TN + n_blk) * BM + q * 32 + lane] = ssq;
         __syncwarp();
       }
 
@@ -964,7 +1099,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         const int blk_row0 = m_blk * TILE_M + static_cast<int>(cta_rank) * BM;
         const int flag_blk = blk_row0 / BM;
         if (p.flag[0] != nullptr) {
-          ptx::fence_acq_rel_sys();
+          if (p.ws == 1) ptx::fence_acq_rel_gpu();  // nobody outside this GPU reads the tile
+          else ptx::fence_acq_rel_sys();
           if (p.nvls) {
             ptx::multimem_red_relaxed_add(p.mc_flag + flag_blk, 1u);  // lands on every rank
           } else if (p.own_mode == OWN_INTERLEAVE) {
@@ -1107,6 +1243,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
   }
 
   // ===================== reduce phase (every warp ends up here) =====================
+  if (p.ssq != nullptr) {
+    norm_stream<BF16>(p, group_scratch + group, gamma_smem, group, wg, lane, deadline, abort_flag);
+    return;
+  }
   comm_dispatch<BF16>(p, group_scratch + group, gamma_smem, group, wg, lane, deadline, abort_flag);
 
   // All-reduce: the kernel may only end once every owner has delivered its

@@ -369,6 +369,11 @@ __device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t* addr) {
   asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* addr) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ uint32_t ld_relaxed_sys(const uint32_t* addr) {
   uint32_t v;
   asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
@@ -391,6 +396,21 @@ __device__ __forceinline__ bool wait_counter_geq(const uint32_t* addr, uint32_t 
       }
     }
     __nanosleep(64);
+  }
+}
+
+// Same for a counter that only this GPU raises.  The caller fences (acquire) after it returns true.
+__device__ __forceinline__ bool wait_counter_relaxed_gpu(const uint32_t* addr, uint32_t target, uint64_t deadline_ns,
+                                                         uint32_t* last) {
+  uint32_t spins = 0;
+  while (true) {
+    const uint32_t v = ld_relaxed_gpu(addr);
+    if (static_cast<int32_t>(v - target) >= 0) return true;
+    if ((++spins & 0x3fu) == 0u && globaltimer_ns() > deadline_ns) {
+      *last = v;
+      return false;
+    }
+    __nanosleep(100);
   }
 }
 

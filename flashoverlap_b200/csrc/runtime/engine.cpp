@@ -168,8 +168,14 @@ void FusedEngine::base_params(FusedParams& p, const SignalArgs* sig) {
   p.epi_layout.ld = 0;
 }
 
+uint32_t* FusedEngine::clear_next_set(int set, cudaStream_t stream) {
+  if (world_ == 1) return flag_ptr(rank_, set ^ 1);
+  check(cudaMemsetAsync(flag_ptr(rank_, set ^ 1), 0, kFlagWords * 4, stream), "cudaMemsetAsync(counters)");
+  return nullptr;
+}
+
 void FusedEngine::gemm(const GemmOperands& g_in, void* C, const OutLayout* layout, const SignalArgs* sig,
-                       cudaStream_t stream) {
+                       cudaStream_t stream, uint32_t* clear_words) {
   NvtxRange range("flashoverlap::gemm");
   if (!initialized()) init(0, 1, nullptr);
   check_previous("gemm");
@@ -184,12 +190,13 @@ void FusedEngine::gemm(const GemmOperands& g_in, void* C, const OutLayout* layou
   p.epi_base[0] = C;
   if (layout != nullptr) p.epi_layout = *layout;
   else p.epi_layout.ld = g.N;
+  p.clear_words = clear_words;
   if (p.raster_group == 0) p.raster_group = 8;
   const char* why = nullptr;
   check_launch(launch_fused(g, p, stream, &why), why, "gemm");
 }
 
-void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* out, const NormArgs& norm,
+void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* out, float* ssq, const NormArgs& norm,
                                cudaStream_t stream) {
   NvtxRange range("flashoverlap::gemm_rmsnorm");
   if (!initialized()) init(0, 1, nullptr);
@@ -219,6 +226,7 @@ void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* ou
   p.reduce = 1;
   if (row_trace_ != nullptr && g.M <= row_trace_rows_) p.row_trace = row_trace_;
   p.stage = scratch;
+  p.ssq = ssq;
   p.flag_target = static_cast<uint32_t>(g.N / tc.bn);
   p.norm = norm.gamma != nullptr;
   p.gamma = norm.gamma;
@@ -254,12 +262,12 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
   if (g.M / 128 > kMaxTileRows) throw std::runtime_error("gemm_allreduce: too many tile rows");
   ensure_workspace(g.M, g.N);
   const int set = static_cast<int>(calls_ & 1ull);
-  check(cudaMemsetAsync(flag_ptr(rank_, set ^ 1), 0, kFlagWords * 4, stream), "cudaMemsetAsync(counters)");
+  uint32_t* const clear_words = clear_next_set(set, stream);
   if (world_ == 1 && norm.gamma == nullptr && !(out_user != nullptr && overlaps_operand(g, out_user))) {
     // One rank and no RMSNorm: nothing to sum or scale, the GEMM writes the result itself, in either layout.
-    // The buffer sets still alternate (and the other set's counters are cleared above) like after any fused call.
+    // The buffer sets still alternate (and the other set's counters are cleared) like after any fused call.
     void* result = out_user != nullptr ? out_user : heap_.local(ws_.result[set]);
-    gemm(g, result, out_layout, sig, stream);
+    gemm(g, result, out_layout, sig, stream, clear_words);
     ++calls_;
     return result;
   }
@@ -296,6 +304,8 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
   p.norm = norm.gamma != nullptr;
   p.gamma = norm.gamma;
   p.eps = norm.eps;
+  p.clear_words = clear_words;
+  if (world_ == 1 && p.norm) p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
   // with one rank there is nobody to deliver to: rows go to the result buffer like a reduce-scatter's
   p.bcast = world_ > 1 ? 1 : 0;
   if (out_layout != nullptr) p.out_layout = *out_layout;
@@ -330,9 +340,9 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
   }
   ensure_workspace(g.M, g.N);
   const int set = static_cast<int>(calls_ & 1ull);
-  check(cudaMemsetAsync(flag_ptr(rank_, set ^ 1), 0, kFlagWords * 4, stream), "cudaMemsetAsync(counters)");
+  uint32_t* const clear_words = clear_next_set(set, stream);
   if (world_ == 1 && norm.gamma == nullptr) {
-    gemm(g, D, out_layout, sig, stream);  // one rank, no RMSNorm: the GEMM writes the rows where they belong
+    gemm(g, D, out_layout, sig, stream, clear_words);  // one rank, no RMSNorm: the GEMM writes the rows where they belong
     ++calls_;
     return;
   }
@@ -374,6 +384,8 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
   p.norm = norm.gamma != nullptr;
   p.gamma = norm.gamma;
   p.eps = norm.eps;
+  p.clear_words = clear_words;
+  if (world_ == 1 && p.norm) p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
   p.bcast = 0;
   p.job_counter = flag_ptr(rank_, set) + kFlagJob;
   p.out[rank_] = D;

@@ -74,11 +74,15 @@ class FusedEngine {
   }
 
   // C[M,N] = A[M,K] * B[N,K]^T on this GPU only.  `layout` null = row-major.
-  void gemm(const GemmOperands& g, void* C, const OutLayout* layout, const SignalArgs* sig, cudaStream_t stream);
+  // `clear_words`: counter set the kernel zeroes on the way (null = none).
+  void gemm(const GemmOperands& g, void* C, const OutLayout* layout, const SignalArgs* sig, cudaStream_t stream,
+            uint32_t* clear_words = nullptr);
 
   // GEMM + RMSNorm on one GPU (world size 1 form of the fused operations):
   // `scratch` receives the un-normalised product, `out` the normalised rows.
-  void gemm_rmsnorm(const GemmOperands& g, void* scratch, void* out, const NormArgs& norm, cudaStream_t stream);
+  // `ssq`: M * N / 64 floats of scratch for the sums of squares (see FusedParams::ssq).
+  void gemm_rmsnorm(const GemmOperands& g, void* scratch, void* out, float* ssq, const NormArgs& norm,
+                    cudaStream_t stream);
 
   // Fused GEMM + all-reduce (+ RMSNorm).  Collective: every rank of the group
   // must call it with the same shapes.  The result lands in a symmetric result
@@ -195,6 +199,9 @@ class FusedEngine {
   void base_params(FusedParams& p, const SignalArgs* sig);
   uint32_t* flag_ptr(int rank, int set) const;
   uint32_t* done_ptr(int rank, int set) const;
+  // Zeroes the counters of the set after `set`: by a memset before the call when other ranks raise them; with one
+  // rank the fused kernel does it on the way (returned for FusedParams::clear_words).
+  uint32_t* clear_next_set(int set, cudaStream_t stream);
 
   int rank_ = 0, world_ = 1;
   AllGatherFn all_gather_;

@@ -87,6 +87,28 @@ def test_gemm_rmsnorm_more_rows_than_one_wave():
     assert (O.float() - want).abs().max().item() <= 3e-2 * want.abs().max().item()
 
 
+@pytest.mark.parametrize("algo,M,N", [(2, 128, 64), (2, 384, 4544), (7, 128, 8256), (5, 256, 1088), (8, 2816, 768)])
+def test_norm_of_scattered_row_statistics(algo, M, N):
+    # sums of squares from 1, 71, 129 and 17 tile columns (more than a lane loads at once), row ends inside a unit of 512
+    # columns, weights beyond shared memory, more units than row groups; a plain call between two normalising ones
+    # leaves the counters of the next call clean
+    K = 200
+    A, B, W = make_inputs(M, N, K, torch.float16, seed=N)
+    impl = make_impl()
+    y = (A.double() @ B.double().t())
+    want = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * W.double()
+    for norm in (True, False, True, True):
+        out = impl.gemm_allreduce_fused(A, B, W if norm else None, 1e-5, algo)
+        D = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float16)
+        impl.gemm_reducescatter_fused(A, B, D, W if norm else None, 1e-5, algo, False)
+        torch.cuda.synchronize()
+        impl.check_status()
+        ref = want if norm else y
+        # the product, its scaling and the weight are each rounded to 11 bits
+        for got in (out, D):
+            assert ((got.double() - ref).abs() <= 2 ** -9.3 * ref.abs() + 1e-4).all(), (norm, algo)
+
+
 def test_phase_trace_records_every_row_once():
     M, N, K = 2048, 2048, 256
     A, B, W = make_inputs(M, N, K, torch.float16, seed=4)
