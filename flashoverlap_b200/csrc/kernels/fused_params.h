@@ -106,7 +106,8 @@ struct alignas(64) FusedParams {
   int a_own_begin, a_own_end;
 
   int M, N, K;
-  int TM, TN;        // tile grid (BM = 128)
+  int TM, TN;        // tile grid; the last tile row and column may reach past M and N (whole blocks of 128 rows, 64 columns)
+  int trace_cols;    // phase trace: columns that count as one tile (those of the tile the caller named)
   int raster_group;  // tile rows walked column-major together (L2 reuse of B)
   int raster_taper;  // 1 = the last groups shrink by halves so that little is left to communicate after the last tile
   int force_full_grid;  // launch the requested number of CTAs even when there are fewer tiles

@@ -972,6 +972,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       ptx::tc_fence_after_sync();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
       const int row0 = m_blk * TILE_M + static_cast<int>(cta_rank) * BM + q * 32;  // first global row of this warp's slab
+      // What of the tile lies inside the matrix: all of this CTA's 128 rows or none, and whole steps of 64 columns.
+      const int steps = row0 >= p.M ? 0 : min(BN, p.N - n_blk * BN) / 64;
+      if (steps == 0) {
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          if constexpr (CTAS == 2) ptx::mbar_arrive_cluster(tempty_addr0 + 8u * buf);
+          else ptx::mbar_arrive(&tempty_bar[buf]);
+          ptx::st_release_cta_shared(&epi_prog[q], static_cast<uint32_t>(it + 1));
+        }
+        continue;
+      }
       const int chunk = lane & 7;  // of a 128-byte row segment; eight lanes write one
       // A slab that stays on this GPU is a plain pitched block, in the natural layout and in the tiled one
       // (its 32 rows lie in one tile row, its 64 columns in one tile): the address is found once per step at most.
@@ -987,12 +999,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       float ssq = 0.f;  // of this lane's row over the tile's columns, as rounded
 
 #pragma unroll 1
-      for (int cc = 0; cc < BN / 64; ++cc) {
+      for (int cc = 0; cc < steps; ++cc) {
         uint32_t r0[32], r1[32];
         ptx::tmem_ld_32x32b_x32(t_row + cc * 64, r0);
         ptx::tmem_ld_32x32b_x32(t_row + cc * 64 + 32, r1);
         ptx::tmem_ld_wait();
-        if (cc == BN / 64 - 1) {
+        if (cc == steps - 1) {
           // accumulator fully read: hand the TMEM buffer back to the MMA warp
           ptx::tc_fence_before_sync();
           __syncwarp();
@@ -1097,6 +1109,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         int m_blk, n_blk;
         tile_coords(p, t, m_blk, n_blk);
         const int blk_row0 = m_blk * TILE_M + static_cast<int>(cta_rank) * BM;
+        if (blk_row0 >= p.M) continue;  // this CTA's half of the last tile row is empty
         const int flag_blk = blk_row0 / BM;
         if (p.flag[0] != nullptr) {
           if (p.ws == 1) ptx::fence_acq_rel_gpu();  // nobody outside this GPU reads the tile
@@ -1233,7 +1246,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       unsigned long long* tr = p.phase_trace + static_cast<unsigned long long>(kTraceWords) * blockIdx.x;
       tr[1] = ptx::globaltimer_ns();
       int mine = 0;
-      for (int t = first_tile; t < num_tiles; t += tile_stride) ++mine;
+      for (int t = first_tile; t < num_tiles; t += tile_stride) {
+        int m_blk, n_blk;
+        tile_coords(p, t, m_blk, n_blk);
+        if (m_blk * TILE_M + static_cast<int>(cta_rank) * BM >= p.M) continue;
+        const int n0 = n_blk * BN, n1 = min(n0 + BN, p.N);
+        mine += (n1 + p.trace_cols - 1) / p.trace_cols - (n0 + p.trace_cols - 1) / p.trace_cols;  // tiles that begin here
+      }
       tr[3] = static_cast<unsigned long long>(mine);
     }
     if (!p.reduce || *abort_flag) return;

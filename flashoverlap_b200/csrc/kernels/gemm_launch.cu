@@ -8,6 +8,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include <cstdlib>
@@ -80,11 +81,48 @@ cudaError_t prepare_fused(int algo, DType dtype) {
   return kPrepareTable[algo][dtype == DT_BF16 ? 1 : 0]();
 }
 
+namespace {
+int ceil_div(int a, int b) { return (a + b - 1) / b; }
+
+// Estimated time in ns of a GEMM in one tile configuration: whole waves of tiles, each as long as K.
+// per_k: ns per value of K and wave (single waves of fp16, K from 2048 to 8192, all SMs busy).  A CTA takes in 110 to
+//   125 GB/s of operands, which is what the tiles of up to 128 columns wait for; only the 256-wide ones wait for the
+//   tensor cores.  A stage of 64 K-values costs 290 ns at least, one of 128 K-values 430 ns.
+// fixed: launch, pipeline fill and the epilogue of the last tile.
+// Where the operands do not stay in L2 the time is at least their way from HBM.
+double estimate_ns(const GemmOperands& g, int algo, int ctas) {
+  struct Measured {
+    double per_k, fixed;
+  };
+  static const Measured measured[] = {{6.7, 7000}, {4.6, 7000}, {4.5, 6000}, {6.1, 9500}, {4.7, 8700}, {4.5, 7700},
+                                      {4.1, 6300}, {3.4, 5500}, {6.0, 9000}, {3.75, 8300}, {3.4, 7300}};
+  static_assert(sizeof(measured) / sizeof(measured[0]) == kNumAlgos, "one entry per tile configuration");
+  const TileConfig& tc = kAlgoTable[algo];
+  const int waves = ceil_div(ceil_div(g.M, tc.bm) * ceil_div(g.N, tc.bn), std::max(1, ctas / tc.ctas));
+  const double operands = 2.0 * (static_cast<double>(g.M) + g.N) * g.K / 6000;  // bytes at 6 TB/s
+  return std::max(waves * static_cast<double>(g.K) * measured[algo].per_k, operands) + measured[algo].fixed + 300.0 * waves;
+}
+}  // namespace
+
+int plan_algo(const GemmOperands& g, int ctas) {
+  if (!g.any_tile) return g.algo;
+  int best = g.algo;
+  double best_ns = 0.97 * estimate_ns(g, g.algo, ctas);  // the named one is kept unless another is clearly faster
+  for (int algo = 0; algo < kNumAlgos; ++algo) {
+    const double ns = estimate_ns(g, algo, ctas);
+    if (ns < best_ns && ctas >= kAlgoTable[algo].ctas) {
+      best_ns = ns;
+      best = algo;
+    }
+  }
+  return best;
+}
+
 cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t stream, const char** why) {
   const char* dummy;
   if (why == nullptr) why = &dummy;
   *why = "";
-  const TileConfig tc = algo_config(g.algo);
+  TileConfig tc = algo_config(g.algo);
   if (g.algo < 0 || g.algo >= kNumAlgos) {
     *why = "Algo index out of range";
     return cudaErrorInvalidValue;
@@ -97,6 +135,12 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
     *why = "A and B must be 16-byte aligned";
     return cudaErrorInvalidValue;
   }
+  int grid = g.sm_count > 0 ? g.sm_count : device_sm_count();
+  const int sms = device_sm_count();
+  if (grid > sms) grid = sms;  // every CTA must be resident: CTAs wait on one another's output
+  const int algo = plan_algo(g, grid);
+  p.trace_cols = tc.bn;
+  tc = kAlgoTable[algo];
   // every CTA stages 128 rows of A and (for a CTA pair) half of the B tile, 64 K-values per box
   const int a_rows = g.a_rows > 0 && g.a_rows < g.M ? g.a_rows : g.M;  // the copy engine fills the rows after them with zero
   if (!make_tensor_map(&p.tmA, g.A, a_rows, g.K, 128, g.dtype) ||
@@ -121,14 +165,12 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
   p.M = g.M;
   p.N = g.N;
   p.K = g.K;
-  p.TM = g.M / tc.bm;
-  p.TN = g.N / tc.bn;
+  p.TM = ceil_div(g.M, tc.bm);
+  p.TN = ceil_div(g.N, tc.bn);
+  if (algo != g.algo && p.reduce) p.flag_target = static_cast<uint32_t>(p.TN);
   if (p.raster_group <= 0) p.raster_group = 1;
   if (p.raster_group > p.TM) p.raster_group = p.TM;
   if (p.rot < 0 || p.rot >= p.TM) p.rot = 0;
-  int grid = g.sm_count > 0 ? g.sm_count : device_sm_count();
-  const int sms = device_sm_count();
-  if (grid > sms) grid = sms;  // every CTA must be resident: CTAs wait on one another's output
   if (p.reduce && p.job_counter == nullptr) {
     *why = "the reduce phase needs a row-job counter";
     return cudaErrorInvalidValue;
@@ -136,7 +178,7 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
   if (!p.reduce && !p.force_full_grid && grid > p.TM * p.TN * tc.ctas) grid = p.TM * p.TN * tc.ctas;
   if (tc.ctas == 2 && grid < 2) grid = 2;
   if (tc.ctas == 2) grid &= ~1;
-  return kLaunchTable[g.algo][g.dtype == DT_BF16 ? 1 : 0](p, grid, stream);
+  return kLaunchTable[algo][g.dtype == DT_BF16 ? 1 : 0](p, grid, stream);
 }
 
 }  // namespace fo

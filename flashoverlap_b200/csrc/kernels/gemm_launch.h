@@ -36,7 +36,13 @@ struct GemmOperands {
   // Rows that A really holds when that is less than M (M is a multiple of the
   // tile height); the rows after them read as zero.  0 = A holds M rows.
   int a_rows;
+  // 1 = the result does not depend on the tile shape (natural or tile-ordered output on one GPU, nothing counts
+  // tiles): `algo` then says which shapes are accepted, and the launch takes the configuration plan_algo finds.
+  int any_tile;
 };
+
+// The tile configuration (index of the table) in which a GEMM on `ctas` CTAs is expected to take least time.
+int plan_algo(const GemmOperands& g, int ctas);
 
 // Fills p.tmA / p.tmB / shape fields from `g`, validates shapes, launches.
 // Everything else in `p` must already be set by the caller.  Returns

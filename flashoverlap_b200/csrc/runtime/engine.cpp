@@ -191,6 +191,7 @@ void FusedEngine::gemm(const GemmOperands& g_in, void* C, const OutLayout* layou
   if (layout != nullptr) p.epi_layout = *layout;
   else p.epi_layout.ld = g.N;
   p.clear_words = clear_words;
+  g.any_tile = sig == nullptr && (layout == nullptr || layout->row_map == nullptr) ? 1 : 0;
   if (p.raster_group == 0) p.raster_group = 8;
   const char* why = nullptr;
   check_launch(launch_fused(g, p, stream, &why), why, "gemm");
@@ -227,6 +228,7 @@ void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* ou
   if (row_trace_ != nullptr && g.M <= row_trace_rows_) p.row_trace = row_trace_;
   p.stage = scratch;
   p.ssq = ssq;
+  g.any_tile = 1;
   p.flag_target = static_cast<uint32_t>(g.N / tc.bn);
   p.norm = norm.gamma != nullptr;
   p.gamma = norm.gamma;
@@ -305,7 +307,10 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
   p.gamma = norm.gamma;
   p.eps = norm.eps;
   p.clear_words = clear_words;
-  if (world_ == 1 && p.norm) p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
+  if (world_ == 1 && p.norm) {
+    p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
+    g.any_tile = 1;
+  }
   // with one rank there is nobody to deliver to: rows go to the result buffer like a reduce-scatter's
   p.bcast = world_ > 1 ? 1 : 0;
   if (out_layout != nullptr) p.out_layout = *out_layout;
@@ -385,7 +390,10 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
   p.gamma = norm.gamma;
   p.eps = norm.eps;
   p.clear_words = clear_words;
-  if (world_ == 1 && p.norm) p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
+  if (world_ == 1 && p.norm) {
+    p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
+    g.any_tile = 1;
+  }
   p.bcast = 0;
   p.job_counter = flag_ptr(rank_, set) + kFlagJob;
   p.out[rank_] = D;

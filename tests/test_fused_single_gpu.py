@@ -177,6 +177,37 @@ def test_world1_allreduce_and_reducescatter(with_norm):
     assert (D.float() - want).abs().max().item() <= 1e-2 * want.abs().max().item()
 
 
+@pytest.mark.parametrize("algo,M,N,K", [
+    (2, 384, 2112, 4096), (1, 5504, 3456, 264), (6, 1152, 1408, 2048), (7, 128, 4672, 520), (0, 2432, 2816, 1000),
+    (9, 2304, 8320, 136), (3, 256, 256, 64)])
+def test_gemm_in_another_tile_configuration(algo, M, N, K):
+    # one rank: the named configuration says which shapes are accepted, the launch may take a larger tile whose last row
+    # or column reaches past the matrix; natural order, tile order and RMSNorm
+    A, B, W = make_inputs(M, N, K, torch.bfloat16, seed=K)
+    impl = make_impl()
+    y = A.double() @ B.double().t()
+    guard = torch.full((M + 1, N), 7.0, device="cuda", dtype=torch.bfloat16)   # the row after the result
+    C = guard[:M]
+    impl.cutlass_gemm(A, B, C, algo)
+    out = impl.gemm_allreduce_fused(A, B, W, 1e-5, algo)
+    bm, bn, _ = impl.algo_tile(algo)
+    tiles = (M // bm) * (N // bn)
+    RA = reorder_indices(tiles, list(range(tiles))[::-1], device="cuda").reshape(M // bm, N // bn)
+    cseg = torch.tensor([tiles], dtype=torch.int32)
+    MM = torch.zeros((M // bm + 1, N // bn), dtype=torch.int32, device="cuda")
+    T = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    impl.gemm_allreduce_overlap(A, B, T, MM, RA, 1, cseg, cseg.cuda(), algo, False)
+    torch.cuda.synchronize()
+    impl.check_status()
+    top = y.abs().max().item()
+    # rounding to 8 significant bits is off by at most 2^-8 of a value (and fp32 sums by far less); with RMSNorm three times
+    assert (C.double() - y).abs().max().item() <= 1.01 * 2 ** -8 * top
+    assert bool((guard[M] == 7).all())
+    assert torch.equal(from_tile_order(T, bm, bn, RA), C)
+    want = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * W.double()
+    assert ((out.double() - want).abs() <= 2 ** -6.3 * want.abs() + 1e-4).all()
+
+
 def test_compat_overlap_api_reordered_layout_and_trace():
     M, N, K, algo = 1024, 2048, 256, 0
     A, B, W = make_inputs(M, N, K, torch.float16, seed=5)
