@@ -139,6 +139,7 @@ TORCH_LIBRARY(flashoverlap_class, m) {
       .def("mutlass_init", &OverlapImpl::CutlassInit)
       .def("overlap_init", &OverlapImpl::OverlapInit)
       .def("cutlass_gemm", &OverlapImpl::Gemm)
+      .def("gemm_swiglu", &OverlapImpl::GemmSwiglu)
       .def("mutlass_gemm", &OverlapImpl::Gemm)
       .def("gemm_allreduce_overlap", &OverlapImpl::GemmAllReduceOverlap)
       .def("gemm_reducescatter_overlap", &OverlapImpl::GemmReduceScatterOverlap)

@@ -142,6 +142,20 @@ void OverlapImpl::Gemm(at::Tensor A, at::Tensor B, at::Tensor C, int64_t algo) {
   engine_.gemm(operands(A, B, algo), C.data_ptr(), nullptr, nullptr, current_stream());
 }
 
+void OverlapImpl::GemmSwiglu(at::Tensor A, at::Tensor B, at::Tensor C, int64_t algo) {
+  check_gemm_args(A, B, nullptr);
+  check_matrix(C, "C");
+  TORCH_CHECK(C.scalar_type() == A.scalar_type() && C.device() == A.device() && C.size(0) == A.size(0) &&
+                  C.size(1) * 2 == B.size(0),
+              "C must be [M, N/2] with A's dtype");
+  c10::cuda::CUDAGuard guard(A.device());
+  GemmOperands g = operands(A, B, algo);
+  const TileConfig tc = algo_config(g.algo);
+  TORCH_CHECK(tc.ctas == 2 && tc.bn >= 128, "gemm_swiglu: Algo ", algo, " is not a CTA-pair tile of at least 128 columns");
+  g.glu = 1;
+  engine_.gemm(g, C.data_ptr(), nullptr, nullptr, current_stream());
+}
+
 void OverlapImpl::GemmAllReduceOverlap(at::Tensor A, at::Tensor B, at::Tensor C, at::Tensor MM, at::Tensor RA,
                                        int64_t rLDN, at::Tensor cSEG_CPU, at::Tensor cSEG_GPU, int64_t algo,
                                        bool if_monitor) {

@@ -28,6 +28,9 @@ class OverlapImpl : public torch::CustomClassHolder {
   void CutlassInit();
   void OverlapInit();
   void Gemm(at::Tensor A, at::Tensor B, at::Tensor C, int64_t algo);
+  // C[M, N/2] = silu(A * Bg^T) * (A * Bu^T) in one launch; B holds the N/2 gate rows, then the N/2 up rows.  Needs a
+  // CTA-pair tile configuration of at least 128 columns.
+  void GemmSwiglu(at::Tensor A, at::Tensor B, at::Tensor C, int64_t algo);
   void GemmAllReduceOverlap(at::Tensor A, at::Tensor B, at::Tensor C, at::Tensor MM, at::Tensor RA, int64_t rLDN,
                             at::Tensor cSEG_CPU, at::Tensor cSEG_GPU, int64_t algo, bool if_monitor);
   // (C is scratch: in the reference it holds this rank's partial products for

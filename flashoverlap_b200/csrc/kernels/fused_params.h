@@ -113,6 +113,10 @@ struct alignas(64) FusedParams {
   int force_full_grid;  // launch the requested number of CTAs even when there are fewer tiles
   int rot;           // first tile row of the walk (gathered operands start at the rank's own rows)
   int owner_stride;  // > 0 (block ownership): tile rows per owner; the walk then cycles through the owners
+  // Gated form (CTA pairs only): B holds N / 2 gate rows, then N / 2 up rows; a tile takes BN / 2 of each (the first CTA of
+  // the pair stages the gate rows, the second the up rows) and stores BN / 2 columns of silu(gate) * up.  0 = off,
+  // else N / 2.
+  int glu;
   int l2_hints;      // 1 = TMA loads carry L2 eviction hints (A panel kept, B panel streamed)
 
   // ---- GEMM epilogue destination -------------------------------------------

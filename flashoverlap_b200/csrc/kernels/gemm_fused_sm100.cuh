@@ -147,6 +147,8 @@ __device__ __forceinline__ uint32_t norm_pack2(float a, float b, float rstd, uin
   }
 }
 
+__device__ __forceinline__ float silu(float x) { return x / (1.f + expf(-x)); }
+
 // Sum of the squares of eight 16-bit values.
 template <bool BF16>
 __device__ __forceinline__ float sum_squares(const uint4& h) {
@@ -799,7 +801,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         int m_blk, n_blk;
         tile_coords(p, t, m_blk, n_blk);
         const int a_row = m_blk * TILE_M + static_cast<int>(cta_rank) * BM;
-        const int b_row = n_blk * BN + static_cast<int>(cta_rank) * T::B_ROWS;
+        const int b_row = p.glu ? n_blk * T::B_ROWS + static_cast<int>(cta_rank) * p.glu
+                                : n_blk * BN + static_cast<int>(cta_rank) * T::B_ROWS;
         // this CTA's 128 rows of A come from the caller's own shard (never copied) or from the (gathered) A
         const bool own_rows = a_row >= p.a_own_begin && a_row + BM <= p.a_own_end;
         const CUtensorMap* map_a = own_rows ? &p.tmA_own : &p.tmA;
@@ -973,7 +976,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
       const int row0 = m_blk * TILE_M + static_cast<int>(cta_rank) * BM + q * 32;  // first global row of this warp's slab
       // What of the tile lies inside the matrix: all of this CTA's 128 rows or none, and whole steps of 64 columns.
-      const int steps = row0 >= p.M ? 0 : min(BN, p.N - n_blk * BN) / 64;
+      const int cols_left = p.glu ? 2 * (p.glu - n_blk * (BN / 2)) : p.N - n_blk * BN;
+      const int steps = row0 >= p.M ? 0 : min(BN, cols_left) / 64;
       if (steps == 0) {
         ptx::tc_fence_before_sync();
         __syncwarp();
@@ -993,16 +997,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       const long long pitch = L.tiled ? static_cast<long long>(L.rldn) * L.bn : L.ld;
       uint16_t* slab_dst = nullptr;
       if (pitched) {
-        slab_dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(L, row0, n_blk * BN) +
+        slab_dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(L, row0, n_blk * (p.glu ? BN / 2 : BN)) +
                    (lane >> 3) * pitch + chunk * 8;
       }
       float ssq = 0.f;  // of this lane's row over the tile's columns, as rounded
 
 #pragma unroll 1
       for (int cc = 0; cc < steps; ++cc) {
+        // 64 columns of the tile; gated: 32 gate columns and the 32 up columns that belong to them
         uint32_t r0[32], r1[32];
-        ptx::tmem_ld_32x32b_x32(t_row + cc * 64, r0);
-        ptx::tmem_ld_32x32b_x32(t_row + cc * 64 + 32, r1);
+        ptx::tmem_ld_32x32b_x32(t_row + (p.glu ? cc : 2 * cc) * 32, r0);
+        ptx::tmem_ld_32x32b_x32(t_row + (p.glu ? BN / 64 + cc : 2 * cc + 1) * 32, r1);
         ptx::tmem_ld_wait();
         if (cc == steps - 1) {
           // accumulator fully read: hand the TMEM buffer back to the MMA warp
@@ -1012,6 +1017,29 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
             if constexpr (CTAS == 2) ptx::mbar_arrive_cluster(tempty_addr0 + 8u * buf);
             else ptx::mbar_arrive(&tempty_bar[buf]);
           }
+        }
+        if (p.glu) {
+          // 32 result columns go to the first or second half of the slab, which is stored when it is full
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int x = 8 * j + 2 * e;
+              o[e] = pack2<BF16>(silu(__uint_as_float(r0[x])) * __uint_as_float(r1[x]),
+                                 silu(__uint_as_float(r0[x + 1])) * __uint_as_float(r1[x + 1]));
+            }
+            ptx::st_shared_v4(slab + lane * 128 + (((j + 4 * (cc & 1)) ^ (lane & 7)) << 4), make_uint4(o[0], o[1], o[2], o[3]));
+          }
+          if ((cc & 1) == 0) continue;
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = i * 4 + (lane >> 3);
+            ptx::st_v4(slab_dst + i * 4 * pitch + (cc >> 1) * 64, ptx::ld_shared_v4(slab + r * 128 + ((chunk ^ (r & 7)) << 4)));
+          }
+          __syncwarp();
+          continue;
         }
         // registers -> swizzled smem slab (row = lane, 8 chunks of 16 bytes)
 #pragma unroll

@@ -83,6 +83,10 @@ cudaError_t prepare_fused(int algo, DType dtype) {
 
 namespace {
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
+int tile_columns(const GemmOperands& g, const TileConfig& tc) {
+  return g.glu ? ceil_div(g.N / 2, tc.bn / 2) : ceil_div(g.N, tc.bn);
+}
+bool can_run(const GemmOperands& g, const TileConfig& tc) { return !g.glu || (tc.ctas == 2 && tc.bn >= 128); }
 
 // Estimated time in ns of a GEMM in one tile configuration: whole waves of tiles, each as long as K.
 // per_k: ns per value of K and wave (single waves of fp16, K from 2048 to 8192, all SMs busy).  A CTA takes in 110 to
@@ -98,7 +102,7 @@ double estimate_ns(const GemmOperands& g, int algo, int ctas) {
                                       {4.1, 6300}, {3.4, 5500}, {6.0, 9000}, {3.75, 8300}, {3.4, 7300}};
   static_assert(sizeof(measured) / sizeof(measured[0]) == kNumAlgos, "one entry per tile configuration");
   const TileConfig& tc = kAlgoTable[algo];
-  const int waves = ceil_div(ceil_div(g.M, tc.bm) * ceil_div(g.N, tc.bn), std::max(1, ctas / tc.ctas));
+  const int waves = ceil_div(ceil_div(g.M, tc.bm) * tile_columns(g, tc), std::max(1, ctas / tc.ctas));
   const double operands = 2.0 * (static_cast<double>(g.M) + g.N) * g.K / 6000;  // bytes at 6 TB/s
   return std::max(waves * static_cast<double>(g.K) * measured[algo].per_k, operands) + measured[algo].fixed + 300.0 * waves;
 }
@@ -110,7 +114,7 @@ int plan_algo(const GemmOperands& g, int ctas) {
   double best_ns = 0.97 * estimate_ns(g, g.algo, ctas);  // the named one is kept unless another is clearly faster
   for (int algo = 0; algo < kNumAlgos; ++algo) {
     const double ns = estimate_ns(g, algo, ctas);
-    if (ns < best_ns && ctas >= kAlgoTable[algo].ctas) {
+    if (ns < best_ns && ctas >= kAlgoTable[algo].ctas && can_run(g, kAlgoTable[algo])) {
       best_ns = ns;
       best = algo;
     }
@@ -133,6 +137,10 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
   }
   if ((reinterpret_cast<uintptr_t>(g.A) & 15u) || (reinterpret_cast<uintptr_t>(g.B) & 15u)) {
     *why = "A and B must be 16-byte aligned";
+    return cudaErrorInvalidValue;
+  }
+  if (!can_run(g, tc)) {
+    *why = "the gated form needs a CTA-pair tile of at least 128 columns";
     return cudaErrorInvalidValue;
   }
   int grid = g.sm_count > 0 ? g.sm_count : device_sm_count();
@@ -162,11 +170,12 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
     p.a_own_begin = g.own_begin;
     p.a_own_end = g.own_begin + g.own_rows;
   }
+  p.glu = g.glu ? g.N / 2 : 0;
   p.M = g.M;
   p.N = g.N;
   p.K = g.K;
   p.TM = ceil_div(g.M, tc.bm);
-  p.TN = ceil_div(g.N, tc.bn);
+  p.TN = tile_columns(g, tc);
   if (algo != g.algo && p.reduce) p.flag_target = static_cast<uint32_t>(p.TN);
   if (p.raster_group <= 0) p.raster_group = 1;
   if (p.raster_group > p.TM) p.raster_group = p.TM;

@@ -39,6 +39,8 @@ struct GemmOperands {
   // 1 = the result does not depend on the tile shape (natural or tile-ordered output on one GPU, nothing counts
   // tiles): `algo` then says which shapes are accepted, and the launch takes the configuration plan_algo finds.
   int any_tile;
+  // 1 = gated form (see FusedParams::glu): the result has N / 2 columns.  CTA-pair tiles of at least 128 columns.
+  int glu;
 };
 
 // The tile configuration (index of the table) in which a GEMM on `ctas` CTAs is expected to take least time.

@@ -189,7 +189,7 @@ void FusedEngine::gemm(const GemmOperands& g_in, void* C, const OutLayout* layou
   p.rows_per_owner = g.M;
   p.epi_base[0] = C;
   if (layout != nullptr) p.epi_layout = *layout;
-  else p.epi_layout.ld = g.N;
+  else p.epi_layout.ld = g.glu ? g.N / 2 : g.N;
   p.clear_words = clear_words;
   g.any_tile = sig == nullptr && (layout == nullptr || layout->row_map == nullptr) ? 1 : 0;
   if (p.raster_group == 0) p.raster_group = 8;

@@ -83,9 +83,7 @@ class TPDecoderBlock(nn.Module):
         h2 = resid + o
         m_in = torch.empty_like(h2)
         torch.ops.flashoverlap_op.rmsnorm(h2, m_in, self.norm_attn, self.eps)
-        gu = torch.empty((T, self.w_gate_up.shape[0]), dtype=h2.dtype, device=h2.device)
-        impl.cutlass_gemm(m_in, self.w_gate_up, gu, self._fit(T, self.w_gate_up.shape[0]))
-        act = self._mlp_act(gu)
+        act = self._gated(m_in)
         rows = T // self.world
         y = torch.empty((rows, self.hidden), dtype=h2.dtype, device=h2.device)
         impl.gemm_reducescatter_fused(act, self.w_down, y, None, self.eps, a, False)  # GEMM + reduce-scatter
@@ -95,6 +93,22 @@ class TPDecoderBlock(nn.Module):
         qkv_next = torch.empty((T, self.w_qkv_next.shape[0]), dtype=h3.dtype, device=h3.device)
         impl.allgather_gemm(n, self.w_qkv_next, qkv_next, self._fit_gather(T, self.w_qkv_next.shape[0]))  # all-gather + GEMM
         return qkv_next, h3
+
+    def _gated(self, x):
+        """silu(x Wg^T) * (x Wu^T).  With a CTA-pair tile the GEMM's epilogue applies the gate to its fp32 sums and
+        stores the half that the down-projection reads; the [tokens, 2 * ffn] product never reaches memory."""
+        from ..utils.config import ALGO_TILES
+
+        T, rows = x.shape[0], self.w_gate_up.shape[0]
+        algo = self._fit(T, rows)
+        bm, bn, _ = ALGO_TILES[algo]
+        if bm == 256 and bn >= 128:
+            act = torch.empty((T, rows // 2), dtype=x.dtype, device=x.device)
+            self.impl.gemm_swiglu(x, self.w_gate_up, act, algo)
+            return act
+        gu = torch.empty((T, rows), dtype=x.dtype, device=x.device)
+        self.impl.cutlass_gemm(x, self.w_gate_up, gu, algo)
+        return self._mlp_act(gu)
 
     def _fit(self, M, N):
         """The preferred tile configuration if it divides the shape, else a smaller one."""

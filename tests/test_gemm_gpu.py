@@ -91,3 +91,26 @@ def test_algo_table_matches_generated_python_copy():
     impl = _impl()
     assert impl.num_algos() == len(ALGO_TILES)
     assert [tuple(impl.algo_tile(a)) for a in ALGOS] == [tuple(t) for t in ALGO_TILES]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("algo,M,ffn", [(8, 256, 128), (3, 512, 1920), (9, 768, 64), (4, 256, 14336 // 8)])
+def test_gemm_swiglu(dtype, algo, M, ffn):
+    # gate and up columns of one tile in the two CTAs of a pair; one tile, ragged last tile column, the narrowest
+    K = 328
+    torch.manual_seed(ffn)
+    impl = torch.classes.flashoverlap_class.OverlapImpl()
+    impl.cutlass_init()
+    x = torch.randn(M, K, device="cuda", dtype=dtype)
+    w = (torch.randn(2 * ffn, K, device="cuda") * 2 / K ** 0.5).to(dtype)
+    guard = torch.full((M + 1, ffn), 3.0, device="cuda", dtype=dtype)
+    impl.gemm_swiglu(x, w, guard[:M], algo)
+    torch.cuda.synchronize()
+    gate, up = (x.double() @ w.double().t()).chunk(2, dim=-1)
+    want = torch.nn.functional.silu(gate) * up
+    # one rounding of the result (11 or 8 bits) on fp32 sums
+    eps = 2 ** -10.9 if dtype == torch.float16 else 2 ** -7.9
+    assert ((guard[:M].double() - want).abs() <= eps * want.abs() + 1e-5).all()
+    assert bool((guard[M] == 3).all())
+    with pytest.raises(RuntimeError):
+        impl.gemm_swiglu(x, w, guard[:M], 0)      # not a CTA-pair tile
