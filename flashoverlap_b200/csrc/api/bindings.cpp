@@ -81,6 +81,30 @@ static void rmsnorm_op(at::Tensor X, at::Tensor O, at::Tensor RW, double eps) {
   TORCH_CHECK(e == cudaSuccess, "rmsnorm launch failed: ", cudaGetErrorString(e));
 }
 
+// add_rmsnorm(X, R, S, O, RW, eps): S = X + R (rounded to the 16-bit type), O = rmsnorm(S); one pass over the rows.
+static void add_rmsnorm_op(at::Tensor X, at::Tensor R, at::Tensor S, at::Tensor O, at::Tensor RW, double eps) {
+  check_matrix(X, "X");
+  check_matrix(R, "R");
+  check_matrix(S, "S");
+  check_matrix(O, "O");
+  const DType dt = dtype_of(X);
+  for (const at::Tensor* t : {&R, &S, &O}) {
+    TORCH_CHECK(t->scalar_type() == X.scalar_type() && t->sizes() == X.sizes() && t->device() == X.device(),
+                "X, R, S and O must have one shape, dtype and device");
+  }
+  TORCH_CHECK(RW.is_cuda() && RW.is_contiguous() && RW.numel() == X.size(1) && RW.scalar_type() == X.scalar_type(),
+              "RW must hold dim values of X's dtype");
+  TORCH_CHECK(X.size(1) % 8 == 0, "dim must be a multiple of 8");
+  for (const at::Tensor* t : {&X, &R, &S, &O, &RW}) {
+    TORCH_CHECK(reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "tensors must be 16-byte aligned");
+  }
+  c10::cuda::CUDAGuard guard(X.device());
+  cudaError_t e = launch_add_rmsnorm(X.data_ptr(), R.data_ptr(), S.data_ptr(), O.data_ptr(), RW.data_ptr(),
+                                     static_cast<int>(X.size(0)), static_cast<int>(X.size(1)), static_cast<float>(eps),
+                                     dt, at::cuda::getCurrentCUDAStream().stream());
+  TORCH_CHECK(e == cudaSuccess, "add_rmsnorm launch failed: ", cudaGetErrorString(e));
+}
+
 // The order in which the persistent kernel walks the tile grid, computed on
 // the host by the function the kernel itself uses: entry i is
 // tile_row * TN + tile_column of the i-th tile of the walk.  For tests and for
@@ -194,5 +218,6 @@ TORCH_LIBRARY(flashoverlap_op, m) {
   m.def("reorder_rmsnorm", &fo::reorder_rmsnorm_op);
   m.def("reorder_rmsnorm_eps", &fo::reorder_rmsnorm_eps);
   m.def("rmsnorm", &fo::rmsnorm_op);
+  m.def("add_rmsnorm", &fo::add_rmsnorm_op);
   m.def("tile_walk", &fo::tile_walk_op);
 }

@@ -15,45 +15,71 @@ namespace {
 
 constexpr int kMaxNormThreads = 1024;
 
-template <bool BF16, bool REORDER, int CPT>
-__global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t* x, uint16_t* out,
-                                                                  const uint16_t* __restrict__ w, int rows, int dim,
-                                                                  float eps, OutLayout L) {
+// What a row is before it is normalised: as stored, stored in tile order, or the sum of two rows (written back).
+enum NormInput { NORM_ROWS, NORM_TILES, NORM_SUM };
+
+template <bool BF16>
+__device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {
+  const float2 f = unpack2<BF16>(a), g = unpack2<BF16>(b);
+  return pack2<BF16>(f.x + g.x, f.y + g.y);
+}
+template <bool BF16>
+__device__ __forceinline__ uint4 add_chunk(const uint4& a, const uint4& b) {
+  return make_uint4(add2<BF16>(a.x, b.x), add2<BF16>(a.y, b.y), add2<BF16>(a.z, b.z), add2<BF16>(a.w, b.w));
+}
+
+// `r` and `sum`: NORM_SUM only.
+template <bool BF16, int INPUT, int CPT>
+__global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t* x, const uint16_t* r, uint16_t* sum,
+                                                                  uint16_t* out, const uint16_t* __restrict__ w,
+                                                                  int rows, int dim, float eps, OutLayout L) {
+  constexpr bool ADD = INPUT == NORM_SUM;
   __shared__ float red[2][kMaxNormThreads / 32];
   const int n_chunks = dim >> 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int warps = blockDim.x >> 5;
 
-  auto load = [&](int row, uint4 (&v)[CPT]) {
+  auto load = [&](int row, uint4 (&v)[CPT], uint4 (&a)[ADD ? CPT : 1]) {
 #pragma unroll
     for (int k = 0; k < CPT; ++k) {
       // a chunk past the end of the row is clamped and its value dropped: the loads stay unconditional and go out together
       const int c = min(static_cast<int>(threadIdx.x + k * blockDim.x), n_chunks - 1);
       const uint16_t* src;
-      if constexpr (REORDER) src = x + layout_offset(L, row, c * 8);
+      if constexpr (INPUT == NORM_TILES) src = x + layout_offset(L, row, c * 8);
       else src = x + static_cast<long long>(row) * dim + c * 8;
       v[k] = *reinterpret_cast<const uint4*>(src);
+      if constexpr (ADD) a[k] = *reinterpret_cast<const uint4*>(r + static_cast<long long>(row) * dim + c * 8);
     }
   };
 
-  constexpr bool KEEP = CPT <= 2;  // room for the weights beside two rows; four chunks read them from L1 for each row
+  // room for the weights beside two rows; four chunks (two of a sum) read them from L1 for each row
+  constexpr bool KEEP = CPT <= (ADD ? 1 : 2);
   const uint4* weights = reinterpret_cast<const uint4*>(w);
-  uint4 v[CPT], g[KEEP ? CPT : 1];
+  uint4 v[CPT], a[ADD ? CPT : 1], g[KEEP ? CPT : 1];
   int row = blockIdx.x;
-  load(row, v);
+  load(row, v, a);
   if constexpr (KEEP) {
 #pragma unroll
     for (int k = 0; k < CPT; ++k) g[k] = __ldg(weights + min(static_cast<int>(threadIdx.x + k * blockDim.x), n_chunks - 1));
   }
   for (int par = 0; row < rows; par ^= 1) {
     float ssq = 0.f;
+    if constexpr (ADD) {
+      uint4* dst = reinterpret_cast<uint4*>(sum + static_cast<long long>(row) * dim);
+#pragma unroll
+      for (int k = 0; k < CPT; ++k) {
+        const int c = threadIdx.x + k * blockDim.x;
+        v[k] = add_chunk<BF16>(v[k], a[k]);
+        if (c < n_chunks) dst[c] = v[k];
+      }
+    }
 #pragma unroll
     for (int k = 0; k < CPT; ++k) {
       ssq += static_cast<int>(threadIdx.x + k * blockDim.x) < n_chunks ? sum_squares<BF16>(v[k]) : 0.f;
     }
     const int next = row + gridDim.x;
     uint4 nv[CPT];
-    if (next < rows) load(next, nv);
+    if (next < rows) load(next, nv, a);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
     if (warps > 1) {
@@ -77,8 +103,9 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t
 }
 
 // Rows wider than the registers of a CTA hold: one CTA per row, read twice.
-template <bool BF16, bool REORDER>
-__global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_wide_kernel(const uint16_t* x, uint16_t* out,
+template <bool BF16, int INPUT>
+__global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_wide_kernel(const uint16_t* x, const uint16_t* r,
+                                                                       uint16_t* sum, uint16_t* out,
                                                                        const uint16_t* __restrict__ w, int dim,
                                                                        float eps, OutLayout L) {
   __shared__ float red[kMaxNormThreads / 32];
@@ -86,8 +113,15 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_wide_kernel(const uin
   const int n_chunks = dim >> 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long row_off = static_cast<long long>(row) * dim;
+  if constexpr (INPUT == NORM_SUM) {  // every thread reads back exactly the chunks it wrote
+    for (int c = threadIdx.x; c < n_chunks; c += kMaxNormThreads) {
+      reinterpret_cast<uint4*>(sum + row_off)[c] = add_chunk<BF16>(reinterpret_cast<const uint4*>(x + row_off)[c],
+                                                                   reinterpret_cast<const uint4*>(r + row_off)[c]);
+    }
+  }
   auto src_ptr = [&](int c) -> const uint4* {
-    if constexpr (REORDER) return reinterpret_cast<const uint4*>(x + layout_offset(L, row, c * 8));
+    if constexpr (INPUT == NORM_SUM) return reinterpret_cast<const uint4*>(sum + row_off) + c;
+    else if constexpr (INPUT == NORM_TILES) return reinterpret_cast<const uint4*>(x + layout_offset(L, row, c * 8));
     else return reinterpret_cast<const uint4*>(x + row_off) + c;
   };
   float ssq = 0.f;
@@ -106,12 +140,12 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_wide_kernel(const uin
   }
 }
 
-template <bool BF16, bool REORDER>
-cudaError_t launch_typed(const uint16_t* x, uint16_t* out, const uint16_t* w, int rows, int dim, float eps,
-                         const OutLayout& L, cudaStream_t stream) {
+template <bool BF16, int INPUT>
+cudaError_t launch_typed(const uint16_t* x, const uint16_t* r, uint16_t* sum, uint16_t* out, const uint16_t* w, int rows,
+                         int dim, float eps, const OutLayout& L, cudaStream_t stream) {
   const int n_chunks = dim >> 3;
   if (n_chunks > 4 * kMaxNormThreads) {
-    rmsnorm_wide_kernel<BF16, REORDER><<<rows, kMaxNormThreads, 0, stream>>>(x, out, w, dim, eps, L);
+    rmsnorm_wide_kernel<BF16, INPUT><<<rows, kMaxNormThreads, 0, stream>>>(x, r, sum, out, w, dim, eps, L);
     return cudaGetLastError();
   }
   const int sms = device_sm_count();
@@ -124,29 +158,27 @@ cudaError_t launch_typed(const uint16_t* x, uint16_t* out, const uint16_t* w, in
   int per_sm = kMaxNormThreads / threads;
   if (per_sm > 32) per_sm = 32;
   const int grid = rows < sms * per_sm ? rows : sms * per_sm;
-  auto kernel = cpt == 1   ? rmsnorm_kernel<BF16, REORDER, 1>
-                : cpt == 2 ? rmsnorm_kernel<BF16, REORDER, 2>
-                           : rmsnorm_kernel<BF16, REORDER, 4>;
-  kernel<<<grid, threads, 0, stream>>>(x, out, w, rows, dim, eps, L);
+  auto kernel = cpt == 1   ? rmsnorm_kernel<BF16, INPUT, 1>
+                : cpt == 2 ? rmsnorm_kernel<BF16, INPUT, 2>
+                           : rmsnorm_kernel<BF16, INPUT, 4>;
+  kernel<<<grid, threads, 0, stream>>>(x, r, sum, out, w, rows, dim, eps, L);
   return cudaGetLastError();
 }
 
-template <bool REORDER>
-cudaError_t launch(const void* x, void* out, const void* w, int rows, int dim, float eps, const OutLayout& L, DType dt,
-                   cudaStream_t stream) {
+template <int INPUT>
+cudaError_t launch(const void* x, const void* r, void* sum, void* out, const void* w, int rows, int dim, float eps,
+                   const OutLayout& L, DType dt, cudaStream_t stream) {
   if (rows <= 0 || dim <= 0 || dim % 8 != 0) return cudaErrorInvalidValue;
-  auto typed = dt == DT_BF16 ? launch_typed<true, REORDER> : launch_typed<false, REORDER>;
-  return typed(static_cast<const uint16_t*>(x), static_cast<uint16_t*>(out), static_cast<const uint16_t*>(w), rows, dim,
-               eps, L, stream);
+  auto typed = dt == DT_BF16 ? launch_typed<true, INPUT> : launch_typed<false, INPUT>;
+  return typed(static_cast<const uint16_t*>(x), static_cast<const uint16_t*>(r), static_cast<uint16_t*>(sum),
+               static_cast<uint16_t*>(out), static_cast<const uint16_t*>(w), rows, dim, eps, L, stream);
 }
 
 }  // namespace
 
 cudaError_t launch_rmsnorm(const void* x, void* out, const void* w, int rows, int dim, float eps, DType dt,
                            cudaStream_t stream) {
-  OutLayout L{};
-  L.ld = dim;
-  return launch<false>(x, out, w, rows, dim, eps, L, dt, stream);
+  return launch<NORM_ROWS>(x, nullptr, nullptr, out, w, rows, dim, eps, OutLayout{}, dt, stream);
 }
 
 cudaError_t launch_reorder_rmsnorm(const void* x, void* out, const void* w, int rows, int dim, float eps,
@@ -154,7 +186,12 @@ cudaError_t launch_reorder_rmsnorm(const void* x, void* out, const void* w, int 
   if (in_layout.tiled && (in_layout.bn % 8 != 0 || in_layout.bm <= 0 || in_layout.rldn <= 0)) {
     return cudaErrorInvalidValue;
   }
-  return launch<true>(x, out, w, rows, dim, eps, in_layout, dt, stream);
+  return launch<NORM_TILES>(x, nullptr, nullptr, out, w, rows, dim, eps, in_layout, dt, stream);
+}
+
+cudaError_t launch_add_rmsnorm(const void* x, const void* r, void* sum, void* out, const void* w, int rows, int dim,
+                               float eps, DType dt, cudaStream_t stream) {
+  return launch<NORM_SUM>(x, r, sum, out, w, rows, dim, eps, OutLayout{}, dt, stream);
 }
 
 }  // namespace fo

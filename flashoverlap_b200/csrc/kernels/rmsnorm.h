@@ -18,4 +18,8 @@ cudaError_t launch_rmsnorm(const void* x, void* out, const void* w, int rows, in
 cudaError_t launch_reorder_rmsnorm(const void* x, void* out, const void* w, int rows, int dim, float eps,
                                    const OutLayout& in_layout, DType dt, cudaStream_t stream);
 
+// sum = x + r (rounded to the 16-bit type), out = RMSNorm of sum; natural layout.  dim % 8 == 0.
+cudaError_t launch_add_rmsnorm(const void* x, const void* r, void* sum, void* out, const void* w, int rows, int dim,
+                               float eps, DType dt, cudaStream_t stream);
+
 }  // namespace fo

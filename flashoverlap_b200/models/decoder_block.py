@@ -80,19 +80,24 @@ class TPDecoderBlock(nn.Module):
         impl.cutlass_gemm(h_norm, self.w_qkv, qkv, self._fit(T, self.w_qkv.shape[0]))
         attn = self._attention(qkv, batch, seq)
         o = impl.gemm_allreduce_fused(attn, self.w_o, None, self.eps, a)          # GEMM + all-reduce
-        h2 = resid + o
-        m_in = torch.empty_like(h2)
-        torch.ops.flashoverlap_op.rmsnorm(h2, m_in, self.norm_attn, self.eps)
+        h2, m_in = self._add_norm(resid, o, self.norm_attn)
         act = self._gated(m_in)
         rows = T // self.world
         y = torch.empty((rows, self.hidden), dtype=h2.dtype, device=h2.device)
         impl.gemm_reducescatter_fused(act, self.w_down, y, None, self.eps, a, False)  # GEMM + reduce-scatter
-        h3 = h2[self.rank * rows:(self.rank + 1) * rows] + y
-        n = torch.empty_like(h3)
-        torch.ops.flashoverlap_op.rmsnorm(h3, n, self.norm_next, self.eps)
+        h3, n = self._add_norm(h2[self.rank * rows:(self.rank + 1) * rows], y, self.norm_next)
         qkv_next = torch.empty((T, self.w_qkv_next.shape[0]), dtype=h3.dtype, device=h3.device)
         impl.allgather_gemm(n, self.w_qkv_next, qkv_next, self._fit_gather(T, self.w_qkv_next.shape[0]))  # all-gather + GEMM
         return qkv_next, h3
+
+    def _add_norm(self, x, r, weight):
+        """x + r and its RMSNorm, in one pass."""
+        x = x.expand_as(r).contiguous()
+        if x.data_ptr() % 16:
+            x = x.clone()
+        s, n = torch.empty_like(x), torch.empty_like(x)
+        torch.ops.flashoverlap_op.add_rmsnorm(x, r, s, n, weight, self.eps)
+        return s, n
 
     def _gated(self, x):
         """silu(x Wg^T) * (x Wu^T).  With a CTA-pair tile the GEMM's epilogue applies the gate to its fp32 sums and

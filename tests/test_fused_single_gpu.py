@@ -337,6 +337,17 @@ def test_rmsnorm_thread_shapes(rows, dim):
     assert torch.equal(x, o)
 
 
+@pytest.mark.parametrize("rows,dim", [(1, 8), (37, 8000), (600, 4096), (300, 16392), (3, 32776)])
+def test_add_rmsnorm(rows, dim):
+    torch.manual_seed(dim)
+    x, r = torch.randn(2, rows, dim, device="cuda", dtype=torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(dim, device="cuda")).to(torch.bfloat16)
+    s, o, o2 = (torch.full_like(x, float("nan")) for _ in range(3))
+    torch.ops.flashoverlap_op.add_rmsnorm(x, r, s, o, w, 1e-5)
+    torch.ops.flashoverlap_op.rmsnorm(x + r, o2, w, 1e-5)
+    assert torch.equal(s, x + r) and torch.equal(o, o2)      # the two steps one after the other
+
+
 def test_reorder_rmsnorm_rldn2():
     M, N, bm, bn = 512, 1024, 128, 256
     tm, tn = M // bm, N // bn
