@@ -725,9 +725,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint64_t t_start = ptx::globaltimer_ns();
-  const uint64_t deadline = t_start + p.timeout_ns;
-
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) {
       ptx::mbar_init(&full_bar[i], 1);
@@ -740,21 +737,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     ptx::mbar_init(pair_bar, 1);
     *abort_flag = 0;
     for (int i = 0; i < 4; ++i) epi_prog[i] = 0;
-    if (p.phase_trace != nullptr) {
-      unsigned long long* tr = p.phase_trace + static_cast<unsigned long long>(kTraceWords) * blockIdx.x;
-      tr[0] = t_start;
-      tr[1] = tr[2] = tr[3] = tr[5] = tr[6] = tr[7] = 0;
-      tr[4] = ~0ull;
-    }
     ptx::mbar_fence_init();
     ptx::fence_proxy_async_smem();
-  }
-  if (p.reduce && p.norm && p.N <= kGammaSmemValues) {
-    // the RMSNorm weights, once per CTA: every row group reads them for every row
-    const uint4* gamma = reinterpret_cast<const uint4*>(p.gamma);
-    for (int c = threadIdx.x; c < (p.N >> 3); c += kThreads) {
-      ptx::st_shared_v4(gamma_smem + (static_cast<uint32_t>(c) << 4), __ldg(gamma + c));
-    }
   }
   if (warp == 0 && lane == 0) {
     ptx::prefetch_tensormap(&p.tmA);
@@ -768,6 +752,24 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     } else {
       ptx::tmem_alloc(tmem_slot, T::TMEM_COLS);
       ptx::tmem_relinquish();
+    }
+  }
+  // Everything above works on this SM alone and may run under the kernel before this one.
+  ptx::wait_for_previous_kernel();
+  ptx::allow_next_kernel();
+  const uint64_t t_start = ptx::globaltimer_ns();
+  const uint64_t deadline = t_start + p.timeout_ns;
+  if (threadIdx.x == 0 && p.phase_trace != nullptr) {
+    unsigned long long* tr = p.phase_trace + static_cast<unsigned long long>(kTraceWords) * blockIdx.x;
+    tr[0] = t_start;
+    tr[1] = tr[2] = tr[3] = tr[5] = tr[6] = tr[7] = 0;
+    tr[4] = ~0ull;
+  }
+  if (p.reduce && p.norm && p.N <= kGammaSmemValues) {
+    // the RMSNorm weights, once per CTA: every row group reads them for every row
+    const uint4* gamma = reinterpret_cast<const uint4*>(p.gamma);
+    for (int c = threadIdx.x; c < (p.N >> 3); c += kThreads) {
+      ptx::st_shared_v4(gamma_smem + (static_cast<uint32_t>(c) << 4), __ldg(gamma + c));
     }
   }
   ptx::tc_fence_before_sync();

@@ -41,7 +41,7 @@ cudaError_t launch_instance(const FusedParams& p, int grid, cudaStream_t stream)
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = T::SMEM_BYTES;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   int n = 0;
   if (CTAS == 2) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
@@ -53,6 +53,11 @@ cudaError_t launch_instance(const FusedParams& p, int grid, cudaStream_t stream)
   if (cooperative_launch_enabled()) {
     attr[n].id = cudaLaunchAttributeCooperative;
     attr[n].val.cooperative = 1;
+    ++n;
+  } else {
+    // barriers, TMEM and descriptors of this launch are set up under the kernel before it
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
     ++n;
   }
   cfg.attrs = attr;

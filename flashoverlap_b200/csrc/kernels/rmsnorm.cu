@@ -35,6 +35,8 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t
                                                                   int rows, int dim, float eps, OutLayout L) {
   constexpr bool ADD = INPUT == NORM_SUM;
   __shared__ float red[2][kMaxNormThreads / 32];
+  ptx::wait_for_previous_kernel();
+  ptx::allow_next_kernel();
   const int n_chunks = dim >> 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int warps = blockDim.x >> 5;
@@ -109,6 +111,8 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_wide_kernel(const uin
                                                                        const uint16_t* __restrict__ w, int dim,
                                                                        float eps, OutLayout L) {
   __shared__ float red[kMaxNormThreads / 32];
+  ptx::wait_for_previous_kernel();
+  ptx::allow_next_kernel();
   const int row = blockIdx.x;
   const int n_chunks = dim >> 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -140,13 +144,27 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_wide_kernel(const uin
   }
 }
 
+// Launch whose CTAs may be placed while the kernel before it drains (they wait for it themselves).
+template <typename... Params, typename... Args>
+cudaError_t launch_after(void (*kernel)(Params...), int grid, int threads, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 template <bool BF16, int INPUT>
 cudaError_t launch_typed(const uint16_t* x, const uint16_t* r, uint16_t* sum, uint16_t* out, const uint16_t* w, int rows,
                          int dim, float eps, const OutLayout& L, cudaStream_t stream) {
   const int n_chunks = dim >> 3;
   if (n_chunks > 4 * kMaxNormThreads) {
-    rmsnorm_wide_kernel<BF16, INPUT><<<rows, kMaxNormThreads, 0, stream>>>(x, r, sum, out, w, dim, eps, L);
-    return cudaGetLastError();
+    return launch_after(rmsnorm_wide_kernel<BF16, INPUT>, rows, kMaxNormThreads, stream, x, r, sum, out, w, dim, eps, L);
   }
   const int sms = device_sm_count();
   // Few rows: as many threads per row as it has chunks, since only the latency of one row counts.  Many rows: two
@@ -161,8 +179,7 @@ cudaError_t launch_typed(const uint16_t* x, const uint16_t* r, uint16_t* sum, ui
   auto kernel = cpt == 1   ? rmsnorm_kernel<BF16, INPUT, 1>
                 : cpt == 2 ? rmsnorm_kernel<BF16, INPUT, 2>
                            : rmsnorm_kernel<BF16, INPUT, 4>;
-  kernel<<<grid, threads, 0, stream>>>(x, r, sum, out, w, rows, dim, eps, L);
-  return cudaGetLastError();
+  return launch_after(kernel, grid, threads, stream, x, r, sum, out, w, rows, dim, eps, L);
 }
 
 template <int INPUT>

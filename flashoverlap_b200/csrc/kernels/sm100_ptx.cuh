@@ -101,6 +101,13 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
   }
 }
 
+// Programmatic dependent launch.  A kernel launched with the attribute may start while the kernel before it in the
+// stream still runs: it touches no global memory before wait_for_previous_kernel(), which returns when that kernel
+// has completed and its writes are visible.  allow_next_kernel() lets the kernel after this one start in the same way
+// (once every CTA has called it, so no CTA of this grid can be kept from an SM by the next one).
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Named barrier over `threads` threads of the CTA (id 1..15; id 0 is __syncthreads).
 __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
