@@ -41,14 +41,41 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int warps = blockDim.x >> 5;
 
+  // Tile order: a thread's columns lie in the same tile column, at the same place in it, in every row.
+  int tile_col[INPUT == NORM_TILES ? CPT : 1], in_tile[INPUT == NORM_TILES ? CPT : 1];
+  if constexpr (INPUT == NORM_TILES) {
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      const int col = min(static_cast<int>(threadIdx.x + k * blockDim.x), n_chunks - 1) * 8;
+      tile_col[k] = col / L.bn;
+      in_tile[k] = col - tile_col[k] * L.bn;
+    }
+  }
   auto load = [&](int row, uint4 (&v)[CPT], uint4 (&a)[ADD ? CPT : 1]) {
+    [[maybe_unused]] const int tile_row = INPUT == NORM_TILES ? row / L.bm : 0;
+    [[maybe_unused]] const int row_in_tile = INPUT == NORM_TILES ? row - tile_row * L.bm : 0;
+    [[maybe_unused]] int slot[INPUT == NORM_TILES ? CPT : 1];
+    if constexpr (INPUT == NORM_TILES) {
+#pragma unroll
+      for (int k = 0; k < CPT; ++k) {
+        slot[k] = tile_row * L.tn + tile_col[k];
+        if (L.ra != nullptr) slot[k] = __ldg(L.ra + slot[k]);
+      }
+    }
 #pragma unroll
     for (int k = 0; k < CPT; ++k) {
       // a chunk past the end of the row is clamped and its value dropped: the loads stay unconditional and go out together
       const int c = min(static_cast<int>(threadIdx.x + k * blockDim.x), n_chunks - 1);
       const uint16_t* src;
-      if constexpr (INPUT == NORM_TILES) src = x + layout_offset(L, row, c * 8);
-      else src = x + static_cast<long long>(row) * dim + c * 8;
+      if constexpr (INPUT == NORM_TILES) {
+        int view = slot[k], place = 0;  // tile row of the view and place in it
+        if (L.rldn > 1) {
+          view = slot[k] / L.rldn;
+          place = slot[k] - view * L.rldn;
+        }
+        src = x + (static_cast<long long>(view) * L.bm + row_in_tile) * (static_cast<long long>(L.rldn) * L.bn) +
+              place * L.bn + in_tile[k];
+      } else src = x + static_cast<long long>(row) * dim + c * 8;
       v[k] = *reinterpret_cast<const uint4*>(src);
       if constexpr (ADD) a[k] = *reinterpret_cast<const uint4*>(r + static_cast<long long>(row) * dim + c * 8);
     }
