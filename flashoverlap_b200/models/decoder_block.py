@@ -59,9 +59,10 @@ class TPDecoderBlock(nn.Module):
         hd, h, kv = self.head_dim, self.heads, self.kv_heads
         q, k, v = qkv.split([h * hd, kv * hd, kv * hd], dim=-1)
         q = q.reshape(batch, seq, h, hd).transpose(1, 2)
-        k = k.reshape(batch, seq, kv, hd).transpose(1, 2).repeat_interleave(h // kv, dim=1)
-        v = v.reshape(batch, seq, kv, hd).transpose(1, 2).repeat_interleave(h // kv, dim=1)
-        o = F.scaled_dot_product_attention(q, k, v, is_causal=True)
+        # a key and value head serves h // kv query heads in place (repeating them is two copies of their own)
+        k = k.reshape(batch, seq, kv, hd).transpose(1, 2)
+        v = v.reshape(batch, seq, kv, hd).transpose(1, 2)
+        o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=h != kv)
         return o.transpose(1, 2).reshape(batch * seq, h * hd).contiguous()
 
     def _mlp_act(self, gu):
