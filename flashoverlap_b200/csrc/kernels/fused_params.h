@@ -161,6 +161,7 @@ struct alignas(64) FusedParams {
   // [M / 128][TN][128], written by the epilogue.  The reduce phase then scales rows without a pass of its own
   // over them (norm_stream).  Null = the row workers find the sums.
   float* ssq;
+  int drop_stage;  // norm_stream: the staged product is scratch, its lines need not reach memory once they are read
   // Counter set of the next call, zeroed by this launch (one rank: nobody else raises it).  Null = the host clears it.
   uint32_t* clear_words;
   const void* stage;               // this GPU's staging: [ws][rows_per_owner][N]

@@ -653,6 +653,15 @@ __device__ __forceinline__ void norm_stream(const FusedParams& p, GroupScratch* 
         }
       }
     }
+    if (p.drop_stage) {
+      // 8 rows of 8 lines; every lane of this warp, the only reader, has used its values
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int line = cu * (CHUNKS / 8) + (lane & 7);
+        if (line * 64 < p.N) ptx::discard_line(src + static_cast<long long>(h * 4 + (lane >> 3)) * p.N + line * 64);
+      }
+    }
     if (timeline) {
       const long long m = p.M;
       const unsigned long long t_end = ptx::globaltimer_ns();

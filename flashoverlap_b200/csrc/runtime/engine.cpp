@@ -178,6 +178,12 @@ int local_group(const GemmOperands& g, bool norm) {
 }
 }  // namespace
 
+namespace {
+// Staged products that crowd the L2 (with the result of the same size) are dropped line by line as they are read:
+// 4096 x 8192 x 1024 93.8 -> 90.8 us.  Smaller ones only pay for the instruction: 128 x 8192 16.7 -> 17.1.
+bool drop_stage(const GemmOperands& g) { return 2.0 * g.M * g.N >= 32e6; }
+}  // namespace
+
 uint32_t* FusedEngine::clear_next_set(int set, cudaStream_t stream) {
   if (world_ == 1) return flag_ptr(rank_, set ^ 1);
   check(cudaMemsetAsync(flag_ptr(rank_, set ^ 1), 0, kFlagWords * 4, stream), "cudaMemsetAsync(counters)");
@@ -319,6 +325,7 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
   p.clear_words = clear_words;
   if (world_ == 1 && p.norm) {
     p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
+    p.drop_stage = drop_stage(g) ? 1 : 0;
     g.any_tile = 1;
   }
   // with one rank there is nobody to deliver to: rows go to the result buffer like a reduce-scatter's
@@ -402,6 +409,7 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
   p.clear_words = clear_words;
   if (world_ == 1 && p.norm) {
     p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
+    p.drop_stage = drop_stage(g) ? 1 : 0;
     g.any_tile = 1;
   }
   p.bcast = 0;

@@ -109,6 +109,24 @@ def test_norm_of_scattered_row_statistics(algo, M, N):
             assert ((got.double() - ref).abs() <= 2 ** -9.3 * ref.abs() + 1e-4).all(), (norm, algo)
 
 
+def test_norm_of_a_product_whose_staging_is_dropped():
+    # 34 MB staged: its lines leave the L2 unwritten once they are read, and are written anew by the next calls
+    M, N, K = 2048, 8256, 64
+    impl = make_impl()
+    for seed in range(3):
+        A, B, W = make_inputs(M, N, K, torch.float16, seed=seed)
+        out = impl.gemm_allreduce_fused(A, B, W, 1e-5, 5)
+        D = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float16)
+        impl.gemm_reducescatter_fused(A, B, D, W, 1e-5, 5, False)
+        torch.cuda.synchronize()
+        impl.check_status()
+        y = A.double() @ B.double().t()
+        want = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * W.double()
+        # the product, its scaling and the weight are each rounded to 11 bits
+        for got in (out, D):
+            assert ((got.double() - want).abs() <= 2 ** -9.3 * want.abs() + 1e-4).all()
+
+
 def test_phase_trace_records_every_row_once():
     M, N, K = 2048, 2048, 256
     A, B, W = make_inputs(M, N, K, torch.float16, seed=4)
