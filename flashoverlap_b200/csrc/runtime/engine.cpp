@@ -257,6 +257,8 @@ void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* ou
 }
 
 namespace {
+bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
 // Does the result at `out` share memory with an operand that the GEMM still reads while it writes tiles?
 bool overlaps_operand(const GemmOperands& g, const void* out) {
   auto meets = [](const void* a, size_t na, const void* b, size_t nb) {
@@ -281,8 +283,10 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
   ensure_workspace(g.M, g.N);
   const int set = static_cast<int>(calls_ & 1ull);
   uint32_t* const clear_words = clear_next_set(set, stream);
-  if (world_ == 1 && norm.gamma == nullptr && !(out_user != nullptr && overlaps_operand(g, out_user))) {
-    // One rank and no RMSNorm: nothing to sum or scale, the GEMM writes the result itself, in either layout.
+  if (world_ == 1 && norm.gamma == nullptr &&
+      (out_user == nullptr || (aligned16(out_user) && !overlaps_operand(g, out_user)))) {
+    // One rank and no RMSNorm: nothing to sum or scale, the GEMM writes the result itself, in either layout.  (Its
+    // stores are 16 bytes wide: a result at another address is copied out of the aligned buffer below.)
     // The buffer sets still alternate (and the other set's counters are cleared) like after any fused call.
     void* result = out_user != nullptr ? out_user : heap_.local(ws_.result[set]);
     gemm(g, result, out_layout, sig, stream, clear_words);

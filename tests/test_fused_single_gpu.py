@@ -287,6 +287,27 @@ def test_compat_overlap_writes_tile_order_in_place(algo, rldn, monitor):
     assert torch.equal(A2, C)
 
 
+@pytest.mark.parametrize("offset", [1, 3, 8])
+def test_compat_overlap_result_at_any_element(offset):
+    # a contiguous result that starts between two 16-byte boundaries (and one on a boundary)
+    M, N, K, algo = 256, 512, 64, 0
+    A, B, _ = make_inputs(M, N, K, torch.float16, seed=offset)
+    impl = make_impl()
+    bm, bn, _ = impl.algo_tile(algo)
+    tm, tn = M // bm, N // bn
+    RA = reorder_indices(tm * tn, [2, 0, 3, 1], device="cuda").reshape(tm, tn)
+    cseg = torch.tensor([tm * tn], dtype=torch.int32)
+    MM = torch.zeros((tm + 1, tn), dtype=torch.int32, device="cuda")
+    want = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float16)
+    impl.gemm_allreduce_overlap(A, B, want, MM, RA, 1, cseg, cseg.cuda(), algo, False)
+    buf = torch.full((M * N + 16,), 7.0, device="cuda", dtype=torch.float16)
+    impl.gemm_allreduce_overlap(A, B, buf[offset:offset + M * N].view(M, N), MM, RA, 1, cseg, cseg.cuda(), algo, False)
+    torch.cuda.synchronize()
+    impl.check_status()
+    assert torch.equal(buf[offset:offset + M * N].view(M, N), want)
+    assert bool((buf[:offset] == 7).all()) and bool((buf[offset + M * N:] == 7).all())
+
+
 def test_index_arrays_are_checked_on_the_host_before_any_launch():
     M, N, K, algo = 256, 512, 64, 0
     A, B, W = make_inputs(M, N, K, torch.float16)
