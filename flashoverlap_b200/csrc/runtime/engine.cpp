@@ -266,7 +266,7 @@ bool overlaps_operand(const GemmOperands& g, const void* out) {
     return x < y + nb && y < x + na;
   };
   const size_t n = static_cast<size_t>(g.M) * g.N * 2, k = static_cast<size_t>(g.K) * 2;
-  return meets(out, n, g.A, k * g.M) || meets(out, n, g.B, k * g.N);
+  return meets(out, n, g.A, k * (g.a_rows > 0 ? g.a_rows : g.M)) || meets(out, n, g.B, k * g.N);
 }
 }  // namespace
 
@@ -552,8 +552,9 @@ void FusedEngine::a2a_gemm(const void* A_send, const void* B, void* C, const int
   const int m_pad = a2a_padded_rows(mlen, algo);  // the same on every rank
   // One rank: the GEMM reads the caller's rows where they are, also when they do not fill the last tile (its
   // missing rows read as zero, and the scratch rows of C become zero).  Copying them through the gathered
-  // buffer costs a pass over A that the first tiles wait for.
-  if (world_ == 1 && mlen[0] > 0 && reinterpret_cast<uintptr_t>(A_send) % 16 == 0) {
+  // buffer costs a pass over A that the first tiles wait for.  A product that takes the place of the rows needs that
+  // copy: the first tiles would overwrite what later ones read.
+  if (world_ == 1 && mlen[0] > 0 && aligned16(A_send)) {
     GemmOperands g{};
     g.A = A_send;
     g.B = B;
@@ -563,8 +564,10 @@ void FusedEngine::a2a_gemm(const void* A_send, const void* B, void* C, const int
     g.K = K;
     g.dtype = dtype;
     g.algo = algo;
-    gemm(g, C, nullptr, nullptr, stream);
-    return;
+    if (!overlaps_operand(g, C)) {
+      gemm(g, C, nullptr, nullptr, stream);
+      return;
+    }
   }
   ensure_workspace(static_cast<long long>(m_pad) * (K > N ? K : N), 1);
   const int set = static_cast<int>(calls_ & 1ull);

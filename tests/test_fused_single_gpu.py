@@ -461,6 +461,24 @@ def test_a2a_dispatch_gemm_ragged_rows_in_place(rows, algo):
     assert bool((C[rows:] == 0).all())
 
 
+@pytest.mark.parametrize("rows,K,N", [(300, 512, 512), (1000, 1024, 256), (512, 256, 768)])
+def test_a2a_dispatch_gemm_in_the_place_of_its_rows(rows, K, N):
+    # the product overwrites the rows it is made of, from their first value on: narrower, as wide, wider than they are
+    impl = make_impl()
+    mlen = torch.tensor([[rows]], dtype=torch.int32)
+    A, B, _ = make_inputs(rows, N, K, torch.float16, seed=K)
+    m_pad = impl.a2a_padded_rows(mlen, 0)
+    want = torch.empty((m_pad, N), device="cuda", dtype=torch.float16)
+    impl.a2a_dispatch_gemm(A, B, want, mlen, 0)
+    buf = torch.zeros(max(m_pad * N, rows * K), device="cuda", dtype=torch.float16)
+    rows_view = buf[:rows * K].view(rows, K)
+    rows_view.copy_(A)
+    impl.a2a_dispatch_gemm(rows_view, B, buf[:m_pad * N].view(m_pad, N), mlen, 0)
+    torch.cuda.synchronize()
+    impl.check_status()
+    assert torch.equal(buf[:rows * N].view(rows, N), want[:rows])
+
+
 def test_host_feeder_double_buffers_inputs():
     from flashoverlap_b200.utils.pipeline import HostFeeder
 
