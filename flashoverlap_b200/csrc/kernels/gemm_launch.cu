@@ -139,6 +139,13 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
     *why = "A and B must be 16-byte aligned";
     return cudaErrorInvalidValue;
   }
+  // every store of the epilogue and of the reduce phase, and every load of the weights, is 16 bytes wide
+  if ((reinterpret_cast<uintptr_t>(p.epi_base[0]) & 15u) ||
+      (p.reduce && (reinterpret_cast<uintptr_t>(p.out[p.me]) & 15u)) ||
+      (p.reduce && p.norm && (reinterpret_cast<uintptr_t>(p.gamma) & 15u))) {
+    *why = "the result and the RMSNorm weights must be 16-byte aligned";
+    return cudaErrorInvalidValue;
+  }
   if (!can_run(g, tc)) {
     *why = "the gated form needs a CTA-pair tile of at least 128 columns";
     return cudaErrorInvalidValue;

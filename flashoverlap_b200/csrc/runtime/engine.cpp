@@ -20,7 +20,11 @@ struct NvtxRange {
 void check(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw std::runtime_error(cuda_error_string(e, what));
 }
-void check_launch(cudaError_t e, const char* why, const char* op) {
+bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+// Launches the fused kernel; throws with the launcher's reason when it refuses the call.
+void launch(const GemmOperands& g, FusedParams& p, cudaStream_t stream, const char* op) {
+  const char* why = nullptr;
+  const cudaError_t e = launch_fused(g, p, stream, &why);
   if (e != cudaSuccess) {
     std::string msg = std::string(op) + ": " + (why && *why ? why : "launch failed");
     throw std::runtime_error(cuda_error_string(e, msg.c_str()));
@@ -209,8 +213,7 @@ void FusedEngine::gemm(const GemmOperands& g_in, void* C, const OutLayout* layou
   p.clear_words = clear_words;
   g.any_tile = sig == nullptr && (layout == nullptr || layout->row_map == nullptr) ? 1 : 0;
   if (p.raster_group == 0) p.raster_group = local_group(g, false);
-  const char* why = nullptr;
-  check_launch(launch_fused(g, p, stream, &why), why, "gemm");
+  launch(g, p, stream, "gemm");
 }
 
 void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* out, float* ssq, const NormArgs& norm,
@@ -252,13 +255,10 @@ void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* ou
   p.bcast = 0;
   p.out[0] = out;
   p.out_layout.ld = g.N;
-  const char* why = nullptr;
-  check_launch(launch_fused(g, p, stream, &why), why, "gemm_rmsnorm");
+  launch(g, p, stream, "gemm_rmsnorm");
 }
 
 namespace {
-bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
-
 // Does the result at `out` share memory with an operand that the GEMM still reads while it writes tiles?
 bool overlaps_operand(const GemmOperands& g, const void* out) {
   auto meets = [](const void* a, size_t na, const void* b, size_t nb) {
@@ -338,8 +338,7 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
   else p.out_layout.ld = g.N;
   p.done_target = static_cast<uint32_t>(g.M) * kGroupWarps;  // one delivery count per warp and row
   p.job_counter = flag_ptr(rank_, set) + kFlagJob;
-  const char* why = nullptr;
-  check_launch(launch_fused(g, p, stream, &why), why, "gemm_allreduce");
+  launch(g, p, stream, "gemm_allreduce");
   ++calls_;
   void* result = heap_.local(ws_.result[set]);
   if (out_user != nullptr) {
@@ -421,8 +420,7 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
   p.out[rank_] = D;
   if (out_layout != nullptr) p.out_layout = *out_layout;
   else p.out_layout.ld = g.N;
-  const char* why = nullptr;
-  check_launch(launch_fused(g, p, stream, &why), why, "gemm_reducescatter");
+  launch(g, p, stream, "gemm_reducescatter");
   ++calls_;
 }
 
@@ -436,6 +434,11 @@ void FusedEngine::gathered_gemm(const void* const* src_for, const long long* byt
                                 const char* op, cudaStream_t stream, size_t mc_slot_offset, const void* a_own,
                                 int own_rows) {
   NvtxRange range(op);
+  for (int r = 0; r < world_; ++r) {
+    if (bytes_for[r] > 0 && !aligned16(src_for[r])) {
+      throw std::runtime_error(std::string(op) + ": the rows of A must be 16-byte aligned");
+    }
+  }
   const TileConfig tc = algo_config(algo);
   const int set = static_cast<int>(calls_ & 1ull);
   check(cudaMemsetAsync(flag_ptr(rank_, set ^ 1), 0, kFlagWords * 4, stream), "cudaMemsetAsync(counters)");
@@ -483,8 +486,7 @@ void FusedEngine::gathered_gemm(const void* const* src_for, const long long* byt
     p.ag_mc_dst = static_cast<char*>(heap_.mc(ws_.stage[set])) + mc_slot_offset;
     p.ag_mc_flag = static_cast<uint32_t*>(heap_.mc(ws_.flags[set])) + kFlagAReady + rank_;
   }
-  const char* why = nullptr;
-  check_launch(launch_fused(g, p, stream, &why), why, op);
+  launch(g, p, stream, op);
   ++calls_;
 }
 

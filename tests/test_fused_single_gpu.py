@@ -308,6 +308,43 @@ def test_compat_overlap_result_at_any_element(offset):
     assert bool((buf[:offset] == 7).all()) and bool((buf[offset + M * N:] == 7).all())
 
 
+def test_addresses_are_checked_on_the_host_before_any_launch():
+    # the kernel moves 16 bytes at a time: whatever starts between two such boundaries is refused with a message
+    M, N, K = 256, 512, 64
+    A, B, W = make_inputs(M, N, K, torch.float16)
+    impl = make_impl()
+
+    def off(rows, cols):
+        return torch.zeros(rows * cols + 8, device="cuda", dtype=torch.float16)[1:1 + rows * cols].view(rows, cols)
+
+    C, O, w = torch.empty(M, N, device="cuda", dtype=torch.float16), off(M, N), off(1, N).view(N)
+    half = torch.empty(M, N // 2, device="cuda", dtype=torch.float16)
+    mlen = torch.tensor([[M]], dtype=torch.int32)
+    bad = [
+        lambda: impl.cutlass_gemm(A, B, O, 0),
+        lambda: impl.gemm_swiglu(A, B, off(M, N // 2), 8),
+        lambda: impl.gemm_rmsnorm(A, B, O, C, W, 1e-5, 0),
+        lambda: impl.gemm_rmsnorm(A, B, C, O, W, 1e-5, 0),
+        lambda: impl.gemm_rmsnorm(A, B, C, torch.empty_like(C), w, 1e-5, 0),
+        lambda: impl.gemm_allreduce_fused(A, B, w, 1e-5, 0),
+        lambda: impl.gemm_reducescatter_fused(A, B, O, None, 1e-5, 0, False),
+        lambda: impl.gemm_reducescatter_fused(A, B, O, W, 1e-5, 0, False),
+        lambda: impl.allgather_gemm(A, B, O, 0),
+        lambda: impl.allgather_gemm(off(M, K), B, C, 0),
+        lambda: impl.a2a_dispatch_gemm(A, B, O, mlen, 0),
+        lambda: impl.a2a_dispatch_gemm(off(M, K), B, C, mlen, 0),
+    ]
+    for i, call in enumerate(bad):
+        with pytest.raises(RuntimeError, match="16-byte aligned"):
+            call()
+            pytest.fail(f"call {i} was accepted")
+    impl.gemm_swiglu(A, B, half, 8)                   # and nothing was broken on the way
+    impl.allgather_gemm(A, B, C, 0)
+    torch.cuda.synchronize()
+    impl.check_status()
+    assert (C.float() - A.float() @ B.float().t()).abs().max().item() < 0.1
+
+
 def test_index_arrays_are_checked_on_the_host_before_any_launch():
     M, N, K, algo = 256, 512, 64, 0
     A, B, W = make_inputs(M, N, K, torch.float16)
