@@ -88,13 +88,15 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t
   constexpr bool KEEP = CPT <= (ADD ? 1 : 2);
   const uint4* weights = reinterpret_cast<const uint4*>(w);
   uint4 v[CPT], a[ADD ? CPT : 1], g[KEEP ? CPT : 1];
-  int row = blockIdx.x;
+  // unsigned: the last step of a CTA may pass the largest int (rows of 8 values can be that many)
+  const unsigned n_rows = rows;
+  unsigned row = blockIdx.x;
   load(row, v, a);
   if constexpr (KEEP) {
 #pragma unroll
     for (int k = 0; k < CPT; ++k) g[k] = __ldg(weights + min(static_cast<int>(threadIdx.x + k * blockDim.x), n_chunks - 1));
   }
-  for (int par = 0; row < rows; par ^= 1) {
+  for (int par = 0; row < n_rows; par ^= 1) {
     float ssq = 0.f;
     if constexpr (ADD) {
       uint4* dst = reinterpret_cast<uint4*>(sum + static_cast<long long>(row) * dim);
@@ -109,9 +111,9 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t
     for (int k = 0; k < CPT; ++k) {
       ssq += static_cast<int>(threadIdx.x + k * blockDim.x) < n_chunks ? sum_squares<BF16>(v[k]) : 0.f;
     }
-    const int next = row + gridDim.x;
+    const unsigned next = row + gridDim.x;
     uint4 nv[CPT];
-    if (next < rows) load(next, nv, a);
+    if (next < n_rows) load(next, nv, a);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
     if (warps > 1) {

@@ -413,6 +413,23 @@ def test_rmsnorm_thread_shapes(rows, dim):
     assert torch.equal(x, o)
 
 
+def test_rmsnorm_of_the_most_rows():
+    # the row numbers of the last step of most CTAs lie past the largest int; in place, 34 GB
+    rows = 2 ** 31 - 1
+    if torch.cuda.mem_get_info()[0] < 40 * 2 ** 30:
+        pytest.skip("needs 34 GB of device memory")
+    x = torch.full((rows, 8), 3.0, device="cuda", dtype=torch.float16)
+    w = torch.arange(1, 9, device="cuda", dtype=torch.float16)
+    torch.ops.flashoverlap_op.rmsnorm(x, x, w, 1e-6)
+    torch.cuda.synchronize()
+    # equal values normalise to one (9 + 1e-6 rounds to 9 in fp32 up to one ulp, which fp16 does not see)
+    for part in x.view(-1)[:rows // 16 * 128].view(16, -1, 8):
+        assert torch.equal(part.amin(0), w) and torch.equal(part.amax(0), w)
+    assert torch.equal(x[rows // 16 * 16:], w.expand(rows % 16, 8))
+    del x, part
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("rows,dim", [(1, 8), (37, 8000), (600, 4096), (300, 16392), (3, 32776)])
 def test_add_rmsnorm(rows, dim):
     torch.manual_seed(dim)
