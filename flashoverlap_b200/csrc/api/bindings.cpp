@@ -34,6 +34,9 @@ static void reorder_rmsnorm_eps(at::Tensor X, at::Tensor RX, at::Tensor RW, int6
   TORCH_CHECK(RW.is_cuda() && RW.is_contiguous() && RW.numel() == dim, "RW must hold dim values");
   TORCH_CHECK(BM > 0 && BN > 0 && bs % BM == 0 && dim % BN == 0 && BN % 8 == 0 && dim % 8 == 0,
               "need bs % BM == 0, dim % BN == 0, BN % 8 == 0");
+  check_aligned(X, "X");
+  check_aligned(RX, "RX");
+  check_aligned(RW, "RW");
   check_int_tensor(RA, "RA", true);
   const int64_t tiles = (bs / BM) * (dim / BN);
   TORCH_CHECK(RA.numel() == tiles, "RA must have ", tiles, " entries, got ", RA.numel());
@@ -74,6 +77,9 @@ static void rmsnorm_op(at::Tensor X, at::Tensor O, at::Tensor RW, double eps) {
   TORCH_CHECK(O.sizes() == X.sizes(), "O must have the shape of X");
   TORCH_CHECK(RW.is_cuda() && RW.is_contiguous() && RW.numel() == X.size(1), "RW must hold dim values");
   TORCH_CHECK(X.size(1) % 8 == 0, "dim must be a multiple of 8");
+  check_aligned(X, "X");
+  check_aligned(O, "O");
+  check_aligned(RW, "RW");
   c10::cuda::CUDAGuard guard(X.device());
   cudaError_t e = launch_rmsnorm(X.data_ptr(), O.data_ptr(), RW.data_ptr(), static_cast<int>(X.size(0)),
                                  static_cast<int>(X.size(1)), static_cast<float>(eps), dt,
@@ -95,9 +101,11 @@ static void add_rmsnorm_op(at::Tensor X, at::Tensor R, at::Tensor S, at::Tensor 
   TORCH_CHECK(RW.is_cuda() && RW.is_contiguous() && RW.numel() == X.size(1) && RW.scalar_type() == X.scalar_type(),
               "RW must hold dim values of X's dtype");
   TORCH_CHECK(X.size(1) % 8 == 0, "dim must be a multiple of 8");
-  for (const at::Tensor* t : {&X, &R, &S, &O, &RW}) {
-    TORCH_CHECK(reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "tensors must be 16-byte aligned");
-  }
+  check_aligned(X, "X");
+  check_aligned(R, "R");
+  check_aligned(S, "S");
+  check_aligned(O, "O");
+  check_aligned(RW, "RW");
   c10::cuda::CUDAGuard guard(X.device());
   cudaError_t e = launch_add_rmsnorm(X.data_ptr(), R.data_ptr(), S.data_ptr(), O.data_ptr(), RW.data_ptr(),
                                      static_cast<int>(X.size(0)), static_cast<int>(X.size(1)), static_cast<float>(eps),

@@ -413,6 +413,20 @@ def test_rmsnorm_thread_shapes(rows, dim):
     assert torch.equal(x, o)
 
 
+def test_rmsnorm_addresses_are_checked_on_the_host():
+    op = torch.ops.flashoverlap_op
+    rows, dim = 128, 256
+    good = torch.ones(rows, dim, device="cuda", dtype=torch.float16)
+    odd = torch.ones(rows * dim + 8, device="cuda", dtype=torch.float16)[3:3 + rows * dim].view(rows, dim)
+    w, w_odd = good[0].clone(), odd[0]
+    RA = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for x, o, g in ((odd, good, w), (good, odd, w), (good, good, w_odd)):
+        for call in (lambda: op.rmsnorm(x, o, g, 1e-5), lambda: op.reorder_rmsnorm_eps(x, o, g, rows, dim, 1, RA, 1e-5),
+                     lambda: op.add_rmsnorm(x, good, good, o, g, 1e-5)):
+            with pytest.raises(RuntimeError, match="16-byte aligned"):
+                call()
+
+
 def test_rmsnorm_of_the_most_rows():
     # the row numbers of the last step of most CTAs lie past the largest int; in place, 34 GB
     rows = 2 ** 31 - 1
