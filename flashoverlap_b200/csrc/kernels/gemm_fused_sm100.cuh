@@ -1266,8 +1266,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     // ===================== teardown of the GEMM phase (GEMM warps only) =====================
     __syncwarp();
     ptx::tc_fence_before_sync();
-    ptx::named_barrier_sync(8, kGemmThreads);
     if constexpr (CTAS == 2) {
+      ptx::named_barrier_sync(8, kGemmThreads);
       // The partner may still read this CTA's operands or signal its barriers:
       // each CTA tells the other that its GEMM warps are done and waits (bounded)
       // to hear the same.
@@ -1278,8 +1278,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
           *abort_flag = 1;
         }
       }
-      ptx::named_barrier_sync(8, kGemmThreads);
     }
+    // One answer for all GEMM warps: the communication warps may raise the flag at this very moment, and the warps of a
+    // row group must either all join the reduce phase, whose barriers have no deadline, or none.  (A warp that gave up
+    // above sees its own store, so a failure of the GEMM phase is always in the answer.)
+    const bool gave_up = ptx::named_barrier_or(8, kGemmThreads, *abort_flag != 0);
     if (warp == 2) {
       ptx::tc_fence_after_sync();
       if constexpr (CTAS == 2) ptx::tmem_dealloc_pair(tmem_base, T::TMEM_COLS);
@@ -1298,7 +1301,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       }
       tr[3] = static_cast<unsigned long long>(mine);
     }
-    if (!p.reduce || *abort_flag) return;
+    if (!p.reduce || gave_up) return;
     // out of tiles: the GEMM warps join the reduce phase as two more row groups
     group = 1 + warp / kGroupWarps;  // warps 0-3 -> group 1, warps 4-7 -> group 2
     wg = warp % kGroupWarps;
