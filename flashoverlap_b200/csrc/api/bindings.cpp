@@ -140,6 +140,20 @@ static std::vector<int64_t> tile_walk_op(int64_t TM, int64_t TN, int64_t raster_
   return out;
 }
 
+// The tile configuration that a one-rank GEMM which names `algo` runs on `ctas` CTAs (0 = all SMs of the device).  For
+// tests and for reasoning about a call's time; needs no GPU when `ctas` is given.
+static int64_t planned_algo_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu) {
+  TORCH_CHECK(M > 0 && N > 0 && K > 0 && algo >= 0 && algo < kNumAlgos && ctas >= 0, "planned_algo: bad arguments");
+  GemmOperands g{};
+  g.M = static_cast<int>(M);
+  g.N = static_cast<int>(N);
+  g.K = static_cast<int>(K);
+  g.algo = static_cast<int>(algo);
+  g.any_tile = 1;
+  g.glu = glu ? 1 : 0;
+  return plan_algo(g, ctas > 0 ? static_cast<int>(ctas) : device_sm_count());
+}
+
 }  // namespace fo
 
 TORCH_LIBRARY(flashoverlap_class, m) {
@@ -208,6 +222,8 @@ TORCH_LIBRARY(flashoverlap_class, m) {
       .def("set_timeout_ms", &OverlapImpl::SetTimeoutMs)
       .def("set_sm_count", &OverlapImpl::SetSmCount)
       .def("set_raster_group", &OverlapImpl::SetRasterGroup)
+      .def("set_keep_tile", &OverlapImpl::SetKeepTile)
+      .def("last_algo", &OverlapImpl::LastAlgo)
       .def("set_l2_hints", &OverlapImpl::SetL2Hints)
       .def("set_raster_taper", &OverlapImpl::SetRasterTaper)
       .def("set_phase_trace", &OverlapImpl::SetPhaseTrace)
@@ -228,4 +244,5 @@ TORCH_LIBRARY(flashoverlap_op, m) {
   m.def("rmsnorm", &fo::rmsnorm_op);
   m.def("add_rmsnorm", &fo::add_rmsnorm_op);
   m.def("tile_walk", &fo::tile_walk_op);
+  m.def("planned_algo", &fo::planned_algo_op);
 }

@@ -685,6 +685,8 @@ void OverlapImpl::SetTimeoutMs(int64_t ms) {
 void OverlapImpl::SetSmCount(int64_t n) { engine_.set_sm_count(static_cast<int>(n)); }
 void OverlapImpl::SetL2Hints(bool on) { engine_.set_l2_hints(on); }
 void OverlapImpl::SetRasterTaper(bool on) { engine_.set_raster_taper(on); }
+void OverlapImpl::SetKeepTile(bool on) { engine_.set_keep_tile(on); }
+int64_t OverlapImpl::LastAlgo() { return engine_.last_algo(); }
 void OverlapImpl::SetRasterGroup(int64_t g) { engine_.set_raster_group(static_cast<int>(g)); }
 void OverlapImpl::SetPhaseTrace(at::Tensor buf) {
   if (buf.numel() == 0) {

@@ -122,6 +122,10 @@ class OverlapImpl : public torch::CustomClassHolder {
   void SetTimeoutMs(int64_t ms);
   void SetSmCount(int64_t n);
   void SetRasterGroup(int64_t g);
+  // Run the tile configuration a call names, also on one rank (see FusedEngine::set_keep_tile).
+  void SetKeepTile(bool on);
+  // Tile configuration that the last launch ran (-1: none yet).
+  int64_t LastAlgo();
   // L2 eviction hints on the GEMM's operand loads (default off).
   void SetL2Hints(bool on);
   // Shrinking last raster groups in operations with a reduce phase (default on).

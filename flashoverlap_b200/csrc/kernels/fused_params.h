@@ -107,6 +107,7 @@ struct alignas(64) FusedParams {
 
   int M, N, K;
   int TM, TN;        // tile grid; the last tile row and column may reach past M and N (whole blocks of 128 rows, 64 columns)
+  int algo;          // tile configuration that runs (index of the table), for the host
   int trace_cols;    // phase trace: columns that count as one tile (those of the tile the caller named)
   int raster_group;  // tile rows walked column-major together (L2 reuse of B)
   int raster_taper;  // 1 = the last groups shrink by halves so that little is left to communicate after the last tile

@@ -154,6 +154,7 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
   const int sms = device_sm_count();
   if (grid > sms) grid = sms;  // every CTA must be resident: CTAs wait on one another's output
   const int algo = plan_algo(g, grid);
+  p.algo = algo;
   p.trace_cols = tc.bn;
   tc = kAlgoTable[algo];
   // every CTA stages 128 rows of A and (for a CTA pair) half of the B tile, 64 K-values per box

@@ -47,8 +47,9 @@ struct GemmOperands {
 int plan_algo(const GemmOperands& g, int ctas);
 
 // Fills p.tmA / p.tmB / shape fields from `g`, validates shapes, launches.
-// Everything else in `p` must already be set by the caller.  Returns
-// cudaSuccess or an error; *why (if not null) receives a static message.
+// Everything else in `p` must already be set by the caller; p.algo says
+// afterwards which configuration runs.  Returns cudaSuccess or an error; *why
+// (if not null) receives a static message.
 cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t stream, const char** why);
 
 // One-time set-up of an instance on the current device (its shared-memory

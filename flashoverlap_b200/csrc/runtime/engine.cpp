@@ -21,16 +21,17 @@ void check(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw std::runtime_error(cuda_error_string(e, what));
 }
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
-// Launches the fused kernel; throws with the launcher's reason when it refuses the call.
-void launch(const GemmOperands& g, FusedParams& p, cudaStream_t stream, const char* op) {
+}  // namespace
+
+void FusedEngine::launch(const GemmOperands& g, FusedParams& p, cudaStream_t stream, const char* op) {
   const char* why = nullptr;
   const cudaError_t e = launch_fused(g, p, stream, &why);
   if (e != cudaSuccess) {
     std::string msg = std::string(op) + ": " + (why && *why ? why : "launch failed");
     throw std::runtime_error(cuda_error_string(e, msg.c_str()));
   }
+  last_algo_ = p.algo;
 }
-}  // namespace
 
 FusedEngine::~FusedEngine() {
   if (status_dev_ != nullptr) cudaFree(status_dev_);
@@ -211,7 +212,7 @@ void FusedEngine::gemm(const GemmOperands& g_in, void* C, const OutLayout* layou
   if (layout != nullptr) p.epi_layout = *layout;
   else p.epi_layout.ld = g.glu ? g.N / 2 : g.N;
   p.clear_words = clear_words;
-  g.any_tile = sig == nullptr && (layout == nullptr || layout->row_map == nullptr) ? 1 : 0;
+  g.any_tile = tile_is_free() && sig == nullptr && (layout == nullptr || layout->row_map == nullptr) ? 1 : 0;
   if (p.raster_group == 0) p.raster_group = local_group(g, false);
   launch(g, p, stream, "gemm");
 }
@@ -247,7 +248,7 @@ void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* ou
   if (row_trace_ != nullptr && g.M <= row_trace_rows_) p.row_trace = row_trace_;
   p.stage = scratch;
   p.ssq = ssq;
-  g.any_tile = 1;
+  g.any_tile = tile_is_free() ? 1 : 0;
   p.flag_target = static_cast<uint32_t>(g.N / tc.bn);
   p.norm = norm.gamma != nullptr;
   p.gamma = norm.gamma;
@@ -330,7 +331,7 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
   if (world_ == 1 && p.norm) {
     p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
     p.drop_stage = drop_stage(g) ? 1 : 0;
-    g.any_tile = 1;
+    g.any_tile = tile_is_free() ? 1 : 0;
   }
   // with one rank there is nobody to deliver to: rows go to the result buffer like a reduce-scatter's
   p.bcast = world_ > 1 ? 1 : 0;
@@ -413,7 +414,7 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
   if (world_ == 1 && p.norm) {
     p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
     p.drop_stage = drop_stage(g) ? 1 : 0;
-    g.any_tile = 1;
+    g.any_tile = tile_is_free() ? 1 : 0;
   }
   p.bcast = 0;
   p.job_counter = flag_ptr(rank_, set) + kFlagJob;

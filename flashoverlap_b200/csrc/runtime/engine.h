@@ -56,7 +56,14 @@ class FusedEngine {
 
   void set_timeout_ms(long long ms) { timeout_ns_ = static_cast<unsigned long long>(ms) * 1000000ull; }
   void set_sm_count(int n) { sm_count_ = n; }
+  // Tile rows walked together; 0 (default) = chosen per operation.  A group that the caller sets counts rows of the tile
+  // that the call names, so that tile runs.
   void set_raster_group(int g) { raster_group_ = g; }
+  // One rank: every call runs the tile configuration it names instead of the one with the least expected time.  For
+  // searches and profiles, whose result is a configuration that several ranks run as named.
+  void set_keep_tile(bool on) { keep_tile_ = on; }
+  // Tile configuration that the last launch ran (-1: none yet).
+  int last_algo() const { return last_algo_; }
   // L2 eviction hints on the operand loads (A row panel kept, B streamed); off by default
   // (they help only the largest K, measured).
   void set_l2_hints(bool on) { l2_hints_ = on; }
@@ -213,6 +220,11 @@ class FusedEngine {
   unsigned long long timeout_ns_ = 20000000000ull;
   int sm_count_ = 0;
   int raster_group_ = 0;  // 0 = choose per operation
+  bool keep_tile_ = false;
+  int last_algo_ = -1;
+  bool tile_is_free() const { return !keep_tile_ && raster_group_ == 0; }
+  // Launches the fused kernel; throws with the launcher's reason when it refuses the call.
+  void launch(const GemmOperands& g, FusedParams& p, cudaStream_t stream, const char* op);
   bool l2_hints_ = false;
   bool raster_taper_ = true;
   int nvls_ar_ = -1;  // -1 = by group size, 0 = off, 1 = on

@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import os
 import sys
+from contextlib import contextmanager
 from typing import Callable, List, Optional, Sequence, Tuple
 
 import torch
@@ -66,6 +67,21 @@ def usable_algos(M: int, N: int) -> List[int]:
 RASTER_CHOICES = (1, 2, 4, 8)
 
 
+@contextmanager
+def named_tile(impl, raster_group: int = 0):
+    """Launches inside run exactly the tile configuration they name (and this
+    raster group).  On one GPU a launch otherwise takes the configuration with
+    the least expected time, so that times taken per ``Algo`` would say nothing
+    about the ``Algo`` that several ranks run."""
+    impl.set_keep_tile(True)
+    impl.set_raster_group(raster_group)
+    try:
+        yield impl
+    finally:
+        impl.set_raster_group(0)
+        impl.set_keep_tile(False)
+
+
 def profile_gemm(impl, M: int, N: int, K: int, dtype=torch.float16, warmup: int = 10, reps: int = 100,
                  keep: int = 10, rasters: Sequence[int] = (), with_raster_table: bool = False):
     """Times every tile configuration that fits the shape and returns the
@@ -81,11 +97,8 @@ def profile_gemm(impl, M: int, N: int, K: int, dtype=torch.float16, warmup: int 
     for algo in usable_algos(M, N):
         best = None
         for rg in (tuple(rasters) or (0,)):
-            impl.set_raster_group(rg)
-            try:
+            with named_tile(impl, rg):
                 ms = mean_time_ms(lambda: impl.cutlass_gemm(A, B, C, algo), warmup, reps)
-            finally:
-                impl.set_raster_group(0)
             table[(algo, rg)] = ms
             best = ms if best is None else min(best, ms)
             dbg(f"profile_gemm: algo {algo} {ALGO_TILES[algo]} raster {rg}: {ms:.4f} ms")
@@ -179,7 +192,6 @@ def perf_running(impl, M: int, N: int, K: int, BM: int, BN: int, algo: int, cseg
     RA = reorder_indices(tiles, hint, device="cuda").reshape(tm, tn)
     D = torch.empty((M // ws, N), dtype=dtype, device="cuda") if comm_op == "reduce_scatter" else None
     RE = generate_row_mapping(M, N, BM, BN, list(cseg), ws, device="cuda") if comm_op == "reduce_scatter" else None
-    impl.set_raster_group(raster_group)
     if len(cseg) == 1:
         if comm_op == "all_reduce":
             fn = lambda: impl.gemm_allreduce(A, B, C, algo)  # noqa: E731
@@ -195,11 +207,9 @@ def perf_running(impl, M: int, N: int, K: int, BM: int, BN: int, algo: int, cseg
     else:
         fn = lambda: impl.gemm_reducescatter_overlap(A, B, C, D, MM, RA, RE, 1, cseg_cpu, cseg_gpu, algo,  # noqa: E731
                                                      False)
-    try:
+    with named_tile(impl, raster_group):
         ms = mean_time_ms(fn, warmup, reps)
         impl.check_status()
-    finally:
-        impl.set_raster_group(0)
     return ms
 
 
@@ -270,7 +280,8 @@ def pick_algo_by_timing(run: Callable[[int], None], algos: Sequence[int], warmup
     returns ``(best algo, [(algo, ms), ...])``: the stage-1 search of the
     tuner for operations whose best tile depends on the ranks' arrival pattern
     (reference: tune/profile_config.py times every instance and keeps the
-    fastest)."""
+    fastest).  For several ranks, which run the named tile; on one rank ``run``
+    pins it (:func:`named_tile`)."""
     timed = []
     for a in algos:
         timed.append((a, mean_time_ms(lambda: run(a), warmup, reps, flush=True)))
@@ -297,7 +308,8 @@ def measure_row_us(impl, N: int, comm_op: str, dtype=torch.float16, algo: int = 
         fused = lambda: impl.gemm_allreduce_fused(A, B, W, 1e-5, algo)  # noqa: E731
     else:
         fused = lambda: impl.gemm_reducescatter_fused(A, B, D, W, 1e-5, algo, False)  # noqa: E731
-    t_fused = mean_time_ms(fused, warmup, reps, flush=True)
-    t_gemm = mean_time_ms(lambda: impl.cutlass_gemm(A, B, C, algo), warmup, reps, flush=True)
+    with named_tile(impl):
+        t_fused = mean_time_ms(fused, warmup, reps, flush=True)
+        t_gemm = mean_time_ms(lambda: impl.cutlass_gemm(A, B, C, algo), warmup, reps, flush=True)
     rows = M // ws
     return max((t_fused - t_gemm) * 1e3, 1.0) * groups * sms / rows

@@ -15,7 +15,7 @@ import torch  # noqa: E402
 
 from flashoverlap_b200.cli import DTYPES  # noqa: E402
 
-from flashoverlap_b200.tune.runtime import make_inputs, mean_time_ms, usable_algos
+from flashoverlap_b200.tune.runtime import make_inputs, mean_time_ms, named_tile, usable_algos
 from flashoverlap_b200.utils import config as cfg
 
 
@@ -43,10 +43,9 @@ def main():
                 t_vendor = mean_time_ms(lambda: base.cublas_gemm(A, B, C), 10, args.reps)
                 timed = []
                 for rg in args.rasters:
-                    impl.set_raster_group(rg)
-                    timed += [(mean_time_ms(lambda a=a: impl.cutlass_gemm(A, B, C, a), 10, args.reps), a, rg)
-                              for a in usable_algos(M, N)]
-                impl.set_raster_group(0)
+                    with named_tile(impl, rg):
+                        timed += [(mean_time_ms(lambda a=a: impl.cutlass_gemm(A, B, C, a), 10, args.reps), a, rg)
+                                  for a in usable_algos(M, N)]
                 best = min(timed)
                 tf = 2.0 * M * N * K / (best[0] * 1e-3) / 1e12
                 tile = cfg.ALGO_TILES[best[1]]

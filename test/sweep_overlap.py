@@ -77,6 +77,7 @@ def main():
     # what one row of N values costs a row group in the reduce phase (measured once per N and collective)
     row_us = {(op, N): measure_row_us(impl, N, op, dt, algo=args.algos[0]) for op in ("all_reduce", "reduce_scatter")
               for N in args.n_list}
+    impl.set_keep_tile(True)  # the sweep compares tile configurations, also on one GPU
     rows_md = []
     if rank == 0:
         print(f"TP={ws} {args.dtype}; measured link {link_gbs:.0f} GB/s per direction ({link_kind}); row time "

@@ -61,6 +61,7 @@ def main(argv=None, rendezvous_retries=0):
     cseg = [(M // BM) * (N // BN)] if args.single_seg else sol["cSeg"]
     impl, base = make_overlap_impl(), make_baseline_impl()
     impl.set_raster_group(int(sol.get("raster_group", 0)))
+    impl.set_keep_tile("search" in sol)  # a searched tile runs as it was timed, also on one GPU
     A, B, C = make_inputs(M, N, K, dtype)
     W = torch.empty(N, dtype=dtype, device="cuda").normal_(1.0, 0.1)
     D = torch.empty((M // ws, N), dtype=dtype, device="cuda")

@@ -18,8 +18,9 @@ OVERLAP_OWN = ["gemm_allreduce_fused", "gemm_reducescatter_fused", "allgather_ge
                "set_raster_group", "set_raster_taper", "set_l2_hints", "set_use_nvls", "allreduce_uses_nvls",
                "set_allgather_multicast", "set_phase_trace", "set_row_trace", "status", "status_string", "check_status",
                "reset", "transport", "num_algos", "algo_tile", "p2p_push", "p2p_push_bulk", "multimem_bench",
-               "detach_symmetric"]
-OPS = ["generate_nccl_id", "generate_mccl_id", "reorder_rmsnorm", "reorder_rmsnorm_eps", "rmsnorm", "tile_walk"]
+               "detach_symmetric", "set_keep_tile", "last_algo", "gemm_swiglu"]
+OPS = ["generate_nccl_id", "generate_mccl_id", "reorder_rmsnorm", "reorder_rmsnorm_eps", "rmsnorm", "add_rmsnorm", "tile_walk",
+       "planned_algo"]
 
 
 def test_baseline_class_has_the_reference_methods():
@@ -39,6 +40,18 @@ def test_ops_are_registered():
     assert not missing, missing
     ident = torch.ops.flashoverlap_op.generate_nccl_id()
     assert len(ident) == 16          # the reference's 128-byte id as 16 int64 (src/mccl_utils.cpp:7-14)
+
+
+def test_planned_tile_needs_no_gpu():
+    from flashoverlap_b200.utils.config import ALGO_TILES
+
+    plan = torch.ops.flashoverlap_op.planned_algo
+    for m, n, k in ((128, 64, 8), (1024, 2048, 4096), (4096, 8192, 8192), (16384, 14336, 28672)):
+        for algo in range(len(ALGO_TILES)):
+            assert 0 <= plan(m, n, k, algo, 148, False) < len(ALGO_TILES)
+            assert ALGO_TILES[plan(m, n, k, algo, 1, False)][0] <= ALGO_TILES[algo][0]   # no pair on a single CTA
+        bm, bn, _ = ALGO_TILES[plan(m, n, k, 8, 148, True)]
+        assert bm == 256 and bn >= 128                                               # gate and up side by side
 
 
 def test_tile_table_matches_the_python_copy():

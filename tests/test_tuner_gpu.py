@@ -8,7 +8,7 @@ import flashoverlap_b200  # noqa: F401
 from flashoverlap_b200.models import OverlapRowParallelLayer, ReorderRMSNorm
 from flashoverlap_b200.parallel import make_overlap_impl
 from flashoverlap_b200.tune import search
-from flashoverlap_b200.tune.runtime import compute_hint, profile_gemm
+from flashoverlap_b200.tune.runtime import compute_hint, measure_row_us, perf_running, profile_gemm
 from flashoverlap_b200.utils import config as cfg
 
 pytestmark = pytest.mark.gpu
@@ -58,6 +58,53 @@ def test_profile_hint_search_and_use(tmp_path):
     ref = x.float() @ layer.weight.float().t()
     ref = ref * torch.rsqrt(ref.pow(2).mean(-1, keepdim=True) + 1e-5)
     assert (y.float() - ref).abs().max().item() < 2e-2
+    impl.check_status()
+
+
+class Recorder:
+    """Passes calls on to an OverlapImpl and notes, for those that launch the kernel, which tile configuration was named
+    (the position of the argument) and which one ran."""
+    NAMED = {"cutlass_gemm": 3, "gemm_allreduce_fused": 4, "gemm_reducescatter_fused": 5, "gemm_allreduce_overlap": 8,
+             "gemm_reducescatter_overlap": 10, "gemm_allreduce": 3, "gemm_reducescatter": 4}
+
+    def __init__(self, impl):
+        self.impl, self.ran = impl, []
+
+    def __getattr__(self, name):
+        method = getattr(self.impl, name)
+        if name not in self.NAMED:
+            return method
+
+        def call(*args):
+            out = method(*args)
+            self.ran.append((name, args[self.NAMED[name]], self.impl.last_algo()))
+            return out
+        return call
+
+
+def test_searches_time_the_tile_they_name():
+    # on one rank a plain call runs the configuration with the least expected time, whatever it names; a search must not
+    M, N, K = 1024, 2048, 4096
+    impl = make_overlap_impl(timeout_ms=3000)
+    rec = Recorder(impl)
+    profile_gemm(rec, M, N, K, torch.float16, warmup=1, reps=2, rasters=(0, 2))
+    for op in ("all_reduce", "reduce_scatter"):
+        measure_row_us(rec, 2048, op, torch.float16, algo=4, M=1024, warmup=1, reps=1)
+        for cseg in ([63, 1], [64]):
+            perf_running(rec, M, N, K, 128, 256, 0, cseg, [], op, warmup=1, reps=1, raster_group=0)
+    assert {a for name, a, _ in rec.ran if name == "cutlass_gemm"} == set(range(len(cfg.ALGO_TILES)))
+    assert {name for name, _, _ in rec.ran} == set(Recorder.NAMED)
+    assert all(asked == ran for _, asked, ran in rec.ran), rec.ran
+    # and afterwards the launch chooses again
+    A = torch.randn(M, K, device="cuda", dtype=torch.float16)
+    B = torch.randn(N, K, device="cuda", dtype=torch.float16)
+    C = torch.empty(M, N, device="cuda", dtype=torch.float16)
+    planned = [torch.ops.flashoverlap_op.planned_algo(M, N, K, a, 0, False) for a in range(len(cfg.ALGO_TILES))]
+    for a, p in enumerate(planned):
+        impl.cutlass_gemm(A, B, C, a)
+        assert impl.last_algo() == p
+    assert planned != list(range(len(cfg.ALGO_TILES)))
+    torch.cuda.synchronize()
     impl.check_status()
 
 

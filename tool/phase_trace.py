@@ -90,6 +90,7 @@ def main():
     args = ap.parse_args()
     rank, ws = start()
     impl = make_overlap_impl()
+    impl.set_keep_tile(True)  # the traces are those of the named tile, also on one GPU
     sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
     lines = []
     for name, op, M, N, Kt, dtn in SHAPES:

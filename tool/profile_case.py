@@ -29,6 +29,7 @@ def main():
     ap.add_argument("k", type=int, nargs="?", default=1024)
     ap.add_argument("--algo", type=int, default=3)
     ap.add_argument("--raster", type=int, default=0)
+    ap.add_argument("--keep-tile", action="store_true", help="run --algo itself, not the tile the launch would choose")
     ap.add_argument("--dtype", default="bfloat16", choices=sorted(DTYPES))
     ap.add_argument("--launches", type=int, default=3)
     args = ap.parse_args()
@@ -39,6 +40,7 @@ def main():
     impl.cutlass_init()
     impl.set_timeout_ms(3000)
     impl.set_raster_group(args.raster)
+    impl.set_keep_tile(args.keep_tile)
     M, N, K = args.m, args.n, args.k
     A = (torch.randn(M, K, device="cuda") / K ** 0.5).to(dt)
     B = (torch.randn(N, K, device="cuda") / K ** 0.5).to(dt)

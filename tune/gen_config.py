@@ -18,7 +18,7 @@ import torch  # noqa: E402
 
 from flashoverlap_b200.cli import DTYPES  # noqa: E402
 
-from flashoverlap_b200.tune.runtime import make_inputs, mean_time_ms
+from flashoverlap_b200.tune.runtime import make_inputs, mean_time_ms, named_tile
 from flashoverlap_b200.utils import config as cfg
 
 
@@ -74,8 +74,9 @@ def main():
     impl = torch.classes.flashoverlap_class.OverlapImpl()
     impl.cutlass_init()
     A, B, C = make_inputs(args.m, args.n, args.k, DTYPES[args.dtype])
-    timed = sorted((mean_time_ms(lambda a=a: impl.cutlass_gemm(A, B, C, a), 10, 100), a) for a in algos
-                   if args.m % cfg.ALGO_TILES[a][0] == 0 and args.n % cfg.ALGO_TILES[a][1] == 0)
+    with named_tile(impl):
+        timed = sorted((mean_time_ms(lambda a=a: impl.cutlass_gemm(A, B, C, a), 10, 100), a) for a in algos
+                       if args.m % cfg.ALGO_TILES[a][0] == 0 and args.n % cfg.ALGO_TILES[a][1] == 0)
     f = cfg.save_stage1(args.m, args.n, args.k, [cfg.ALGO_TILES[a][0] for _, a in timed],
                         [cfg.ALGO_TILES[a][1] for _, a in timed], [t for t, _ in timed], [a for _, a in timed],
                         args.config_dir)
