@@ -52,7 +52,11 @@ class OverlapRowParallelLayer(nn.Module):
     (``BM``, ``BN``, ``Algo``, ``hint``, ``cSeg``); ``nccl_id`` the 16-word id
     broadcast from rank 0.  The all-reduce output is in tile-reordered layout
     (feed it to :class:`ReorderRMSNorm`); the reduce-scatter output holds this
-    rank's interleaved rows in the same slot order."""
+    rank's interleaved rows in the same slot order.
+
+    ``Algo`` fixes the layout.  A configuration that a search of this library
+    found (it has the key ``search``) is run as it was timed; with any other, one
+    rank takes the tile with the least expected time for the same layout."""
 
     def __init__(self, rank: int, world_size: int, in_features: int, out_features: int, M: int, config: dict,
                  comm_op: str, nccl_id, dtype=torch.float16, device=None):
@@ -66,6 +70,7 @@ class OverlapRowParallelLayer(nn.Module):
         self.overlap_class.nccl_init(rank, world_size, [int(v) for v in nccl_id])
         self.overlap_class.cutlass_init()
         self.overlap_class.overlap_init()
+        self.overlap_class.set_keep_tile("search" in config)
         BM, BN = config["BM"], config["BN"]
         hint, cseg = config["hint"], config["cSeg"]
         tm, tn = div_up(M, BM), div_up(out_features, BN)
@@ -103,8 +108,9 @@ class FusedRowParallelLinear(nn.Module):
 
     ``algo`` and ``raster_group`` are what the tuner searches for a shape
     (``tune/search.py`` stores them as ``Algo`` and ``raster_group`` in the
-    stage-2 JSON; :meth:`from_config` reads them); ``raster_group=0`` leaves the
-    library's default."""
+    stage-2 JSON; :meth:`from_config` reads them).  With a raster group the
+    named tile runs; ``raster_group=0`` leaves the group, and on one rank the
+    tile, to the library."""
 
     def __init__(self, impl, in_features: int, out_features: int, comm_op: str = "all_reduce",
                  norm: bool = False, eps: float = 1e-5, algo: int = 0, interleave: bool = False,

@@ -108,6 +108,36 @@ def test_searches_time_the_tile_they_name():
     impl.check_status()
 
 
+def test_layers_run_a_searched_configuration_as_named():
+    from flashoverlap_b200.models import FusedRowParallelLinear
+
+    M, N, K, algo = 1024, 2048, 4096, 5
+    chosen = torch.ops.flashoverlap_op.planned_algo(M, N, K, algo, 0, False)
+    assert chosen != algo        # a shape at which one rank would take another tile
+    x = torch.randn(M, K, device="cuda", dtype=torch.float16) / K ** 0.5
+    impl = make_overlap_impl(timeout_ms=3000)
+    outs = []
+    for op in ("all_reduce", "reduce_scatter"):
+        for norm in (False, True):
+            for config, ran in (({"Algo": algo, "raster_group": 4, "comm_op": op}, algo),
+                                ({"Algo": algo, "comm_op": op}, chosen)):     # no raster group: not from this search
+                torch.manual_seed(1)
+                layer = FusedRowParallelLinear.from_config(impl, config, K, N, norm=norm)
+                outs.append(layer(x).clone())
+                assert impl.last_algo() == ran
+            assert torch.equal(outs[-1], outs[-2]) or norm      # the tile does not change a product's sums
+            torch.testing.assert_close(outs[-1], outs[-2], rtol=2 ** -9, atol=1e-6)
+    bm, bn, _ = cfg.ALGO_TILES[algo]
+    tiles = (M // bm) * (N // bn)
+    for extra, ran in (({"search": "exhaustive", "raster_group": 2}, algo), ({}, chosen)):
+        config = {"BM": bm, "BN": bn, "Algo": algo, "hint": list(range(tiles)), "cSeg": [tiles], **extra}
+        layer = OverlapRowParallelLayer(0, 1, K, N, M, config, "all_reduce", [0] * 16)
+        layer(x)
+        assert layer.overlap_class.last_algo() == ran
+    torch.cuda.synchronize()
+    impl.check_status()
+
+
 def test_measured_row_time_is_sane():
     from flashoverlap_b200.tune.runtime import gather_algo_candidates, measure_row_us, pick_algo_by_timing
 
