@@ -59,10 +59,15 @@ class TPDecoderBlock(nn.Module):
         hd, h, kv = self.head_dim, self.heads, self.kv_heads
         q, k, v = qkv.split([h * hd, kv * hd, kv * hd], dim=-1)
         q = q.reshape(batch, seq, h, hd).transpose(1, 2)
-        # a key and value head serves h // kv query heads in place (repeating them is two copies of their own)
         k = k.reshape(batch, seq, kv, hd).transpose(1, 2)
         v = v.reshape(batch, seq, kv, hd).transpose(1, 2)
-        o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=h != kv)
+        # Up to 256 values wide, a key and value head serves h // kv query heads in place (1.3 to 2.5 times as fast as
+        # repeating them: 2 x 1024 tokens, 32 heads of 128, 0.078 -> 0.031 ms).  Wider heads have no fused attention
+        # for groups, only the one that stores all scores: 4096 tokens, 8 heads of 512, 1.18 ms repeated, 6.49 in place.
+        grouped = h != kv and hd <= 256
+        if h != kv and not grouped:
+            k, v = k.repeat_interleave(h // kv, dim=1), v.repeat_interleave(h // kv, dim=1)
+        o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=grouped)
         return o.transpose(1, 2).reshape(batch * seq, h * hd).contiguous()
 
     def _mlp_act(self, gu):

@@ -547,6 +547,34 @@ def test_a2a_dispatch_gemm_in_the_place_of_its_rows(rows, K, N):
     assert torch.equal(buf[:rows * N].view(rows, N), want[:rows])
 
 
+@pytest.mark.parametrize("heads,kv_heads", [(16, 16), (16, 4), (4, 2), (2, 1)])
+def test_attention_of_grouped_heads_stores_no_scores(heads, kv_heads):
+    # head widths 128 to 1024: one attention kernel each time, whose memory grows with the tokens and not their square
+    from flashoverlap_b200.models.decoder_block import TPDecoderBlock
+
+    hidden, batch, seq = 2048, 1, 2048
+    block = TPDecoderBlock(make_impl(), hidden, 256, heads, kv_heads, 1e-5, 8, dtype=torch.bfloat16)
+    hd = hidden // heads
+    torch.manual_seed(heads)
+    qkv = torch.randn(batch * seq, (heads + 2 * kv_heads) * hd, device="cuda", dtype=torch.bfloat16)
+    block._attention(qkv, batch, seq)                   # whatever the first call keeps
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    got = block._attention(qkv, batch, seq)
+    used = torch.cuda.max_memory_allocated() - before
+    # the output, its copy, repeated keys and values, each as large as the queries, and as much again for padding
+    assert used <= 8 * batch * seq * hidden * 2, f"{used >> 20} MB"
+    q, k, v = (z.reshape(batch, seq, -1, hd).transpose(1, 2).double()
+               for z in qkv.split([hidden, kv_heads * hd, kv_heads * hd], dim=-1))
+    k, v = (z.repeat_interleave(heads // kv_heads, dim=1) for z in (k, v))
+    mask = torch.ones(seq, seq, dtype=torch.bool, device="cuda").triu(1)
+    want = (q @ k.transpose(-1, -2) / hd ** 0.5).masked_fill(mask, float("-inf")).softmax(-1) @ v
+    want = want.transpose(1, 2).reshape(batch * seq, hidden)
+    # probabilities and results are rounded to 8 bits: each within 2^-8 of values up to the largest one
+    assert (got.double() - want).abs().max().item() <= 2 ** -7 * want.abs().max().item()
+
+
 def test_host_feeder_double_buffers_inputs():
     from flashoverlap_b200.utils.pipeline import HostFeeder
 
