@@ -42,9 +42,11 @@ def test_gemm_rmsnorm_single_kernel(dtype, algo):
     C = torch.empty(M, N, device="cuda", dtype=dtype)
     O = torch.full((M, N), float("nan"), device="cuda", dtype=dtype)
     impl = make_impl()
+    impl.set_keep_tile(True)     # this tile configuration and no other
     impl.gemm_rmsnorm(A, B, C, O, W, 1e-5, algo)
     torch.cuda.synchronize()
     impl.check_status()
+    assert impl.last_algo() == algo
     ref = A.float() @ B.float().t()
     tol = 1e-2 if dtype == torch.float16 else 3e-2
     assert (C.float() - ref).abs().max().item() <= tol * ref.abs().max().item()
@@ -55,9 +57,8 @@ def test_gemm_rmsnorm_single_kernel(dtype, algo):
 
 @pytest.mark.parametrize("N", [512, 2304, 8192, 16384, 16640])
 def test_gemm_rmsnorm_row_widths(N):
-    # rows that fill a fraction of the row group's registers (512), that end inside a
-    # warp's chunk range (2304), that fill them exactly (8192), and wide rows
-    # that take the two-pass path (16384, 16640)
+    # one unit of 512 columns per row (512), several with the last one half empty (2304), as many
+    # weights as shared memory holds (8192), and rows whose weights come from memory (16384, 16640)
     M, K = 256, 128
     A, B, W = make_inputs(M, N, K, torch.float16, seed=N)
     C = torch.empty(M, N, device="cuda", dtype=torch.float16)
@@ -72,7 +73,7 @@ def test_gemm_rmsnorm_row_widths(N):
 
 
 def test_gemm_rmsnorm_more_rows_than_one_wave():
-    # 8192 rows: every row group takes many rows; the GEMM warps join the reduce phase
+    # 8192 rows: every row group takes many units; the GEMM warps join the reduce phase
     M, N, K = 8192, 2048, 256
     A, B, W = make_inputs(M, N, K, torch.bfloat16, seed=21)
     C = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
@@ -197,7 +198,10 @@ def test_world1_allreduce_and_reducescatter(with_norm):
 
 @pytest.mark.parametrize("algo,M,N,K", [
     (2, 384, 2112, 4096), (1, 5504, 3456, 264), (6, 1152, 1408, 2048), (7, 128, 4672, 520), (0, 2432, 2816, 1000),
-    (9, 2304, 8320, 136), (3, 256, 256, 64)])
+    (9, 2304, 8320, 136), (3, 256, 256, 64),
+    # an odd number of 128-row blocks in pairs of them: the second half of the last tile row is empty; 256 columns, 128,
+    # with a last tile column of 192 and of 64, and a staged product that is dropped
+    (0, 2176, 4096, 4096), (0, 2432, 2816, 4096), (2, 384, 6336, 4096), (2, 640, 8256, 4096), (2, 1920, 8384, 2048)])
 def test_gemm_in_another_tile_configuration(algo, M, N, K):
     # one rank: the named configuration says which shapes are accepted, the launch may take a larger tile whose last row
     # or column reaches past the matrix; natural order, tile order and RMSNorm
@@ -207,6 +211,9 @@ def test_gemm_in_another_tile_configuration(algo, M, N, K):
     guard = torch.full((M + 1, N), 7.0, device="cuda", dtype=torch.bfloat16)   # the row after the result
     C = guard[:M]
     impl.cutlass_gemm(A, B, C, algo)
+    assert impl.last_algo() == torch.ops.flashoverlap_op.planned_algo(M, N, K, algo, 0, False)
+    # the cases from 2176 rows on are here for their pair tiles: a planner that decides otherwise needs other shapes
+    assert (ALGO_TILES[impl.last_algo()][0] == 256) == (K >= 2048 and N >= 2816)
     out = impl.gemm_allreduce_fused(A, B, W, 1e-5, algo)
     bm, bn, _ = impl.algo_tile(algo)
     tiles = (M // bm) * (N // bn)
@@ -259,12 +266,14 @@ def test_compat_overlap_api_reordered_layout_and_trace():
     assert (out.float() - want).abs().max().item() <= 1e-2 * want.abs().max().item()
 
 
-@pytest.mark.parametrize("algo,rldn", [(2, 1), (4, 2), (8, 1), (9, 4)])
+@pytest.mark.parametrize("algo,rldn,keep", [(2, 1, False), (4, 2, False), (8, 1, False), (9, 4, False)] +
+                         [(a, (1, 2, 4)[a % 3], True) for a in range(len(ALGO_TILES))])
 @pytest.mark.parametrize("monitor", [False, True])
-def test_compat_overlap_writes_tile_order_in_place(algo, rldn, monitor):
+def test_compat_overlap_writes_tile_order_in_place(algo, rldn, keep, monitor):
     # one rank: the epilogue stores the tile-ordered result itself; tiles of every width, wide view rows, and a result
     # that takes the place of an operand (which then goes through the staging buffer)
     impl = make_impl()
+    impl.set_keep_tile(keep)
     bm, bn, _ = impl.algo_tile(algo)
     M, N, K = 4 * bm, 8 * bn, 8 * bn
     A, B, _ = make_inputs(M, N, K, torch.bfloat16, seed=algo)
@@ -273,6 +282,7 @@ def test_compat_overlap_writes_tile_order_in_place(algo, rldn, monitor):
     MM = torch.zeros((5, 8), dtype=torch.int32, device="cuda")
     C = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
     impl.gemm_allreduce_overlap(A, B, C, MM, RA, rldn, cseg, cseg.cuda(), algo, monitor)
+    assert impl.last_algo() == (algo if keep or monitor else torch.ops.flashoverlap_op.planned_algo(M, N, K, algo, 0, False))
     ref = A.double() @ B.double().t()
     want = to_tile_order(ref.to(torch.bfloat16), bm, bn, RA, rldn)
     torch.cuda.synchronize()
@@ -284,7 +294,7 @@ def test_compat_overlap_writes_tile_order_in_place(algo, rldn, monitor):
     impl.gemm_allreduce_overlap(A2, B, A2, MM, RA, rldn, cseg, cseg.cuda(), algo, False)
     torch.cuda.synchronize()
     impl.check_status()
-    assert torch.equal(A2, C)
+    assert torch.equal(A2, C) and impl.last_algo() == algo
 
 
 @pytest.mark.parametrize("offset", [1, 3, 8])
@@ -511,11 +521,11 @@ def test_a2a_dispatch_gemm_world1():
     assert (C.float() - ref2).abs().max().item() <= 1e-2 * ref2.abs().max().item()
 
 
-@pytest.mark.parametrize("rows", [1, 127, 129, 255, 257])
-@pytest.mark.parametrize("algo", [0, 8])
-def test_a2a_dispatch_gemm_ragged_rows_in_place(rows, algo):
-    # rows that end inside the last tile: read where they are, the rest of the tile counts as zero
-    K, N = 136, 512
+@pytest.mark.parametrize("algo,rows,N,K", [(a, r, 512, 136) for a in (0, 8) for r in (1, 127, 129, 255, 257)] +
+                         [(0, 2100, 4096, 4096), (1, 2427, 2816, 4096)])
+def test_a2a_dispatch_gemm_ragged_rows_in_place(algo, rows, N, K):
+    # rows that end inside the last tile: read where they are, the rest of the tile counts as zero; the last two cases in
+    # pair tiles whose last second half holds nothing
     impl = make_impl()
     mlen = torch.tensor([[rows]], dtype=torch.int32)
     A, B, _ = make_inputs(rows, N, K, torch.float16, seed=rows)
@@ -523,8 +533,9 @@ def test_a2a_dispatch_gemm_ragged_rows_in_place(rows, algo):
     impl.a2a_dispatch_gemm(A, B, C, mlen, algo)
     torch.cuda.synchronize()
     impl.check_status()
+    assert rows < 2000 or ALGO_TILES[impl.last_algo()][0] == 256
     ref = A.double() @ B.double().t()
-    # one rounding to 11 bits and fp32 sums of 136 products
+    # one rounding to 11 bits and fp32 sums
     assert (C[:rows].double() - ref).abs().max().item() <= 2 ** -10 * ref.abs().max().item()
     assert bool((C[rows:] == 0).all())
 

@@ -34,14 +34,24 @@ def test_gemm_matches_fp32_reference(dtype, algo, shape):
     B = (torch.randn(N, K, device="cuda") / K ** 0.5).to(dtype)
     C = torch.full((M, N), float("nan"), device="cuda", dtype=dtype)
     impl = _impl()
+    impl.set_keep_tile(True)     # this tile configuration and no other
     impl.cutlass_gemm(A, B, C, algo)
     torch.cuda.synchronize()
     impl.check_status()
+    assert impl.last_algo() == algo
     ref = _ref(A, B)
     tol = 2e-2 if dtype == torch.bfloat16 else 4e-3
     assert torch.isfinite(C.float()).all(), "unwritten or non-finite output"
     err = (C.float() - ref).abs().max().item()
     assert err <= tol * max(1.0, ref.abs().max().item()), f"max abs err {err}"
+    # and in the configuration that the launch chooses: the same sums in the same order
+    D = torch.full_like(C, float("nan"))
+    impl.set_keep_tile(False)
+    impl.cutlass_gemm(A, B, D, algo)
+    torch.cuda.synchronize()
+    impl.check_status()
+    assert impl.last_algo() == torch.ops.flashoverlap_op.planned_algo(M, N, K, algo, 0, False)
+    assert torch.equal(C, D)
 
 
 def test_gemm_many_tiles_persistent_loop():
@@ -52,11 +62,13 @@ def test_gemm_many_tiles_persistent_loop():
     B = (torch.randn(N, K, device="cuda") / K ** 0.5).to(torch.bfloat16)
     C = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
     impl = _impl()
+    impl.set_keep_tile(True)
     for algo in ALGOS:
         C.fill_(float("nan"))
         impl.cutlass_gemm(A, B, C, algo)
         torch.cuda.synchronize()
         impl.check_status()
+        assert impl.last_algo() == algo
         ref = _ref(A, B)
         err = (C.float() - ref).abs().max().item()
         assert err <= 2e-2 * ref.abs().max().item(), f"algo {algo}: max abs err {err}"
@@ -94,18 +106,23 @@ def test_algo_table_matches_generated_python_copy():
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("algo,M,ffn", [(8, 256, 128), (3, 512, 1920), (9, 768, 64), (4, 256, 14336 // 8)])
-def test_gemm_swiglu(dtype, algo, M, ffn):
-    # gate and up columns of one tile in the two CTAs of a pair; one tile, ragged last tile column, the narrowest
-    K = 328
+@pytest.mark.parametrize("algo,M,ffn", [(8, 256, 128), (3, 512, 1920), (9, 768, 64), (4, 256, 14336 // 8), (4, 256, 4800)])
+@pytest.mark.parametrize("K", [8, 328])
+@pytest.mark.parametrize("keep", [True, False])
+def test_gemm_swiglu(dtype, algo, M, ffn, K, keep):
+    # gate and up columns of one tile in the two CTAs of a pair, for each pair of at least 128 columns: one tile, many,
+    # the narrowest; in the tile that the launch chooses also a last tile that is half full (4800 of 38 x 128)
     torch.manual_seed(ffn)
     impl = torch.classes.flashoverlap_class.OverlapImpl()
     impl.cutlass_init()
+    impl.set_keep_tile(keep)
     x = torch.randn(M, K, device="cuda", dtype=dtype)
     w = (torch.randn(2 * ffn, K, device="cuda") * 2 / K ** 0.5).to(dtype)
     guard = torch.full((M + 1, ffn), 3.0, device="cuda", dtype=dtype)
     impl.gemm_swiglu(x, w, guard[:M], algo)
     torch.cuda.synchronize()
+    assert impl.last_algo() == (algo if keep else torch.ops.flashoverlap_op.planned_algo(M, 2 * ffn, K, algo, 0, True))
+    assert (ffn, K) != (4800, 328) or keep or ALGO_TILES[impl.last_algo()][:2] == (256, 256)
     gate, up = (x.double() @ w.double().t()).chunk(2, dim=-1)
     want = torch.nn.functional.silu(gate) * up
     # one rounding of the result (11 or 8 bits) on fp32 sums
@@ -114,3 +131,4 @@ def test_gemm_swiglu(dtype, algo, M, ffn):
     assert bool((guard[M] == 3).all())
     with pytest.raises(RuntimeError):
         impl.gemm_swiglu(x, w, guard[:M], 0)      # not a CTA-pair tile
+

@@ -79,6 +79,30 @@ def test_no_alloc_entry_matches_regular_entry_twice(dtype):
         assert err32 <= 2 * tol * max(1.0, ref.abs().max().item()), f"call {call}: max abs err vs fp32 {err32}"
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,N", [(256, 512), (256, 2304), (1024, 8192), (256, 8448), (384, 16640), (8192, 2048)])
+def test_row_workers_on_rows_of_every_width(dtype, M, N):
+    # the row workers that several ranks run, on one rank: rows that fill a part of a row group's registers, that end
+    # inside a warp's chunks, that fill them exactly, that take two passes, and more rows than row groups
+    torch.cuda.set_device(0)
+    fn = _entry()
+    K, eps = 264, 1e-5
+    torch.manual_seed(N)
+    A = torch.randn(M, K, device="cuda", dtype=dtype)
+    B = (torch.randn(N, K, device="cuda") / K ** 0.5).to(dtype)
+    W = (1 + 0.1 * torch.randn(N, device="cuda")).to(dtype)
+    out = torch.full((M, N), float("nan"), device="cuda", dtype=dtype)
+    status = torch.zeros(8, dtype=torch.int32, device="cuda")
+    rc, msg = _call(fn, A, B, W, out, eps, status)
+    torch.cuda.synchronize()
+    assert rc == 0 and int(status[0]) == 0, msg
+    y = A.double() @ B.double().t()
+    want = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + eps) * W.double()
+    # the product, its scaling and the weighted value are each rounded to 11 or 8 bits
+    ulp = 2 ** -9.3 if dtype == torch.float16 else 2 ** -6.3
+    assert ((out.double() - want).abs() <= ulp * want.abs() + 1e-4).all()
+
+
 def test_no_alloc_entry_rejects_oversized_and_misshapen_problems():
     torch.cuda.set_device(0)
     fn = _entry()
