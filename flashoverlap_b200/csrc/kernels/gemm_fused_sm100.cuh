@@ -767,7 +767,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
   }
   // Everything above works on this SM alone and may run under the kernel before this one.
   ptx::wait_for_previous_kernel();
-  ptx::allow_next_kernel();
   const uint64_t t_start = ptx::globaltimer_ns();
   const uint64_t deadline = t_start + p.timeout_ns;
   if (threadIdx.x == 0 && p.phase_trace != nullptr) {
@@ -890,6 +889,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
           }
         }
       }
+      // The next kernel in the stream may set itself up from here on, under the last tiles.  Earlier, its waiting CTAs
+      // would keep SMs that this launch does not use from other streams for all of its time.  A launch that waits for
+      // other ranks lets nobody in before it ends: what the others wait for may still need an SM here.
+      if (ok && p.ws == 1) ptx::allow_next_kernel();
       if (ok && p.a_ready != nullptr && blockIdx.x == 0) {
         // The kernel may only end when every rank's pushes of this call have
         // arrived, also those of ranks that sent this rank no rows: it keeps a

@@ -128,6 +128,33 @@ def test_norm_of_a_product_whose_staging_is_dropped():
             assert ((got.double() - want).abs() <= 2 ** -9.3 * want.abs() + 1e-4).all()
 
 
+def test_sms_left_to_another_stream_stay_free():
+    # a GEMM on 100 SMs, then an RMSNorm that waits for it: the other SMs belong to whatever other streams bring meanwhile
+    # (a CTA of this RMSNorm takes more than half of an SM's registers), and are not held by the waiting kernel
+    M = N = K = 8192
+    A, B, W = make_inputs(M, N, K, torch.bfloat16)
+    impl = make_impl()
+    impl.set_sm_count(100)
+    C, O = torch.empty(M, N, device="cuda", dtype=torch.bfloat16), torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    x, y = A[:32].clone(), A[:32].clone()
+    other = torch.cuda.Stream()
+    waited = []
+    for _ in range(4):
+        start, end, mid = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+        torch.cuda.synchronize()
+        start.record()
+        impl.cutlass_gemm(A, B, C, 8)
+        torch.ops.flashoverlap_op.rmsnorm(C, O, W, 1e-5)
+        end.record()
+        with torch.cuda.stream(other):
+            torch.ops.flashoverlap_op.rmsnorm(x, y, W, 1e-5)
+            mid.record()
+        torch.cuda.synchronize()
+        waited.append(start.elapsed_time(mid) / start.elapsed_time(end))
+    impl.check_status()
+    assert sorted(waited)[1] < 0.5, waited
+
+
 def test_phase_trace_records_every_row_once():
     M, N, K = 2048, 2048, 256
     A, B, W = make_inputs(M, N, K, torch.float16, seed=4)
