@@ -53,8 +53,10 @@ inline void check_int_tensor(const at::Tensor& t, const char* name, bool cuda) {
 // Index arrays that a kernel stores through are validated on the host before
 // the launch: a stale or corrupt tuning file must not become a write outside a
 // buffer (possibly a peer GPU's).  The check costs a device synchronisation,
-// so its outcome is remembered per (storage address, tensor version, length):
-// the same tensor object is checked again only after it has been written.
+// so its outcome is remembered per (storage, place in it, tensor version, length):
+// the same tensor is checked again only after it has been written.  The storage
+// is held weakly: its memory is free to go, but the next array at the same
+// address is another storage and is checked anew.
 class IndexCheckCache {
  public:
   // `t` must hold every value of [0, n) exactly once (a tile-to-slot map).
@@ -81,30 +83,29 @@ class IndexCheckCache {
   }
 
  private:
-  struct Key {
+  struct Entry {
+    c10::weak_intrusive_ptr<c10::StorageImpl> storage;  // keeps the identity from being used again
     const void* ptr;
     uint32_t version;
     int64_t numel, bound;
     int kind;
-    bool operator==(const Key& o) const {
-      return ptr == o.ptr && version == o.version && numel == o.numel && bound == o.bound && kind == o.kind;
-    }
   };
-  static Key key_of(const at::Tensor& t, int64_t bound, int kind) {
-    return Key{t.data_ptr(), static_cast<uint32_t>(t._version()), t.numel(), bound, kind};
-  }
   bool seen(const at::Tensor& t, int64_t bound, int kind) const {
-    const Key k = key_of(t, bound, kind);
-    for (const Key& e : entries_) {
-      if (e == k) return true;
+    const c10::StorageImpl* storage = t.storage().unsafeGetStorageImpl();
+    for (const Entry& e : entries_) {
+      if (e.storage._unsafe_get_target() == storage && e.ptr == t.data_ptr() &&
+          e.version == static_cast<uint32_t>(t._version()) && e.numel == t.numel() && e.bound == bound && e.kind == kind) {
+        return true;
+      }
     }
     return false;
   }
   void remember(const at::Tensor& t, int64_t bound, int kind) {
     if (entries_.size() >= 16) entries_.erase(entries_.begin());
-    entries_.push_back(key_of(t, bound, kind));
+    entries_.push_back(Entry{t.storage().getWeakStorageImpl(), t.data_ptr(), static_cast<uint32_t>(t._version()),
+                             t.numel(), bound, kind});
   }
-  std::vector<Key> entries_;
+  std::vector<Entry> entries_;
 };
 
 }  // namespace fo

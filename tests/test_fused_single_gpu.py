@@ -345,6 +345,37 @@ def test_compat_overlap_result_at_any_element(offset):
     assert bool((buf[:offset] == 7).all()) and bool((buf[offset + M * N:] == 7).all())
 
 
+def test_index_arrays_are_checked_anew_in_the_memory_of_an_earlier_one():
+    # the outcome of a check belongs to the array, not to its address: a freed array's memory holds another one next
+    M, N, K, algo = 256, 512, 64, 0
+    A, B, W = make_inputs(M, N, K, torch.float16)
+    impl = make_impl()
+    C, O = (torch.empty(M, N, device="cuda", dtype=torch.float16) for _ in range(2))
+    MM = torch.zeros((3, 2), dtype=torch.int32, device="cuda")
+    cseg = torch.tensor([4], dtype=torch.int32)
+    cseg_gpu = cseg.cuda()
+
+    def overlap(ra):
+        impl.gemm_allreduce_overlap(A, B, C, MM, ra, 1, cseg, cseg_gpu, algo, False)
+
+    def norm(ra):
+        torch.ops.flashoverlap_op.reorder_rmsnorm_eps(C, O, W, 128, 256, 1, ra, 1e-5)
+
+    for call in (overlap, norm):
+        good = torch.arange(4, dtype=torch.int32, device="cuda").view(2, 2)
+        call(good)
+        call(good)
+        address = good.data_ptr()
+        del good
+        bad = torch.zeros(4, dtype=torch.int32, device="cuda").view(2, 2)     # one slot four times: in range, no order
+        assert bad.data_ptr() == address
+        with pytest.raises(RuntimeError, match="not a permutation"):
+            call(bad)
+        del bad
+    torch.cuda.synchronize()
+    impl.check_status()
+
+
 def test_addresses_are_checked_on_the_host_before_any_launch():
     # the kernel moves 16 bytes at a time: whatever starts between two such boundaries is refused with a message
     M, N, K = 256, 512, 64
