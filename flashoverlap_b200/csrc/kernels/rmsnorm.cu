@@ -233,7 +233,9 @@ cudaError_t launch_rmsnorm(const void* x, void* out, const void* w, int rows, in
 
 cudaError_t launch_reorder_rmsnorm(const void* x, void* out, const void* w, int rows, int dim, float eps,
                                    const OutLayout& in_layout, DType dt, cudaStream_t stream) {
-  if (in_layout.tiled && (in_layout.bn % 8 != 0 || in_layout.bm <= 0 || in_layout.rldn <= 0)) {
+  // the kernel finds its tiles itself: no natural layout (bn = 0) and no row map
+  if (!in_layout.tiled || in_layout.row_map != nullptr || in_layout.bn <= 0 || in_layout.bn % 8 != 0 ||
+      in_layout.bm <= 0 || in_layout.rldn <= 0) {
     return cudaErrorInvalidValue;
   }
   return launch<NORM_TILES>(x, nullptr, nullptr, out, w, rows, dim, eps, in_layout, dt, stream);

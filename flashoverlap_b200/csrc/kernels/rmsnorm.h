@@ -14,7 +14,7 @@ cudaError_t launch_rmsnorm(const void* x, void* out, const void* w, int rows, in
                            cudaStream_t stream);
 
 // Same, but x is stored in the tile-reordered layout described by `in_layout`
-// (OutLayout::tiled == 1) and the output is written in natural order.
+// (OutLayout::tiled == 1, no row map) and the output is written in natural order.
 cudaError_t launch_reorder_rmsnorm(const void* x, void* out, const void* w, int rows, int dim, float eps,
                                    const OutLayout& in_layout, DType dt, cudaStream_t stream);
 
