@@ -2,11 +2,12 @@
 //
 // One CTA works on one row at a time and walks several rows; a thread owns the same one, two or four 16-byte chunks
 // (8 values each) of every row, so that the weights can stay in registers, and the next row is on its way from memory
-// while the current one is reduced, scaled and stored (one barrier per row).  Rows of more than 32768 values are read
-// twice.  Bound by HBM: 16384 x 4096 bf16 takes 45.1 us (5.95 TB/s) where one CTA per row, with nothing in flight
-// while it reduced, took 63.0; 37 x 8000 fp16 takes 2.2 us where it took 3.1.  Tile order reads at 2048 x 8192 behind
-// its GEMM: 54.3 us for the pair against 57.2 with the tile found anew for every load.  With a sum (two rows in, two
-// out) 2048 x 4096 bf16 takes 9.8 us.  Unlike the reference kernels (reference: src/rmsnorm/rmsnorm.cuh:12-115, block size dim/16, eps fixed to
+// while the current one is reduced, scaled and stored (one barrier per row).  Wide rows of matrices beyond the L2 take one
+// CTA each (rmsnorm_row_kernel), rows of more than 32768 values (of a sum: 16384) are read twice.  Bound by HBM: 16384 x
+// 4096 bf16 takes 45.1 us (5.95 TB/s) where one CTA per row, with nothing in flight while it reduced, took 63.0; 37 x
+// 8000 fp16 takes 2.2 us where it took 3.1; a single launch of 4096 x 8192 bf16 on a cold L2 28.7 where it took 30.7.
+// Tile order reads at 2048 x 8192 behind its GEMM: 54.3 us for the pair against 57.2 with the tile found anew for every
+// load.  With a sum (two rows in, two out) 2048 x 4096 bf16 takes 9.8 us.  Unlike the reference kernels (reference: src/rmsnorm/rmsnorm.cuh:12-115, block size dim/16, eps fixed to
 // 1e-5, default stream) any dim % 8 == 0 works, eps is an argument and the launch goes to the caller's stream.
 #include "rmsnorm.h"
 
@@ -17,6 +18,8 @@ namespace fo {
 namespace {
 
 constexpr int kMaxNormThreads = 1024;
+constexpr int kRowThreads = 256;  // rmsnorm_row_kernel
+constexpr int kRowChunks = 8;
 
 // What a row is before it is normalised: as stored, stored in tile order, or the sum of two rows (written back).
 enum NormInput { NORM_ROWS, NORM_TILES, NORM_SUM };
@@ -136,6 +139,40 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t
   }
 }
 
+// Rows as stored, of up to 16384 values, one CTA of 256 threads per row: five rows of an SM are loaded, reduced and stored
+// independently of one another.  For matrices that stream through HBM (see launch_typed).
+template <bool BF16>
+__global__ void __launch_bounds__(kRowThreads, 5) rmsnorm_row_kernel(const uint16_t* x, uint16_t* out,
+                                                                     const uint16_t* __restrict__ w, int dim, float eps) {
+  __shared__ float red[kRowThreads / 32];
+  const int n_chunks = dim >> 3;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long row_off = static_cast<long long>(blockIdx.x) * dim;
+  const uint4* src = reinterpret_cast<const uint4*>(x + row_off);
+  uint4 v[kRowChunks];
+#pragma unroll
+  for (int k = 0; k < kRowChunks; ++k) v[k] = src[min(static_cast<int>(threadIdx.x) + k * kRowThreads, n_chunks - 1)];
+  float ssq = 0.f;
+#pragma unroll
+  for (int k = 0; k < kRowChunks; ++k) {
+    if (static_cast<int>(threadIdx.x) + k * kRowThreads < n_chunks) ssq += sum_squares<BF16>(v[k]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+  if (lane == 0) red[warp] = ssq;
+  __syncthreads();
+  ssq = 0.f;
+#pragma unroll
+  for (int i = 0; i < kRowThreads / 32; ++i) ssq += red[i];
+  const float rstd = rsqrtf(ssq / static_cast<float>(dim) + eps);
+  uint4* dst = reinterpret_cast<uint4*>(out + row_off);
+#pragma unroll
+  for (int k = 0; k < kRowChunks; ++k) {
+    const int c = static_cast<int>(threadIdx.x) + k * kRowThreads;
+    if (c < n_chunks) dst[c] = scale_chunk<BF16>(v[k], rstd, __ldg(reinterpret_cast<const uint4*>(w) + c));
+  }
+}
+
 // Rows wider than the registers of a CTA hold: one CTA per row, read twice.
 template <bool BF16, int INPUT>
 __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_wide_kernel(const uint16_t* x, const uint16_t* r,
@@ -195,7 +232,9 @@ template <bool BF16, int INPUT>
 cudaError_t launch_typed(const uint16_t* x, const uint16_t* r, uint16_t* sum, uint16_t* out, const uint16_t* w, int rows,
                          int dim, float eps, const OutLayout& L, cudaStream_t stream) {
   const int n_chunks = dim >> 3;
-  if (n_chunks > 4 * kMaxNormThreads) {
+  // A sum of more than two chunks per thread does not fit the registers beside the next row (the kernel spills):
+  // 4096 x 20480 bf16 takes 154 us in that form, 113 here, 137 as an addition and an RMSNorm of their own.
+  if (n_chunks > (INPUT == NORM_SUM ? 2 : 4) * kMaxNormThreads) {
     return launch_after(rmsnorm_wide_kernel<BF16, INPUT>, rows, kMaxNormThreads, stream, x, r, sum, out, w, dim, eps, L);
   }
   const int sms = device_sm_count();
@@ -204,14 +243,28 @@ cudaError_t launch_typed(const uint16_t* x, const uint16_t* r, uint16_t* sum, ui
   // registers; four need the registers of the weights (the kernel spills at 64 a thread) and serve the widest rows only.
   int cpt = rows <= 2 * sms || n_chunks <= 32 ? 1 : 2;
   while (n_chunks > cpt * kMaxNormThreads) cpt *= 2;
+  if constexpr (INPUT == NORM_ROWS) {
+    // Past the L2 (126 MB) the matrix streams, and CTAs that do not wait for one another keep HBM busier than few large ones
+    // that walk: 8192 x 12288 bf16 74.8 -> 64.7 us, 24576 x 6144 116 -> 96, 24576 x 8192 130 -> 121.  Rows of up to 5120
+    // values leave most of the registers of such a CTA empty (24576 x 5120: 83 us walked, 100 one by one).
+    if (cpt == 2 && n_chunks > 640 && 2.0 * rows * dim >= 126e6) {
+      rmsnorm_row_kernel<BF16><<<rows, kRowThreads, 0, stream>>>(x, out, w, dim, eps);
+      return cudaGetLastError();
+    }
+    // More than 8192 values: with two chunks per thread a single CTA fits an SM and nothing runs while it waits at its
+    // barrier.  From ten rows per SM on, four chunks and two or three CTAs: 4096 x 9216 32.5 -> 27.1 us, 2048 x 16384 24.8 ->
+    // 23.9; with fewer rows two chunks are the faster form (1024 x 16384 13.7 us against 15.1).
+    if (cpt == 2 && n_chunks > kMaxNormThreads && rows > 10 * sms) cpt = 4;
+  }
   const int threads = ((n_chunks + cpt - 1) / cpt + 31) / 32 * 32;
   // 64 registers a thread: the CTAs that are resident together
   int per_sm = kMaxNormThreads / threads;
   if (per_sm > 32) per_sm = 32;
   const int grid = rows < sms * per_sm ? rows : sms * per_sm;
-  auto kernel = cpt == 1   ? rmsnorm_kernel<BF16, INPUT, 1>
-                : cpt == 2 ? rmsnorm_kernel<BF16, INPUT, 2>
-                           : rmsnorm_kernel<BF16, INPUT, 4>;
+  auto kernel = cpt == 1 ? rmsnorm_kernel<BF16, INPUT, 1> : rmsnorm_kernel<BF16, INPUT, 2>;
+  if constexpr (INPUT != NORM_SUM) {
+    if (cpt == 4) kernel = rmsnorm_kernel<BF16, INPUT, 4>;
+  }
   return launch_after(kernel, grid, threads, stream, x, r, sum, out, w, rows, dim, eps, L);
 }
 

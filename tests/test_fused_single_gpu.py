@@ -481,6 +481,24 @@ def test_rmsnorm_thread_shapes(rows, dim):
     assert torch.equal(x, o)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,dim", [(1481, 8200), (1500, 16384), (3000, 12296),      # four chunks per thread
+                                      (12300, 5128), (10500, 6104), (7700, 8200), (3900, 16384)])     # 126 MB: a CTA per row
+def test_rmsnorm_of_many_wide_rows(dtype, rows, dim):
+    torch.manual_seed(dim)
+    x = torch.randn(rows, dim, device="cuda", dtype=dtype)
+    w = (1 + 0.1 * torch.randn(dim, device="cuda")).to(dtype)
+    o = torch.full_like(x, float("nan"))
+    torch.ops.flashoverlap_op.rmsnorm(x, o, w, 1e-6)
+    xd = x.double()
+    want = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    # two roundings to 11 or 8 bits each
+    ulp = 2 ** -9.9 if dtype == torch.float16 else 2 ** -6.9
+    assert ((o.double() - want).abs() <= ulp * want.abs() + 1e-7).all()
+    torch.ops.flashoverlap_op.rmsnorm(x, x, w, 1e-6)
+    assert torch.equal(x, o)
+
+
 def test_rmsnorm_addresses_are_checked_on_the_host():
     op = torch.ops.flashoverlap_op
     rows, dim = 128, 256
