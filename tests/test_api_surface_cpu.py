@@ -54,6 +54,14 @@ def test_planned_tile_needs_no_gpu():
         assert bm == 256 and bn >= 128                                               # gate and up side by side
 
 
+def test_planned_tile_is_not_one_that_measured_slower():
+    # shapes at which the tile of the least single-wave time took 5 to 16 % longer than the named one (M, N, K, named)
+    for m, n, k, algo in ((6656, 1024, 16232, 8), (3072, 2048, 792, 8), (1280, 640, 4424, 10), (4352, 1536, 10304, 8),
+                          (2560, 2304, 6600, 8), (1024, 2560, 1128, 8), (768, 7168, 4056, 8), (3072, 2304, 5792, 8),
+                          (6016, 8960, 440, 0), (1792, 1152, 2952, 4)):
+        assert torch.ops.flashoverlap_op.planned_algo(m, n, k, algo, 148, False) == algo
+
+
 def test_tile_table_matches_the_python_copy():
     from flashoverlap_b200.utils.config import ALGO_TILES
 
