@@ -18,6 +18,11 @@
 
 namespace fo {
 
+static void check_norm_launch(cudaError_t e, const char* op) {
+  TORCH_CHECK(e == cudaSuccess, op, " launch failed: ",
+              e == cudaErrorMisalignedAddress ? "tensors must be 16-byte aligned" : cudaGetErrorString(e));
+}
+
 static std::vector<int64_t> generate_id_op() { return generate_nccl_id(); }
 
 // reorder_rmsnorm(X, RX, RW, BM, BN, rldn, RA): X holds a [bs, dim] matrix in
@@ -34,9 +39,6 @@ static void reorder_rmsnorm_eps(at::Tensor X, at::Tensor RX, at::Tensor RW, int6
   TORCH_CHECK(RW.is_cuda() && RW.is_contiguous() && RW.numel() == dim, "RW must hold dim values");
   TORCH_CHECK(BM > 0 && BN > 0 && bs % BM == 0 && dim % BN == 0 && BN % 8 == 0 && dim % 8 == 0,
               "need bs % BM == 0, dim % BN == 0, BN % 8 == 0");
-  check_aligned(X, "X");
-  check_aligned(RX, "RX");
-  check_aligned(RW, "RW");
   check_int_tensor(RA, "RA", true);
   const int64_t tiles = (bs / BM) * (dim / BN);
   TORCH_CHECK(RA.numel() == tiles, "RA must have ", tiles, " entries, got ", RA.numel());
@@ -59,7 +61,7 @@ static void reorder_rmsnorm_eps(at::Tensor X, at::Tensor RX, at::Tensor RW, int6
   cudaError_t e = launch_reorder_rmsnorm(X.data_ptr(), RX.data_ptr(), RW.data_ptr(), static_cast<int>(bs),
                                          static_cast<int>(dim), static_cast<float>(eps), L, dt,
                                          at::cuda::getCurrentCUDAStream().stream());
-  TORCH_CHECK(e == cudaSuccess, "reorder_rmsnorm launch failed: ", cudaGetErrorString(e));
+  check_norm_launch(e, "reorder_rmsnorm");
 }
 
 static void reorder_rmsnorm_op(at::Tensor X, at::Tensor RX, at::Tensor RW, int64_t BM, int64_t BN, int64_t rldn,
@@ -77,14 +79,11 @@ static void rmsnorm_op(at::Tensor X, at::Tensor O, at::Tensor RW, double eps) {
   TORCH_CHECK(O.sizes() == X.sizes(), "O must have the shape of X");
   TORCH_CHECK(RW.is_cuda() && RW.is_contiguous() && RW.numel() == X.size(1), "RW must hold dim values");
   TORCH_CHECK(X.size(1) % 8 == 0, "dim must be a multiple of 8");
-  check_aligned(X, "X");
-  check_aligned(O, "O");
-  check_aligned(RW, "RW");
   c10::cuda::CUDAGuard guard(X.device());
   cudaError_t e = launch_rmsnorm(X.data_ptr(), O.data_ptr(), RW.data_ptr(), static_cast<int>(X.size(0)),
                                  static_cast<int>(X.size(1)), static_cast<float>(eps), dt,
                                  at::cuda::getCurrentCUDAStream().stream());
-  TORCH_CHECK(e == cudaSuccess, "rmsnorm launch failed: ", cudaGetErrorString(e));
+  check_norm_launch(e, "rmsnorm");
 }
 
 // add_rmsnorm(X, R, S, O, RW, eps): S = X + R (rounded to the 16-bit type), O = rmsnorm(S); one pass over the rows.
@@ -101,16 +100,11 @@ static void add_rmsnorm_op(at::Tensor X, at::Tensor R, at::Tensor S, at::Tensor 
   TORCH_CHECK(RW.is_cuda() && RW.is_contiguous() && RW.numel() == X.size(1) && RW.scalar_type() == X.scalar_type(),
               "RW must hold dim values of X's dtype");
   TORCH_CHECK(X.size(1) % 8 == 0, "dim must be a multiple of 8");
-  check_aligned(X, "X");
-  check_aligned(R, "R");
-  check_aligned(S, "S");
-  check_aligned(O, "O");
-  check_aligned(RW, "RW");
   c10::cuda::CUDAGuard guard(X.device());
   cudaError_t e = launch_add_rmsnorm(X.data_ptr(), R.data_ptr(), S.data_ptr(), O.data_ptr(), RW.data_ptr(),
                                      static_cast<int>(X.size(0)), static_cast<int>(X.size(1)), static_cast<float>(eps),
                                      dt, at::cuda::getCurrentCUDAStream().stream());
-  TORCH_CHECK(e == cudaSuccess, "add_rmsnorm launch failed: ", cudaGetErrorString(e));
+  check_norm_launch(e, "add_rmsnorm");
 }
 
 // The order in which the persistent kernel walks the tile grid, computed on

@@ -23,11 +23,6 @@ inline void check_matrix(const at::Tensor& t, const char* name) {
   TORCH_CHECK(t.is_contiguous(), name, " must be contiguous (row-major)");
 }
 
-// The kernels load and store 16 bytes at a time.
-inline void check_aligned(const at::Tensor& t, const char* name) {
-  TORCH_CHECK(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, name, " must be 16-byte aligned");
-}
-
 inline void check_gemm_args(const at::Tensor& A, const at::Tensor& B, const at::Tensor* C) {
   check_matrix(A, "A");
   check_matrix(B, "B");

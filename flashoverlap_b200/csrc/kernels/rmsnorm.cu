@@ -272,6 +272,9 @@ template <int INPUT>
 cudaError_t launch(const void* x, const void* r, void* sum, void* out, const void* w, int rows, int dim, float eps,
                    const OutLayout& L, DType dt, cudaStream_t stream) {
   if (rows <= 0 || dim <= 0 || dim % 8 != 0) return cudaErrorInvalidValue;
+  // the kernels load and store 16 bytes at a time
+  auto address = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
+  if ((address(x) | address(r) | address(sum) | address(out) | address(w)) & 15u) return cudaErrorMisalignedAddress;
   auto typed = dt == DT_BF16 ? launch_typed<true, INPUT> : launch_typed<false, INPUT>;
   return typed(static_cast<const uint16_t*>(x), static_cast<const uint16_t*>(r), static_cast<uint16_t*>(sum),
                static_cast<uint16_t*>(out), static_cast<const uint16_t*>(w), rows, dim, eps, L, stream);

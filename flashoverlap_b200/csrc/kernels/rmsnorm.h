@@ -8,6 +8,8 @@
 
 namespace fo {
 
+// All tensors start on a 16-byte boundary (else cudaErrorMisalignedAddress, before anything is launched).
+
 // out[r][:] = round16(x[r][:] * rsqrt(mean(x[r][:]^2) + eps)) * w[:], natural
 // layout in and out.  dim % 8 == 0.
 cudaError_t launch_rmsnorm(const void* x, void* out, const void* w, int rows, int dim, float eps, DType dt,
