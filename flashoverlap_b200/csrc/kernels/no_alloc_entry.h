@@ -14,9 +14,12 @@
  * of the library image, so that a call consists of a small memset and one
  * kernel launch and nothing else.
  *
- * What it computes.  out[M,N] = RMSNorm(A[M,K] * B[N,K]^T) * gamma, the same
- * fused kernel as OverlapImpl.gemm_rmsnorm with the 128x256 tile: fp32
- * accumulation, the product rounded to the 16-bit type, fp32 row statistics.
+ * What it computes.  out[M,N] = RMSNorm(A[M,K] * B[N,K]^T) * gamma, the result
+ * of OverlapImpl.gemm_rmsnorm: fp32 accumulation, the product rounded to the
+ * 16-bit type, fp32 row statistics.  It runs the fused kernel always in the
+ * 128x256 tile and with the row workers of several ranks, which find the row
+ * statistics themselves; gemm_rmsnorm takes the tile with the least expected
+ * time and has the statistics from the epilogue, which is faster.
  * A, B, gamma and out are device pointers supplied by the caller, row-major,
  * 16-byte aligned; dtype 0 = float16, 1 = bfloat16.
  *

@@ -240,7 +240,7 @@ cudaError_t launch_typed(const uint16_t* x, const uint16_t* r, uint16_t* sum, ui
   const int sms = device_sm_count();
   // Few rows (up to two per SM): as many threads per row as it has chunks, since only the latency of one row counts.
   // Many rows: two chunks per thread, which leaves fewer warps to wait at the row's barrier and keeps the weights in
-  // registers; four need the registers of the weights (the kernel spills at 64 a thread) and serve the widest rows only.
+  // registers; four need the registers of the weights (the kernel spills at 64 a thread) and serve wide rows only.
   int cpt = rows <= 2 * sms || n_chunks <= 32 ? 1 : 2;
   while (n_chunks > cpt * kMaxNormThreads) cpt *= 2;
   if constexpr (INPUT == NORM_ROWS) {

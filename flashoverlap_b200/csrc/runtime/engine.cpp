@@ -175,8 +175,10 @@ void FusedEngine::base_params(FusedParams& p, const SignalArgs* sig) {
 
 namespace {
 // Tile rows walked together on one GPU.  A group reads every B panel once for all of its rows; rows that are normalised
-// wait for their whole group, so operands that stay in L2 anyway (up to a third of it) take a narrower one: 4096 x 8192 x
-// 1024 93.5 -> 91.8 us.  Groups of 16 were no better than 8 for larger operands (8192 x 8192 x 3584: 394 and 392 us).
+// wait for their whole group, so operands that stay in L2 anyway (up to a third of it) take a narrower one.  Groups of 8
+// and 4 in turn, fp16: 2304 x 8192 x 1024 57.9 and 54.4 us, 4096 x 8192 x 1024 93.9 and 91.5, 4096 x 8192 x 1536 118 and
+// 112, 8192 x 8192 x 1024 181 and 177; the other way round at 4096 x 4096 x 2048, 74.0 and 76.2.  With 50 to 101 MB of
+// operands the two differ by 1 % either way (8192 x 8192 x 2048: 276 and 270).
 int local_group(const GemmOperands& g, bool norm) {
   const double operands = 2.0 * (static_cast<double>(g.M) + g.N) * g.K;
   return norm && operands <= 40e6 ? 4 : 8;
@@ -184,8 +186,11 @@ int local_group(const GemmOperands& g, bool norm) {
 }  // namespace
 
 namespace {
-// Staged products that crowd the L2 (with the result of the same size) are dropped line by line as they are read:
-// 4096 x 8192 x 1024 93.8 -> 90.8 us.  Smaller ones only pay for the instruction: 128 x 8192 16.7 -> 17.1.
+// Staged products that crowd the L2 (with the result of the same size) are dropped line by line as they are read.  Of a
+// 4096 x 8192 x 1024 fp16 call 75 MB are written to HBM in place of 133 (67 MB are the product), and 28 read in place of
+// 44: 93.7 -> 91.5 us.  2048 x 8192 x 1024 50.6 -> 49.0, 4096 x 8192 x 512 74.7 -> 71.0; no difference beyond 1 % from K =
+// 1536 on, where the main loop hides the traffic.  Small products only pay for the instruction: 128 x 8192 16.1 -> 16.5,
+// 1024 x 4096 27.7 both ways.
 bool drop_stage(const GemmOperands& g) { return 2.0 * g.M * g.N >= 32e6; }
 }  // namespace
 
