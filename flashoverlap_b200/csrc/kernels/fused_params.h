@@ -126,6 +126,10 @@ struct alignas(64) FusedParams {
   int rows_per_owner;       // M / ws
   void* epi_base[kMaxRanks];  // own_mode SINGLE: [0] = C; else staging slot of `me` on each owner
   OutLayout epi_layout;       // layout within the destination (tiled only with OWN_SINGLE)
+  // Set by the launch.  epi_direct: the destination is on this GPU and pitched, so each lane stores its row from registers;
+  // epi_wide: 32-byte stores are aligned there; epi_halves: 2 = the communication warps have nothing of their own to do and
+  // take half of a tile's columns.
+  int epi_direct, epi_wide, epi_halves;
   uint32_t* flag[kMaxRanks];  // per-owner arrival counters, one per tile row; null = no signalling
 
   // ---- reference-compatible signalling / tracing ----------------------------

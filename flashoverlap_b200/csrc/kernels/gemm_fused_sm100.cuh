@@ -12,14 +12,16 @@
 //   warp 2      TMEM allocator (allocates 2 x BN columns, frees them at the end)
 //   warp 3      signalling     (one lane publishes finished tiles at system scope
 //                               and bumps the owners' arrival counters)
-//   warps 4-7   epilogue       (tcgen05.ld -> convert -> smem transpose ->
-//                               coalesced 16-byte stores, local or to a peer)
+//   warps 4-7   epilogue       (tcgen05.ld -> convert -> 32 bytes of its row per
+//                               lane; to a peer: smem transpose -> coalesced
+//                               16-byte stores)
 //   warps 8-11  communication  (reduce phase: from the first cycle on they claim
 //                               owned rows in completion order, wait (bounded)
 //                               for the row's partials from every rank, sum them
 //                               in fp32, apply RMSNorm and deliver the row;
 //                               all-gather / all-to-all mode: they push this
-//                               rank's rows of A to the other ranks)
+//                               rank's rows of A to the other ranks; with neither:
+//                               they take half of the epilogue's columns)
 // With CTAS == 2 two such CTAs form a cluster: both stage operands and run an
 // epilogue for their own 128 rows, the MMA warp of rank 0 issues for the pair.
 // After its last tile the eight GEMM warps of a CTA join the reduce phase as two
@@ -171,6 +173,31 @@ __device__ __forceinline__ uint4 scale_chunk(const uint4& h, float rstd, const u
   f = unpack2<BF16>(h.z); o.z = norm_pack2<BF16>(f.x, f.y, rstd, w.z);
   f = unpack2<BF16>(h.w); o.w = norm_pack2<BF16>(f.x, f.y, rstd, w.w);
   return o;
+}
+
+// 32 values of a row, from registers.
+__device__ __forceinline__ void store_row32(uint16_t* dst, const uint32_t (&o)[16], bool wide) {
+  if (wide) {
+    ptx::st_v8(dst, o);
+    ptx::st_v8(dst + 16, o + 8);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ptx::st_v4(dst + 8 * e, make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]));
+  }
+}
+
+// 32 accumulators rounded to the 16-bit type.
+template <bool BF16>
+__device__ __forceinline__ void pack_row32(uint32_t (&o)[16], const uint32_t (&r)[32]) {
+#pragma unroll
+  for (int e = 0; e < 16; ++e) o[e] = pack2<BF16>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+}
+template <bool BF16>
+__device__ __forceinline__ float sum_squares32(const uint32_t (&o)[16]) {
+  float s = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) s += sum_squares<BF16>(make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]));
+  return s;
 }
 
 // ---------------------------------------------------------------------------
@@ -730,8 +757,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
   uint64_t* tempty_bar = bars + 2 * STAGES + 2;  // [2] epilogue -> MMA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  uint32_t* epi_prog = tmem_slot + 4;  // [4] tiles finished by each epilogue warp
-  uint64_t* pair_bar = bars + 2 * STAGES + 8;  // teardown handshake between the CTAs of a pair
+  uint32_t* epi_prog = tmem_slot + 4;  // [8] tiles finished by each epilogue warp
+  uint64_t* pair_bar = bars + 2 * STAGES + 10;  // teardown handshake between the CTAs of a pair
   GroupScratch* group_scratch = reinterpret_cast<GroupScratch*>(bars + 40);  // [3] row groups of the reduce phase
 
   const int warp = threadIdx.x >> 5;
@@ -743,11 +770,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&tfull_bar[i], 1);
-      ptx::mbar_init(&tempty_bar[i], T::EPI_WARPS * CTAS);  // the leader hears from both epilogues
+      ptx::mbar_init(&tempty_bar[i], T::EPI_WARPS * p.epi_halves * CTAS);  // the leader hears from both epilogues
     }
     ptx::mbar_init(pair_bar, 1);
     *abort_flag = 0;
-    for (int i = 0; i < 4; ++i) epi_prog[i] = 0;
+    for (int i = 0; i < 2 * T::EPI_WARPS; ++i) epi_prog[i] = 0;
     ptx::mbar_fence_init();
     ptx::fence_proxy_async_smem();
   }
@@ -765,7 +792,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       ptx::tmem_relinquish();
     }
   }
-  // Everything above works on this SM alone and may run under the kernel before this one.
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  if constexpr (CTAS == 2) ptx::cluster_sync();  // both CTAs' barriers exist before anyone signals across
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  // Everything above works on this SM (pair) alone and may run under the kernel before this one.
   ptx::wait_for_previous_kernel();
   const uint64_t t_start = ptx::globaltimer_ns();
   const uint64_t deadline = t_start + p.timeout_ns;
@@ -781,12 +813,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     for (int c = threadIdx.x; c < (p.N >> 3); c += kThreads) {
       ptx::st_shared_v4(gamma_smem + (static_cast<uint32_t>(c) << 4), __ldg(gamma + c));
     }
+    __syncthreads();
   }
-  ptx::tc_fence_before_sync();
-  __syncthreads();
-  if constexpr (CTAS == 2) ptx::cluster_sync();  // both CTAs' barriers exist before anyone signals across
-  ptx::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
 
   const int num_tiles = p.TM * p.TN;
   const int num_kb = (p.K + BK - 1) / BK;  // a K tail is zero-filled by TMA
@@ -967,9 +995,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         }
       }
     }
-  } else if (warp >= 4 && warp < kGemmWarps) {
+  } else if (warp >= 4 && warp < kGemmWarps + (p.epi_halves - 1) * kCommWarps) {
     // ===================== epilogue =====================
+    // Without a reduce phase or a push the communication warps take the second half of the columns.
     const int q = warp & 3;  // TMEM lane quarter this warp may access
+    const int half = warp >= kGemmWarps ? 1 : 0;
     const uint32_t slab = ptx::smem_u32(smem_epi + q * T::EPI_SLAB_BYTES);
     int it = 0;
     bool ok = true;
@@ -991,74 +1021,86 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       ptx::tc_fence_after_sync();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
       const int row0 = m_blk * TILE_M + static_cast<int>(cta_rank) * BM + q * 32;  // first global row of this warp's slab
-      // What of the tile lies inside the matrix: all of this CTA's 128 rows or none, and whole steps of 64 columns.
+      // What of the tile lies inside the matrix: all of this CTA's 128 rows or none, and whole chunks of 32 result columns.
       const int cols_left = p.glu ? 2 * (p.glu - n_blk * (BN / 2)) : p.N - n_blk * BN;
-      const int steps = row0 >= p.M ? 0 : min(BN, cols_left) / 64;
-      if (steps == 0) {
+      const int chunks = row0 >= p.M ? 0 : min(BN, cols_left) / (p.glu ? 64 : 32);
+      // this warp's share of them
+      const int c_begin = half * ((chunks + 1) / 2);
+      const int c_end = p.epi_halves == 2 && half == 0 ? (chunks + 1) / 2 : chunks;
+      // accumulator fully read: hand the TMEM buffer back to the MMA warp
+      auto release = [&] {
         ptx::tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) {
           if constexpr (CTAS == 2) ptx::mbar_arrive_cluster(tempty_addr0 + 8u * buf);
           else ptx::mbar_arrive(&tempty_bar[buf]);
-          ptx::st_release_cta_shared(&epi_prog[q], static_cast<uint32_t>(it + 1));
         }
+      };
+      if (c_begin >= c_end) {
+        release();
+        if (lane == 0) ptx::st_release_cta_shared(&epi_prog[warp - 4], static_cast<uint32_t>(it + 1));
+        continue;
+      }
+      if (p.epi_direct) {
+        // A pitched block on this GPU, in the natural layout or in the tiled one (32 rows lie in one tile row, 64 columns in
+        // one tile).  Every lane stores its own row, 32 bytes (a whole L2 sector) at a time, from registers: through a
+        // shared-memory transpose, four warps took 4.2 us for a tile of 256 x 256 against the 1.5 us of its main loop at
+        // K = 256.
+        const OutLayout& L = p.epi_layout;
+        const long long pitch = L.tiled ? static_cast<long long>(L.rldn) * L.bn : L.ld;
+        uint16_t* const base = reinterpret_cast<uint16_t*>(p.epi_base[0]) + lane * pitch;
+        const int col0 = n_blk * (p.glu ? BN / 2 : BN);
+        float ssq = 0.f;  // of this lane's row over the tile's columns, as rounded
+        auto put = [&](int c, const uint32_t (&o)[16]) {
+          store_row32(base + layout_offset(L, row0, col0 + c * 32), o, p.epi_wide);
+        };
+        auto pack = [&](int c, const uint32_t (&r)[32]) {
+          uint32_t o[16];
+          pack_row32<BF16>(o, r);
+          if (p.ssq != nullptr) ssq += sum_squares32<BF16>(o);
+          put(c, o);
+        };
+#pragma unroll 1
+        for (int c = c_begin; c < c_end; c += p.glu ? 1 : 2) {
+          uint32_t r0[32], r1[32];
+          const bool second = p.glu || c + 1 < c_end;
+          ptx::tmem_ld_32x32b_x32(t_row + c * 32, r0);
+          if (second) ptx::tmem_ld_32x32b_x32(t_row + (p.glu ? BN / 2 + c * 32 : (c + 1) * 32), r1);
+          ptx::tmem_ld_wait();
+          if (c + (p.glu ? 1 : 2) >= c_end) release();
+          if (p.glu) {
+            // (The exp and the division of 128 x 128 values take a tenth of a tile's main loop at K = 4096 and run beside
+            // the next one; the two element-wise passes that they replace took 80 us of a 2048 x 28672 product.)
+            uint32_t o[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              o[e] = pack2<BF16>(silu(__uint_as_float(r0[2 * e])) * __uint_as_float(r1[2 * e]),
+                                 silu(__uint_as_float(r0[2 * e + 1])) * __uint_as_float(r1[2 * e + 1]));
+            }
+            put(c, o);
+          } else {
+            pack(c, r0);
+            if (second) pack(c + 1, r1);
+          }
+        }
+        if (p.ssq != nullptr) {
+          p.ssq[(static_cast<long long>(row0 / BM) * p.TN + n_blk) * BM + q * 32 + lane] = ssq;
+        }
+        __syncwarp();
+        if (lane == 0) ptx::st_release_cta_shared(&epi_prog[warp - 4], static_cast<uint32_t>(it + 1));
         continue;
       }
       const int chunk = lane & 7;  // of a 128-byte row segment; eight lanes write one
-      // A slab that stays on this GPU is a plain pitched block, in the natural layout and in the tiled one
-      // (its 32 rows lie in one tile row, its 64 columns in one tile): the address is found once per step at most.
+      // Slabs for other GPUs, or rows that go through a map: transposed in shared memory, eight lanes per row segment.
       const bool local = p.own_mode == OWN_SINGLE || p.nvls;
-      const OutLayout& L = p.epi_layout;
-      const bool pitched = local && (!L.tiled || (L.row_map == nullptr && L.bm % 32 == 0 && L.bn % 64 == 0));
-      const long long pitch = L.tiled ? static_cast<long long>(L.rldn) * L.bn : L.ld;
-      uint16_t* slab_dst = nullptr;
-      if (pitched) {
-        slab_dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(L, row0, n_blk * (p.glu ? BN / 2 : BN)) +
-                   (lane >> 3) * pitch + chunk * 8;
-      }
-      float ssq = 0.f;  // of this lane's row over the tile's columns, as rounded
 
 #pragma unroll 1
-      for (int cc = 0; cc < steps; ++cc) {
-        // 64 columns of the tile; gated: 32 gate columns and the 32 up columns that belong to them
+      for (int cc = 0; cc < chunks / 2; ++cc) {  // 64 columns of the tile
         uint32_t r0[32], r1[32];
-        ptx::tmem_ld_32x32b_x32(t_row + (p.glu ? cc : 2 * cc) * 32, r0);
-        ptx::tmem_ld_32x32b_x32(t_row + (p.glu ? BN / 64 + cc : 2 * cc + 1) * 32, r1);
+        ptx::tmem_ld_32x32b_x32(t_row + 2 * cc * 32, r0);
+        ptx::tmem_ld_32x32b_x32(t_row + (2 * cc + 1) * 32, r1);
         ptx::tmem_ld_wait();
-        if (cc == steps - 1) {
-          // accumulator fully read: hand the TMEM buffer back to the MMA warp
-          ptx::tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) {
-            if constexpr (CTAS == 2) ptx::mbar_arrive_cluster(tempty_addr0 + 8u * buf);
-            else ptx::mbar_arrive(&tempty_bar[buf]);
-          }
-        }
-        if (p.glu) {
-          // 32 result columns go to the first or second half of the slab, which is stored when it is full.  (The exp and
-          // the division of 128 x 128 values take a tenth of a tile's main loop at K = 4096 and run beside the next one;
-          // the two element-wise passes that they replace took 80 us of a 2048 x 28672 product.)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t o[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int x = 8 * j + 2 * e;
-              o[e] = pack2<BF16>(silu(__uint_as_float(r0[x])) * __uint_as_float(r1[x]),
-                                 silu(__uint_as_float(r0[x + 1])) * __uint_as_float(r1[x + 1]));
-            }
-            ptx::st_shared_v4(slab + lane * 128 + (((j + 4 * (cc & 1)) ^ (lane & 7)) << 4), make_uint4(o[0], o[1], o[2], o[3]));
-          }
-          if ((cc & 1) == 0) continue;
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int r = i * 4 + (lane >> 3);
-            ptx::st_v4(slab_dst + i * 4 * pitch + (cc >> 1) * 64, ptx::ld_shared_v4(slab + r * 128 + ((chunk ^ (r & 7)) << 4)));
-          }
-          __syncwarp();
-          continue;
-        }
+        if (cc == chunks / 2 - 1) release();
         // registers -> swizzled smem slab (row = lane, 8 chunks of 16 bytes)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -1067,7 +1109,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
           v.y = pack2<BF16>(__uint_as_float(r0[8 * j + 2]), __uint_as_float(r0[8 * j + 3]));
           v.z = pack2<BF16>(__uint_as_float(r0[8 * j + 4]), __uint_as_float(r0[8 * j + 5]));
           v.w = pack2<BF16>(__uint_as_float(r0[8 * j + 6]), __uint_as_float(r0[8 * j + 7]));
-          if (p.ssq != nullptr) ssq += sum_squares<BF16>(v);
           ptx::st_shared_v4(slab + lane * 128 + ((j ^ (lane & 7)) << 4), v);
         }
 #pragma unroll
@@ -1077,29 +1118,19 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
           v.y = pack2<BF16>(__uint_as_float(r1[8 * j + 2]), __uint_as_float(r1[8 * j + 3]));
           v.z = pack2<BF16>(__uint_as_float(r1[8 * j + 4]), __uint_as_float(r1[8 * j + 5]));
           v.w = pack2<BF16>(__uint_as_float(r1[8 * j + 6]), __uint_as_float(r1[8 * j + 7]));
-          if (p.ssq != nullptr) ssq += sum_squares<BF16>(v);
           ptx::st_shared_v4(slab + lane * 128 + (((j + 4) ^ (lane & 7)) << 4), v);
         }
         __syncwarp();
         // smem slab -> global: 8 lanes cover one 128-byte row segment
         const int col = n_blk * BN + cc * 64 + chunk * 8;
-        uint16_t* step_dst = slab_dst + cc * 64;
-        if (pitched && L.tiled) {
-          step_dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(L, row0, col - chunk * 8) +
-                     (lane >> 3) * pitch + chunk * 8;
-        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int r = i * 4 + (lane >> 3);
           const uint4 v = ptx::ld_shared_v4(slab + r * 128 + ((chunk ^ (r & 7)) << 4));
-          if (pitched) {
-            ptx::st_v4(step_dst + i * 4 * pitch, v);
-            continue;
-          }
           const int g = row0 + r;
           uint16_t* dst;
           if (local) {
-            dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(L, g, col);
+            dst = reinterpret_cast<uint16_t*>(p.epi_base[0]) + layout_offset(p.epi_layout, g, col);
           } else if (p.own_mode == OWN_BLOCK) {
             const int o = g / p.rows_per_owner;
             const int lr = g - o * p.rows_per_owner;
@@ -1113,16 +1144,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         }
         __syncwarp();
       }
-      if (p.ssq != nullptr) {
-        p.ssq[(static_cast<long long>(row0 / BM) * p.TN + n_blk) * BM + q * 32 + lane] = ssq;
-        __syncwarp();
-      }
-
       // ---- progress: this warp's slab of the tile is written ----
       // (__syncwarp above ordered every lane's stores before this release; the
       // signalling warp acquires it and publishes the tile at system scope, so
       // that no epilogue warp ever waits for a system-scope fence.)
-      if (lane == 0) ptx::st_release_cta_shared(&epi_prog[q], static_cast<uint32_t>(it + 1));
+      if (lane == 0) ptx::st_release_cta_shared(&epi_prog[warp - 4], static_cast<uint32_t>(it + 1));
     }
   } else if (warp == 3) {
     // ===================== signalling =====================
@@ -1139,8 +1165,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         uint32_t spins = 0;
         while (true) {
           uint32_t lo = ptx::ld_acquire_cta_shared(&epi_prog[0]);
-#pragma unroll
-          for (int w = 1; w < 4; ++w) {
+          for (int w = 1; w < T::EPI_WARPS * p.epi_halves; ++w) {
             const uint32_t v = ptx::ld_acquire_cta_shared(&epi_prog[w]);
             lo = v < lo ? v : lo;
           }
@@ -1198,7 +1223,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
 
   int group = 0;  // row group of this warp in the reduce phase
   int wg = 0;     // warp inside the group
-  if (warp >= kGemmWarps) {
+  if (warp >= kGemmWarps && p.epi_halves == 1) {
     // ===================== communication warps =====================
     const int cw = warp - kGemmWarps;
     if (p.ag_push) {
@@ -1266,11 +1291,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     group = 0;  // reduces rows from the first cycle on
     wg = cw;
   } else {
-    // ===================== teardown of the GEMM phase (GEMM warps only) =====================
+    // ============ teardown of the GEMM phase (GEMM warps, and the communication warps that shared the epilogue) ============
+    const int gemm_threads = p.epi_halves == 2 ? kThreads : kGemmThreads;
     __syncwarp();
     ptx::tc_fence_before_sync();
     if constexpr (CTAS == 2) {
-      ptx::named_barrier_sync(8, kGemmThreads);
+      ptx::named_barrier_sync(8, gemm_threads);
       // The partner may still read this CTA's operands or signal its barriers:
       // each CTA tells the other that its GEMM warps are done and waits (bounded)
       // to hear the same.
@@ -1285,7 +1311,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     // One answer for all GEMM warps: the communication warps may raise the flag at this very moment, and the warps of a
     // row group must either all join the reduce phase, whose barriers have no deadline, or none.  (A warp that gave up
     // above sees its own store, so a failure of the GEMM phase is always in the answer.)
-    const bool gave_up = ptx::named_barrier_or(8, kGemmThreads, *abort_flag != 0);
+    const bool gave_up = ptx::named_barrier_or(8, gemm_threads, *abort_flag != 0);
     if (warp == 2) {
       ptx::tc_fence_after_sync();
       if constexpr (CTAS == 2) ptx::tmem_dealloc_pair(tmem_base, T::TMEM_COLS);

@@ -491,6 +491,12 @@ __device__ __forceinline__ void st_v4(void* p, const uint4& v) {
                "r"(v.w)
                : "memory");
 }
+// Same, 32 bytes (one L2 sector) from eight registers; p on a 32-byte boundary.
+__device__ __forceinline__ void st_v8(void* p, const uint32_t* v) {
+  asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]),
+               "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
 __device__ __forceinline__ void st_shared_v4(uint32_t saddr, const uint4& v) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                : "memory");

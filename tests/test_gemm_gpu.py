@@ -132,3 +132,33 @@ def test_gemm_swiglu(dtype, algo, M, ffn, K, keep):
     with pytest.raises(RuntimeError):
         impl.gemm_swiglu(x, w, guard[:M], 0)      # not a CTA-pair tile
 
+
+
+@pytest.mark.parametrize("offset", [0, 8])
+@pytest.mark.parametrize("algo,M,N", [(2, 128, 64), (7, 384, 192), (1, 128, 128), (0, 256, 768), (5, 256, 64), (8, 512, 2560)])
+@pytest.mark.parametrize("glu", [False, True])
+def test_gemm_result_on_16_and_32_byte_boundaries(offset, algo, M, N, glu):
+    # eight warps share a tile's columns (one chunk of 32 each, an even and an odd number of them) and store 32 bytes at a
+    # time where the result allows it, 16 elsewhere; the values around the result stay as they were
+    if glu and (ALGO_TILES[algo][0] != 256 or ALGO_TILES[algo][1] < 128):
+        pytest.skip("the gated form needs a pair tile of 128 columns")
+    K = 72
+    torch.manual_seed(N)
+    A = torch.randn(M, K, device="cuda", dtype=torch.float16)
+    B = (torch.randn(N, K, device="cuda") / K ** 0.5).half()
+    n = N // 2 if glu else N
+    buf = torch.full((M * n + 32,), 5.0, device="cuda", dtype=torch.float16)
+    C = buf[offset:offset + M * n].view(M, n)
+    assert C.data_ptr() % 32 == 2 * offset
+    impl = _impl()
+    impl.set_keep_tile(True)
+    (impl.gemm_swiglu if glu else impl.cutlass_gemm)(A, B, C, algo)
+    torch.cuda.synchronize()
+    impl.check_status()
+    want = A.double() @ B.double().t()
+    if glu:
+        gate, up = want.chunk(2, dim=-1)
+        want = torch.nn.functional.silu(gate) * up
+    # one rounding to 11 bits of fp32 sums
+    assert ((C.double() - want).abs() <= 2 ** -10.9 * want.abs() + 1e-5).all()
+    assert bool((buf[:offset] == 5).all()) and bool((buf[offset + M * n:] == 5).all())
