@@ -136,7 +136,7 @@ static std::vector<int64_t> tile_walk_op(int64_t TM, int64_t TN, int64_t raster_
 
 // The tile configuration that a one-rank GEMM which names `algo` runs on `ctas` CTAs (0 = all SMs of the device).  For
 // tests and for reasoning about a call's time; needs no GPU when `ctas` is given.
-static int64_t planned_algo_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu) {
+static LaunchPlan plan_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu, bool norm) {
   TORCH_CHECK(M > 0 && N > 0 && K > 0 && algo >= 0 && algo < kNumAlgos && ctas >= 0, "planned_algo: bad arguments");
   GemmOperands g{};
   g.M = static_cast<int>(M);
@@ -144,8 +144,19 @@ static int64_t planned_algo_op(int64_t M, int64_t N, int64_t K, int64_t algo, in
   g.K = static_cast<int>(K);
   g.algo = static_cast<int>(algo);
   g.any_tile = 1;
+  g.may_keep = norm ? 1 : 0;
   g.glu = glu ? 1 : 0;
-  return plan_algo(g, ctas > 0 ? static_cast<int>(ctas) : device_sm_count());
+  return plan_launch(g, ctas > 0 ? static_cast<int>(ctas) : device_sm_count());
+}
+static int64_t planned_algo_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu) {
+  return plan_op(M, N, K, algo, ctas, glu, false).algo;
+}
+// The whole plan of a call on one rank: configuration, tile columns, and for a GEMM with RMSNorm whose rows stay on the chip
+// the tile rows of a wave (else 0).
+static std::vector<int64_t> planned_tile_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu,
+                                            bool norm) {
+  const LaunchPlan p = plan_op(M, N, K, algo, ctas, glu, norm);
+  return {p.algo, p.bn, p.rows};
 }
 
 }  // namespace fo
@@ -239,4 +250,5 @@ TORCH_LIBRARY(flashoverlap_op, m) {
   m.def("add_rmsnorm", &fo::add_rmsnorm_op);
   m.def("tile_walk", &fo::tile_walk_op);
   m.def("planned_algo", &fo::planned_algo_op);
+  m.def("planned_tile", &fo::planned_tile_op);
 }

@@ -107,6 +107,7 @@ struct alignas(64) FusedParams {
 
   int M, N, K;
   int TM, TN;        // tile grid; the last tile row and column may reach past M and N (whole blocks of 128 rows, 64 columns)
+  int bn;            // columns of a tile (a multiple of 32, at most those of the configuration that runs)
   int algo;          // tile configuration that runs (index of the table), for the host
   int trace_cols;    // phase trace: columns that count as one tile (those of the tile the caller named)
   int raster_group;  // tile rows walked column-major together (L2 reuse of B)
@@ -166,6 +167,12 @@ struct alignas(64) FusedParams {
   // [M / 128][TN][128], written by the epilogue.  The reduce phase then scales rows without a pass of its own
   // over them (norm_stream).  Null = the row workers find the sums.
   float* ssq;
+  // One rank and RMSNorm, all tiles of a row block in the same wave: row statistics are exchanged, the product stays on the
+  // chip and there is no reduce phase (resident_norm).  exchange: one word per row and tile column, [M / 128][TN][128],
+  // all zero between launches; readers: tiles that have read a row block's entries, zero between launches.
+  int resident;
+  uint32_t* exchange;
+  uint32_t* readers;
   int drop_stage;  // norm_stream: the staged product is scratch, its lines need not reach memory once they are read
   // Counter set of the next call, zeroed by this launch (one rank: nobody else raises it).  Null = the host clears it.
   uint32_t* clear_words;

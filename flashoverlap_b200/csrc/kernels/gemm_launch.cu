@@ -83,9 +83,7 @@ cudaError_t prepare_fused(int algo, DType dtype) {
 
 namespace {
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
-int tile_columns(const GemmOperands& g, const TileConfig& tc) {
-  return g.glu ? ceil_div(g.N / 2, tc.bn / 2) : ceil_div(g.N, tc.bn);
-}
+int tile_columns(const GemmOperands& g, int bn) { return g.glu ? ceil_div(g.N / 2, bn / 2) : ceil_div(g.N, bn); }
 bool can_run(const GemmOperands& g, const TileConfig& tc) { return !g.glu || (tc.ctas == 2 && tc.bn >= 128); }
 
 // Estimated time in ns of a GEMM in one tile configuration: whole waves of tiles, each as long as K, plus what every wave
@@ -111,7 +109,7 @@ static_assert(sizeof(kWholeCalls) / sizeof(kWholeCalls[0]) == kNumAlgos, "one en
 
 double estimate_ns(const TileTime (&times)[kNumAlgos], const GemmOperands& g, int algo, int ctas) {
   const TileConfig& tc = kAlgoTable[algo];
-  const int waves = ceil_div(ceil_div(g.M, tc.bm) * tile_columns(g, tc), std::max(1, ctas / tc.ctas));
+  const int waves = ceil_div(ceil_div(g.M, tc.bm) * tile_columns(g, tc.bn), std::max(1, ctas / tc.ctas));
   const double operands = 2.0 * (static_cast<double>(g.M) + g.N) * g.K / 6000;  // bytes at 6 TB/s
   return std::max(waves * static_cast<double>(g.K) * times[algo].per_k, operands) + times[algo].fixed +
          times[algo].wave * waves;
@@ -122,7 +120,7 @@ double estimate_ns(const TileTime (&times)[kNumAlgos], const GemmOperands& g, in
 // calls.  On 700 shapes other than the fitted ones, the tile that runs is more than 3 % slower than the named one in 0.3 %
 // of the calls that name the first of gather_algo_candidates (5.1 % without the second condition) and in 1.4 % (4.1 %) of
 // those that name any other; it is 1.25 times as fast on average over all.
-int plan_algo(const GemmOperands& g, int ctas) {
+static int plan_algo(const GemmOperands& g, int ctas) {
   if (!g.any_tile) return g.algo;
   int best = g.algo;
   double best_ns = 0.97 * estimate_ns(kSingleWave, g, g.algo, ctas);
@@ -134,6 +132,71 @@ int plan_algo(const GemmOperands& g, int ctas) {
     }
   }
   return estimate_ns(kWholeCalls, g, best, ctas) <= estimate_ns(kWholeCalls, g, g.algo, ctas) ? best : g.algo;
+}
+
+namespace {
+// GEMM + RMSNorm of one rank, staged and resident, in ns.  Both are least-squares fits (of the logarithm; 8 % rms) to 900
+// random shapes (M 128 to 16384, N 1024 to 14336, K 256 to 28672, both types), timed call after call in every form.  A value
+// of K costs what the tensor cores take for bn columns (more as the chip warms up), or what a CTA takes in: 107 to 119 GB/s
+// from L2, less where the rows of 128 bytes that the copy engine reads straddle two lines, or two sectors.
+struct NormFit {
+  double mma, droop, rate_one, rate_pair, odd_line, odd_sector;
+};
+double per_k_ns(const NormFit& f, int K, int ctas, int bn, int waves) {
+  const double mma = f.mma * bn * (1 + f.droop * std::min(1.0, waves * static_cast<double>(K) * f.mma * bn / 200e3));
+  const double intake = 2.0 * (128 + bn / ctas) / (ctas == 1 ? f.rate_one : f.rate_pair) *
+                        (K % 16 != 0 ? f.odd_sector : K % 64 != 0 ? f.odd_line : 1.0);
+  return std::max(mma, intake);
+}
+double staged_ns(const GemmOperands& g, int algo, int ctas) {
+  constexpr NormFit kFit = {0.0210, 0.09, 117.2, 108.9, 1.04, 1.39};
+  const TileConfig& tc = kAlgoTable[algo];
+  const int waves = ceil_div(ceil_div(g.M, tc.bm) * tile_columns(g, tc.bn), std::max(1, ctas / tc.ctas));
+  const double main = waves * static_cast<double>(g.K) * per_k_ns(kFit, g.K, tc.ctas, tc.bn, waves);
+  return std::max(main, 2.0 * (static_cast<double>(g.M) + g.N) * g.K / 4230) + 10700 + 0.5 * tc.bn +
+         0.96e-3 * g.M * static_cast<double>(g.N) + (tc.ctas == 2 ? 780 : 0);
+}
+double resident_ns(const GemmOperands& g, const TileConfig& tc, int bn, int tn, int rows, int waves) {
+  constexpr NormFit kFit = {0.0211, 0.05, 118.9, 107.0, 1.10, 1.37};
+  const double main = g.K * per_k_ns(kFit, g.K, tc.ctas, bn, waves) + 1760;
+  // collecting a row's statistics, and the whole epilogue of a tile from its last MMA to its last store
+  const double collect = 19 * tn + 805 * ceil_div(tn, 40), epilogue = 380 + 16.8 * bn + collect;
+  const double hbm = std::min(3960.0, 64.0 * rows * tn * tc.ctas);  // few CTAs do not fill it
+  return std::max((waves - 1) * std::max(main, epilogue) + main, 2.0 * (static_cast<double>(g.M) + g.N) * g.K / hbm) + 4480 +
+         4.8 * bn + collect + (tc.ctas == 2 ? 1480 : 0);
+}
+}  // namespace
+
+// A resident RMSNorm (see resident_norm) takes as many tile rows per wave as have all their tiles in it.  It runs where it
+// is expected to save 5 %: in 89 % of the fitted shapes, slower than the staged form by more than 3 % in 1.6 % of all, 1.17
+// times as fast over all (1.19 with the best choice each time).  4096 x 8192 x 1024 fp16 88 -> 74 us (one run in turn; the
+// chip warm), 2048 x 4096 x 2048 43.5 -> 35.8, 4096 x 4096 x 512 34.6 -> 28.9, 128 x 8192 x 1024 14.2 -> 12.2.  From 1.5e11
+// multiply-adds on (some 220 us) every form runs at the power cap, and the staged one, whose tiles have the full width, comes
+// out the same or better: 4096 x 8192 x 8192 464 against 474, 8192 x 8192 x 28672 bf16 2950 against 3098.
+// Among forms within the fit's error the configuration of a call without RMSNorm is kept.
+LaunchPlan plan_launch(const GemmOperands& g, int ctas) {
+  LaunchPlan plan{plan_algo(g, ctas), 0, 0};
+  plan.bn = kAlgoTable[plan.algo].bn;
+  if (!g.any_tile || !g.may_keep || static_cast<double>(g.M) * g.N * g.K >= 1.5e11) return plan;
+  const int plain = plan.algo;
+  const double staged = 0.95 * staged_ns(g, plain, ctas);
+  double best = staged;
+  for (int algo : {8, 9, 0, 6, 7}) {
+    const TileConfig& tc = kAlgoTable[algo];
+    const int slots = ctas / tc.ctas, tm = ceil_div(g.M, tc.bm);
+    for (int bn = tc.bn; bn >= 32 && (tc.bn == 64 || bn > tc.bn / 2); bn -= 32) {
+      const int tn = ceil_div(g.N, bn), rows = std::min(tm, slots / tn);
+      if (rows == 0) continue;
+      double ns = resident_ns(g, tc, bn, tn, rows, ceil_div(tm, rows));
+      if (ns >= staged) continue;
+      if (algo == plain) ns *= 0.92;
+      if (ns < best) {
+        best = ns;
+        plan = LaunchPlan{algo, bn, rows};
+      }
+    }
+  }
+  return plan;
 }
 
 cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t stream, const char** why) {
@@ -167,14 +230,16 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
   int grid = g.sm_count > 0 ? g.sm_count : device_sm_count();
   const int sms = device_sm_count();
   if (grid > sms) grid = sms;  // every CTA must be resident: CTAs wait on one another's output
-  const int algo = plan_algo(g, grid);
+  const LaunchPlan plan = plan_launch(g, grid);
+  const int algo = plan.algo;
   p.algo = algo;
+  p.bn = plan.bn;
   p.trace_cols = tc.bn;
   tc = kAlgoTable[algo];
   // every CTA stages 128 rows of A and (for a CTA pair) half of the B tile, 64 K-values per box
   const int a_rows = g.a_rows > 0 && g.a_rows < g.M ? g.a_rows : g.M;  // the copy engine fills the rows after them with zero
   if (!make_tensor_map(&p.tmA, g.A, a_rows, g.K, 128, g.dtype) ||
-      !make_tensor_map(&p.tmB, g.B, g.N, g.K, tc.bn / tc.ctas, g.dtype)) {
+      !make_tensor_map(&p.tmB, g.B, g.N, g.K, p.bn / tc.ctas, g.dtype)) {
     *why = "cuTensorMapEncodeTiled failed";
     return cudaErrorInvalidValue;
   }
@@ -197,8 +262,16 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
   p.N = g.N;
   p.K = g.K;
   p.TM = ceil_div(g.M, tc.bm);
-  p.TN = tile_columns(g, tc);
-  if (algo != g.algo && p.reduce) p.flag_target = static_cast<uint32_t>(p.TN);
+  p.TN = tile_columns(g, p.bn);
+  if (g.any_tile && p.reduce) p.flag_target = static_cast<uint32_t>(p.TN);
+  p.resident = plan.rows > 0 ? 1 : 0;
+  if (p.resident) {
+    p.reduce = 0;
+    p.epi_base[0] = p.out[p.me];
+    p.raster_group = plan.rows;
+    p.raster_taper = 0;
+    grid = tc.ctas * plan.rows * p.TN;
+  }
   const OutLayout& L = p.epi_layout;
   p.epi_direct = (p.own_mode == OWN_SINGLE || p.nvls) && (!L.tiled || (L.row_map == nullptr && L.bm % 32 == 0 && L.bn % 64 == 0));
   p.epi_wide = reinterpret_cast<uintptr_t>(p.epi_base[0]) % 32 == 0 && (L.tiled || L.ld % 16 == 0);

@@ -39,12 +39,19 @@ struct GemmOperands {
   // 1 = the result does not depend on the tile shape (natural or tile-ordered output on one GPU, nothing counts
   // tiles): `algo` then says which shapes are accepted, and the launch takes the configuration plan_algo finds.
   int any_tile;
+  // 1 = GEMM + RMSNorm of one rank whose product nobody asks for: it may stay on the chip (FusedParams::resident).
+  int may_keep;
   // 1 = gated form (see FusedParams::glu): the result has N / 2 columns.  CTA-pair tiles of at least 128 columns.
   int glu;
 };
 
-// The tile configuration (index of the table) in which a GEMM on `ctas` CTAs is expected to take least time.
-int plan_algo(const GemmOperands& g, int ctas);
+// What a launch runs: the tile configuration (index of the table), the width of its tiles, and for a resident RMSNorm the
+// tile rows of a wave (0: not resident).
+struct LaunchPlan {
+  int algo, bn, rows;
+};
+// The plan with which a GEMM on `ctas` CTAs is expected to take least time.
+LaunchPlan plan_launch(const GemmOperands& g, int ctas);
 
 // Fills p.tmA / p.tmB / shape fields from `g`, validates shapes, launches.
 // Everything else in `p` must already be set by the caller; p.algo says

@@ -34,6 +34,8 @@ void FusedEngine::launch(const GemmOperands& g, FusedParams& p, cudaStream_t str
 }
 
 FusedEngine::~FusedEngine() {
+  if (exchange_ != nullptr) cudaFree(exchange_);
+  exchange_ = nullptr;
   if (status_dev_ != nullptr) cudaFree(status_dev_);
   if (status_host_ != nullptr) cudaFreeHost(status_host_);
   status_dev_ = nullptr;
@@ -85,6 +87,19 @@ size_t workspace_bytes(long long elems) {
 }  // namespace
 
 void FusedEngine::carve_workspace(long long elems) {
+  if (world_ == 1) {
+    // row statistics of tiles of 32 columns at least, and the counters of kMaxTileRows row blocks
+    const size_t bytes = (static_cast<size_t>(elems) / 32 + kMaxTileRows) * sizeof(uint32_t);
+    if (bytes > exchange_bytes_) {
+      if (exchange_ != nullptr) cudaFree(exchange_);
+      exchange_ = nullptr;
+      exchange_bytes_ = 0;
+      check(cudaMalloc(reinterpret_cast<void**>(&exchange_), bytes), "cudaMalloc(row statistics)");
+      exchange_bytes_ = bytes;
+    }
+    check(cudaMemset(exchange_, 0, exchange_bytes_), "cudaMemset(row statistics)");
+    check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+  }
   const size_t mat = static_cast<size_t>(elems) * 2;
   heap_.reset_allocator();
   for (int s = 0; s < 2; ++s) ws_.stage[s] = heap_.alloc(mat, 1024);
@@ -337,6 +352,10 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
     p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
     p.drop_stage = drop_stage(g) ? 1 : 0;
     g.any_tile = tile_is_free() ? 1 : 0;
+    // (the traces record the phases of the staged form)
+    g.may_keep = p.phase_trace == nullptr && p.row_trace == nullptr ? 1 : 0;
+    p.readers = exchange_;
+    p.exchange = exchange_ + kMaxTileRows;
   }
   // with one rank there is nobody to deliver to: rows go to the result buffer like a reduce-scatter's
   p.bcast = world_ > 1 ? 1 : 0;
@@ -420,6 +439,10 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
     p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
     p.drop_stage = drop_stage(g) ? 1 : 0;
     g.any_tile = tile_is_free() ? 1 : 0;
+    // (the traces record the phases of the staged form)
+    g.may_keep = p.phase_trace == nullptr && p.row_trace == nullptr ? 1 : 0;
+    p.readers = exchange_;
+    p.exchange = exchange_ + kMaxTileRows;
   }
   p.bcast = 0;
   p.job_counter = flag_ptr(rank_, set) + kFlagJob;
@@ -716,6 +739,7 @@ void FusedEngine::reset_counters() {
   if (heap_.valid()) {
     for (int s = 0; s < 2; ++s) check(cudaMemset(flag_ptr(rank_, s), 0, kFlagWords * 4), "cudaMemset(counters)");
     check(cudaMemset(heap_.local(ws_.misc), 0, 4096), "cudaMemset(counters)");
+    if (exchange_ != nullptr) check(cudaMemset(exchange_, 0, exchange_bytes_), "cudaMemset(row statistics)");
     check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
   }
   if (world_ > 1 && all_gather_) {

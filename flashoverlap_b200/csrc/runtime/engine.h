@@ -214,6 +214,10 @@ class FusedEngine {
   AllGatherFn all_gather_;
   SymmHeap heap_;
   Workspace ws_;
+  // One rank: row statistics of a resident RMSNorm (FusedParams::readers, then FusedParams::exchange), as large as the
+  // workspace asks for and allocated with it.
+  uint32_t* exchange_ = nullptr;
+  size_t exchange_bytes_ = 0;
   StatusWord* status_dev_ = nullptr;
   StatusWord* status_host_ = nullptr;    // mirror of the status word in mapped host memory (host address)
   StatusWord* status_mirror_ = nullptr;  // the same memory as the device sees it

@@ -69,3 +69,29 @@ def test_tile_table_matches_the_python_copy():
     assert obj.num_algos() == len(ALGO_TILES)
     for i, tile in enumerate(ALGO_TILES):
         assert tuple(obj.algo_tile(i))[:3] == tuple(tile)
+
+
+def test_resident_plans_fit_the_chip():
+    # every tile of a row block in one wave, whole chunks of 32 columns, tiles inside their configuration
+    import random
+
+    from flashoverlap_b200.utils.config import ALGO_TILES
+
+    rng = random.Random(3)
+    plan, seen = torch.ops.flashoverlap_op.planned_tile, 0
+    for _ in range(400):
+        ctas = rng.choice([1, 2, 37, 100, 148])
+        algo = rng.randrange(len(ALGO_TILES))
+        m, n = rng.randrange(1, 65) * ALGO_TILES[algo][0], rng.randrange(1, 40) * ALGO_TILES[algo][1]
+        k = rng.randrange(1, 1024) * 8
+        a, bn, rows = plan(m, n, k, algo, ctas, False, True)
+        bm, width, _ = ALGO_TILES[a]
+        assert plan(m, n, k, algo, ctas, False, False)[2] == 0
+        if rows:
+            seen += 1
+            tiles = -(-n // bn)
+            assert bn % 32 == 0 and 0 < bn <= width and 0 < rows <= -(-m // bm)
+            assert rows * tiles * (bm // 128) <= ctas
+        else:
+            assert bn == width
+    assert seen > 100

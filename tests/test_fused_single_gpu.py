@@ -678,3 +678,87 @@ def test_host_feeder_double_buffers_inputs():
         seen.append(y)
     torch.cuda.synchronize()
     assert [float(v) for v in seen] == [0.0, 1.0, 2.0, 3.0, 4.0]
+
+
+RESIDENT = [
+    # M, N, K, named configuration, plan (configuration, tile columns, tile rows per wave)
+    (128, 64, 64, 2, (7, 32, 1)),           # the narrowest tiles: the second half of the columns is empty
+    (128, 8192, 1024, 7, (6, 128, 1)),      # one row block over 64 CTAs: statistics in more than one batch
+    (384, 4544, 200, 2, (6, 128, 3)),       # the last tile column holds 64
+    (2048, 8256, 64, 5, (0, 224, 4)),       # four waves, seven chunks of columns for two warps
+    (1152, 5120, 1720, 1, (8, 224, 3)),     # pairs, the second half of the last tile row is empty; two waves
+    (4096, 8192, 1024, 8, (8, 224, 2)),     # every SM, eight waves
+    (2048, 4096, 2048, 8, (8, 256, 4)),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K,algo,plan", RESIDENT)
+def test_resident_norm_matches_the_staged_form(dtype, M, N, K, algo, plan):
+    # rows that stay on the chip between the product and its RMSNorm, call after call with another shape in between (the
+    # exchange has to be left clean), results on a 32-byte boundary and on a 16-byte one; the same call with the named tile
+    # kept goes through the staging buffer
+    assert tuple(torch.ops.flashoverlap_op.planned_tile(M, N, K, algo, 0, False, True)) == plan
+    A, B, W = make_inputs(M, N, K, dtype, seed=N)
+    A2, B2, W2 = make_inputs(256, 1024, 264, dtype, seed=1)
+    impl = make_impl()
+    y = A.double() @ B.double().t()
+    want = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * W.double()
+    y2 = A2.double() @ B2.double().t()
+    want2 = y2 * torch.rsqrt(y2.pow(2).mean(-1, keepdim=True) + 1e-5) * W2.double()
+    # the product, its scaling and the weight are each rounded to 11 or 8 bits
+    rel = 2 ** -9.3 if dtype == torch.float16 else 2 ** -6.3
+    buf = torch.empty(M * N + 32, device="cuda", dtype=dtype)
+    first = None
+    for offset in (0, 8, 0):
+        buf.fill_(9.0)
+        D = buf[offset:offset + M * N].view(M, N)
+        impl.gemm_reducescatter_fused(A, B, D, W, 1e-5, algo, False)
+        assert impl.last_algo() == plan[0]
+        small = impl.gemm_allreduce_fused(A2, B2, W2, 1e-5, 2)
+        torch.cuda.synchronize()
+        impl.check_status()
+        assert ((D.double() - want).abs() <= rel * want.abs() + 1e-4).all()
+        assert ((small.double() - want2).abs() <= rel * want2.abs() + 1e-4).all()
+        assert bool((buf[:offset] == 9).all()) and bool((buf[offset + M * N:] == 9).all())
+        assert first is None or torch.equal(D, first)      # the same bits every time
+        first = D.clone()
+    impl.set_keep_tile(True)
+    out = impl.gemm_allreduce_fused(A, B, W, 1e-5, algo)
+    torch.cuda.synchronize()
+    impl.check_status()
+    assert impl.last_algo() == algo
+    assert ((out.double() - want).abs() <= rel * want.abs() + 1e-4).all()
+
+
+def test_resident_norm_in_a_graph():
+    # replays run with the parameters of the capture: what one replay leaves in the exchange would be taken for the next
+    # one's statistics
+    M, N, K = 384, 4544, 200
+    A, B, W = make_inputs(M, N, K, torch.float16)
+    impl = make_impl()
+    D = torch.empty(M, N, device="cuda", dtype=torch.float16)
+    E = torch.empty_like(D)
+
+    def calls():
+        impl.gemm_reducescatter_fused(A, B, D, W, 1e-5, 2, False)      # RMSNorm: resident
+        impl.gemm_reducescatter_fused(A, B, E, None, 1e-5, 2, False)   # none (an even number of fused calls)
+
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        calls()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        calls()
+    for seed in range(3):
+        A2, _, _ = make_inputs(M, N, K, torch.float16, seed=10 + seed)
+        A.copy_(A2 * (seed + 1))
+        graph.replay()
+        torch.cuda.synchronize()
+        impl.check_status()
+        y = A.double() @ B.double().t()
+        want = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * W.double()
+        # the product, its scaling and the weight are each rounded to 11 bits
+        assert ((D.double() - want).abs() <= 2 ** -9.3 * want.abs() + 1e-4).all()
+        assert ((E.double() - y).abs() <= 2 ** -10.9 * y.abs() + 1e-5).all()
