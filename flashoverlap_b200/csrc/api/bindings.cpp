@@ -145,18 +145,19 @@ static LaunchPlan plan_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t
   g.algo = static_cast<int>(algo);
   g.any_tile = 1;
   g.may_keep = norm ? 1 : 0;
+  g.normed = g.may_keep;
   g.glu = glu ? 1 : 0;
   return plan_launch(g, ctas > 0 ? static_cast<int>(ctas) : device_sm_count());
 }
 static int64_t planned_algo_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu) {
   return plan_op(M, N, K, algo, ctas, glu, false).algo;
 }
-// The whole plan of a call on one rank: configuration, tile columns, and for a GEMM with RMSNorm whose rows stay on the chip
-// the tile rows of a wave (else 0).
+// The whole plan of a call on one rank: configuration, tile columns, for a GEMM with RMSNorm whose rows stay on the chip the
+// tile rows of a wave (else 0), and over how many CTAs the K of a tile is split.
 static std::vector<int64_t> planned_tile_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu,
                                             bool norm) {
   const LaunchPlan p = plan_op(M, N, K, algo, ctas, glu, norm);
-  return {p.algo, p.bn, p.rows};
+  return {p.algo, p.bn, p.rows, p.split};
 }
 
 }  // namespace fo

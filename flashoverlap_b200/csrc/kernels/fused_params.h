@@ -108,6 +108,7 @@ struct alignas(64) FusedParams {
   int M, N, K;
   int TM, TN;        // tile grid; the last tile row and column may reach past M and N (whole blocks of 128 rows, 64 columns)
   int bn;            // columns of a tile (a multiple of 32, at most those of the configuration that runs)
+  int split;         // > 1: K of a tile is split over that many CTAs of a cluster (single-CTA configurations, no reduce phase)
   int algo;          // tile configuration that runs (index of the table), for the host
   int trace_cols;    // phase trace: columns that count as one tile (those of the tile the caller named)
   int raster_group;  // tile rows walked column-major together (L2 reuse of B)

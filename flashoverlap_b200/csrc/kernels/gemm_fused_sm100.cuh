@@ -928,6 +928,90 @@ __device__ __forceinline__ void resident_clear(const FusedParams& p, uint32_t ct
   }
 }
 
+// Epilogue of a tile whose K is split over the CTAs of a cluster (one tile per cluster): every CTA owns a stretch of the
+// tile's columns, gets the other parts' sums for it through distributed shared memory (in place of the operands, which
+// everybody has read by then), adds them up in the order of the parts and stores.  Two warps to a quarter of the rows share
+// the chunks of 32 columns.
+template <bool BF16>
+__device__ __forceinline__ void split_epilogue(const FusedParams& p, uint32_t tmem_base, uint64_t* tfull_bar,
+                                               uint64_t* split_bar, uint32_t inbox, int part, int q, int half, int lane,
+                                               uint64_t deadline, volatile uint32_t* abort_flag) {
+  constexpr int BM = 128;
+  constexpr uint32_t CHUNK = 32 * 32 * 4;  // 32 rows x 32 columns of fp32; [8 pieces of 16 bytes][32 rows]
+  int m_blk, n_blk;
+  tile_coords(p, static_cast<int>(blockIdx.x) / p.split, m_blk, n_blk);
+  const int col0 = n_blk * p.bn;
+  const int row0 = m_blk * BM + q * 32;
+  const int chunks = min(p.bn, p.N - col0) / 32;
+  const int most = (chunks + p.split - 1) / p.split;  // chunks of an owner, at most
+  auto first_of = [&](int owner) { return chunks * owner / p.split; };
+  auto give_up = [&](uint32_t where) {
+    if (lane == 0) {
+      report_error(p, ST_TIMEOUT_PIPE, where, part, blockIdx.x);
+      *abort_flag = 1;
+    }
+    __syncwarp();
+  };
+  if (!__all_sync(0xffffffffu, ptx::mbar_wait(tfull_bar, 0u, deadline))) return give_up(0x400u);
+  ptx::tc_fence_after_sync();
+  // all MMAs of this CTA are complete: its operands may be overwritten
+  if (q == 0 && half == 0 && lane < p.split && lane != part) {
+    ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&split_bar[0]), lane));
+  }
+  if (!__all_sync(0xffffffffu, ptx::mbar_wait_cluster(&split_bar[0], 0u, deadline))) return give_up(0x800u);
+  const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+  for (int i = 1; i < p.split; ++i) {
+    int owner = part + i;  // start with the next part: the parts write to different CTAs
+    if (owner >= p.split) owner -= p.split;
+    const int from = part < owner ? part : part - 1;  // this part's place in the owner's inbox
+    const uint32_t box = ptx::mapa_shared(inbox, owner);
+    for (int c = first_of(owner) + half; c < first_of(owner + 1); c += 2) {
+      uint32_t r[32];
+      ptx::tmem_ld_32x32b_x32(t_row + c * 32, r);
+      ptx::tmem_ld_wait();
+      const uint32_t dst = box + ((from * most + c - first_of(owner)) * 4 + q) * CHUNK + lane * 16;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        ptx::st_cluster_v4(dst + e * 512, make_uint4(r[4 * e], r[4 * e + 1], r[4 * e + 2], r[4 * e + 3]));
+      }
+    }
+    __syncwarp();  // every lane's stores before the release
+    if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&split_bar[1]), owner));
+  }
+  if (!__all_sync(0xffffffffu, ptx::mbar_wait_cluster(&split_bar[1], 0u, deadline))) return give_up(0x900u);
+  const OutLayout& L = p.epi_layout;
+  const long long pitch = L.tiled ? static_cast<long long>(L.rldn) * L.bn : L.ld;
+  uint16_t* const base = reinterpret_cast<uint16_t*>(p.epi_base[0]) + lane * pitch;
+  for (int c = first_of(part) + half; c < first_of(part + 1); c += 2) {
+    uint32_t r[32], o[16];
+    ptx::tmem_ld_32x32b_x32(t_row + c * 32, r);
+    ptx::tmem_ld_wait();
+    float sum[32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e) sum[e] = part == 0 ? __uint_as_float(r[e]) : 0.f;
+    for (int s = 0; s < p.split; ++s) {
+      if (s == part) {
+        if (s == 0) continue;
+#pragma unroll
+        for (int e = 0; e < 32; ++e) sum[e] += __uint_as_float(r[e]);
+        continue;
+      }
+      const uint32_t src = inbox + (((s < part ? s : s - 1) * most + c - first_of(part)) * 4 + q) * CHUNK + lane * 16;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const uint4 v = ptx::ld_shared_v4(src + e * 512);
+        sum[4 * e] += __uint_as_float(v.x);
+        sum[4 * e + 1] += __uint_as_float(v.y);
+        sum[4 * e + 2] += __uint_as_float(v.z);
+        sum[4 * e + 3] += __uint_as_float(v.w);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) o[e] = pack2<BF16>(sum[2 * e], sum[2 * e + 1]);
+    store_row32(base + layout_offset(L, row0, col0 + c * 32), o, p.epi_wide);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
@@ -937,8 +1021,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
   constexpr int BM = T::BM, BK = T::BK, STAGES = T::STAGES, TILE_M = T::TILE_M;
   // rank inside the CTA pair; rank 0 (the leader) issues the MMAs of the pair
   const uint32_t cta_rank = CTAS == 2 ? ptx::cluster_ctarank() : 0u;
-  const int first_tile = static_cast<int>(blockIdx.x) / CTAS;
-  const int tile_stride = static_cast<int>(gridDim.x) / CTAS;
+  // tiles split along K (one CTA each part): rank of this CTA's part in its cluster
+  const int split = CTAS == 1 ? p.split : 1;
+  const int part = CTAS == 1 && split > 1 ? static_cast<int>(ptx::cluster_ctarank()) : 0;
+  const int first_tile = static_cast<int>(blockIdx.x) / (CTAS * split);
+  const int tile_stride = static_cast<int>(gridDim.x) / (CTAS * split);
 
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: required by the 128-byte swizzle of TMA and UMMA.
@@ -956,6 +1043,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
   volatile uint32_t* abort_flag = tmem_slot + 1;
   uint32_t* epi_prog = tmem_slot + 4;  // [8] tiles finished by each epilogue warp
   uint64_t* pair_bar = bars + 2 * STAGES + 10;  // teardown handshake between the CTAs of a pair
+  uint64_t* split_bar = pair_bar + 1;  // [2] split tiles: the other parts' operands are read; their sums have arrived here
   GroupScratch* group_scratch = reinterpret_cast<GroupScratch*>(bars + 40);  // [3] row groups of the reduce phase
 
   const int warp = threadIdx.x >> 5;
@@ -970,6 +1058,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       ptx::mbar_init(&tempty_bar[i], T::EPI_WARPS * p.epi_halves * CTAS);  // the leader hears from both epilogues
     }
     ptx::mbar_init(pair_bar, 1);
+    if (split > 1) {
+      ptx::mbar_init(&split_bar[0], split - 1);
+      ptx::mbar_init(&split_bar[1], (split - 1) * 2 * T::EPI_WARPS);
+    }
     *abort_flag = 0;
     for (int i = 0; i < 2 * T::EPI_WARPS; ++i) epi_prog[i] = 0;
     ptx::mbar_fence_init();
@@ -991,7 +1083,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
   }
   ptx::tc_fence_before_sync();
   __syncthreads();
-  if constexpr (CTAS == 2) ptx::cluster_sync();  // both CTAs' barriers exist before anyone signals across
+  if (CTAS == 2 || split > 1) ptx::cluster_sync();  // all CTAs' barriers exist before anyone signals across
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   // Everything above works on this SM (pair) alone and may run under the kernel before this one.
@@ -1015,6 +1107,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
 
   const int num_tiles = p.TM * p.TN;
   const int num_kb = (p.K + BK - 1) / BK;  // a K tail is zero-filled by TMA
+  const int kb_begin = num_kb * part / split, kb_end = num_kb * (part + 1) / split;
   if (p.clear_words != nullptr && warp == 2 && blockIdx.x == 0) {
     for (int i = lane; i < kFlagWords / 4; i += 32) {
       reinterpret_cast<uint4*>(p.clear_words)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -1069,7 +1162,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
             if (tr[4] == ~0ull) tr[4] = ptx::globaltimer_ns();
           }
         }
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1u, deadline)) {
             report_error(p, ST_TIMEOUT_PIPE, 0x100u + stage, kb, t);
             *abort_flag = 1;
@@ -1158,7 +1251,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         }
         ptx::tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BN);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (!ptx::mbar_wait(&full_bar[stage], phase, deadline)) {
             report_error(p, ST_TIMEOUT_PIPE, 0x300u + stage, kb, t);
             *abort_flag = 1;
@@ -1175,7 +1268,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
 #pragma unroll
             for (int k = 0; k < T::ATOM_K / T::UMMA_K; ++k) {
               // advancing K by 16 elements = 32 bytes = 2 descriptor address units
-              const uint32_t acc = (kb | h | k) != 0 ? 1u : 0u;
+              const uint32_t acc = ((kb - kb_begin) | h | k) != 0 ? 1u : 0u;
               if constexpr (CTAS == 2) ptx::umma_f16_ss_pair(d_tmem, da + 2u * k, db + 2u * k, idesc, acc);
               else ptx::umma_f16_ss(d_tmem, da + 2u * k, db + 2u * k, idesc, acc);
             }
@@ -1208,6 +1301,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
       resident_norm<BN, CTAS, BF16>(p, tmem_base, tfull_bar, tempty_bar, tempty_addr0, cta_rank, q, half, lane,
                                     reinterpret_cast<ResidentScratch*>(smem_epi), epi_prog, deadline, abort_flag);
       ok = false;  // no tiles are left for the loop below
+    }
+    if constexpr (CTAS == 1) {
+      if (split > 1) {
+        split_epilogue<BF16>(p, tmem_base, tfull_bar, split_bar, ptx::smem_u32(smem_a), part, q, half, lane, deadline, abort_flag);
+        ok = false;  // its one tile is done
+      }
     }
     for (int t = first_tile; t < num_tiles && ok; t += tile_stride, ++it) {
       int m_blk, n_blk;

@@ -43,9 +43,9 @@ cudaError_t launch_instance(const FusedParams& p, int grid, cudaStream_t stream)
   cfg.stream = stream;
   cudaLaunchAttribute attr[3];
   int n = 0;
-  if (CTAS == 2) {
+  if (CTAS == 2 || p.split > 1) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = 2;
+    attr[n].val.clusterDim.x = CTAS == 2 ? 2 : static_cast<unsigned>(p.split);
     attr[n].val.clusterDim.y = 1;
     attr[n].val.clusterDim.z = 1;
     ++n;

@@ -9,6 +9,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include <cstdlib>
@@ -135,6 +136,64 @@ static int plan_algo(const GemmOperands& g, int ctas) {
 }
 
 namespace {
+// Clusters of so many CTAs that fit the chip together (148 SMs in groups of unequal size); the launch asks for no more.
+constexpr int kMaxSplit = 8;
+constexpr int kClusters[kMaxSplit + 1] = {0, 148, 73, 44, 32, 25, 21, 14, 14};
+
+// A plain GEMM in a tile of any width, its K split over `split` CTAs, in ns: least squares of the logarithm (8 % rms) over
+// 11000 timings, the dozen most promising forms of 1300 random shapes (M 128 to 16384, N 1024 to 14336, K 256 to 28672, both
+// types).  A value of K costs what the tensor cores take (more as the chip warms up), what a CTA takes in (see NormFit), or
+// its part of the least time of a stage; a split adds the way of the sums through distributed shared memory.
+double plain_ns(const GemmOperands& g, int algo, int bn, int split, int ctas) {
+  const TileConfig& tc = kAlgoTable[algo];
+  const int tiles = ceil_div(g.M, tc.bm) * tile_columns(g, bn);
+  const int waves = split > 1 ? 1 : ceil_div(tiles, std::max(1, ctas / tc.ctas));
+  const double k = static_cast<double>(ceil_div(ceil_div(g.K, tc.bk), split)) * tc.bk;
+  const double mma = 0.0203 * bn * (1 + 0.096 * std::min(1.0, waves * static_cast<double>(g.K) * 0.0203 * bn / 200e3));
+  const double intake = 2.0 * (128 + bn / tc.ctas) / (tc.ctas == 1 ? 120.0 : 100.1) *
+                        (g.K % 16 != 0 ? (tc.ctas == 1 ? 1.52 : 1.37) : g.K % 64 != 0 ? 1.10 : 1.0);
+  const double per_k = std::max(std::max(mma, intake) * (tc.bk == 64 ? 0.985 : 1.0), 324.0 / tc.bk);
+  const double main = waves * (k * per_k + 117.0 + 5.84 * bn);
+  const double operands = 2.0 * (static_cast<double>(g.M) + g.N) * g.K / std::min(7833.0, 150.0 * std::min(ctas, tiles * split * tc.ctas));
+  return std::sqrt(main * main + operands * operands) + 4425.0 + 0.52 * bn + (tc.ctas == 2 ? 1231.0 : 0) +
+         (split > 1 ? 1777.0 + 21.2 * bn * (split - 1) / split : 0);
+}
+
+// The plan of a plain GEMM: the configuration that plan_algo finds, in the width that suits the wave, or another one where
+// that is clearly better.  Short K gives little to go by (rounds of the epilogue and of HBM writes), and a split pays where
+// the tiles leave SMs without work.  Over the fitted shapes 1.11 times as fast as plan_algo's tile alone (1.15 with the best
+// choice each time), slower by more than 3 % in 0.2 %.  1152 x 5120 x 1720 bf16 38 -> 28 us (256 x 192), 128 x 10240 x 8192
+// bf16 42 -> 37 (three CTAs per 128 x 256 tile), 128 x 1024 x 28672 113 -> 29 (eight per 128 x 128), 2048 x 8192 x 1024 38.7
+// -> 35.
+LaunchPlan plan_plain(const GemmOperands& g, int base, int ctas) {
+  LaunchPlan plan{base, kAlgoTable[base].bn, 0, 1};
+  const TileConfig& named = kAlgoTable[base];
+  const double base_ns = plain_ns(g, base, named.bn, 1, ctas);
+  const bool idle = ceil_div(g.M, named.bm) * tile_columns(g, named.bn) * named.ctas <= 0.6 * ctas;
+  double best = base_ns;
+  for (int algo = 0; algo < kNumAlgos; ++algo) {
+    const TileConfig& tc = kAlgoTable[algo];
+    if (ctas < tc.ctas || !can_run(g, tc)) continue;
+    const int step = g.glu ? 64 : 32;  // of the gated form every CTA of a pair stages whole chunks
+    for (int bn = tc.bn; bn >= 64 && (bn == tc.bn || bn > tc.bn / 2); bn -= step) {
+      const int tiles = ceil_div(g.M, tc.bm) * tile_columns(g, bn);
+      for (int split = 1; split <= (tc.ctas == 1 ? kMaxSplit : 1); ++split) {
+        if (split > 1 && (split == 7 || tiles > kClusters[split] || tiles * split > ctas || ceil_div(g.K, tc.bk) < 3 * split)) continue;
+        const bool same = algo == base && split == 1;
+        const double ns = plain_ns(g, algo, bn, split, ctas);
+        const double limit = same ? 0.95 : split > 1 ? (idle ? 0.9 : 0.79) : g.K >= 1024 ? 0.92 : 0.78;
+        if (ns >= limit * base_ns) continue;
+        const double rank = same ? 0.97 * ns : ns;  // among equals the configuration stays
+        if (rank < best) {
+          best = rank;
+          plan = LaunchPlan{algo, bn, 0, split};
+        }
+      }
+    }
+  }
+  return plan;
+}
+
 // GEMM + RMSNorm of one rank, staged and resident, in ns.  Both are least-squares fits (of the logarithm; 8 % rms) to 900
 // random shapes (M 128 to 16384, N 1024 to 14336, K 256 to 28672, both types), timed call after call in every form.  A value
 // of K costs what the tensor cores take for bn columns (more as the chip warms up), or what a CTA takes in: 107 to 119 GB/s
@@ -174,10 +233,12 @@ double resident_ns(const GemmOperands& g, const TileConfig& tc, int bn, int tn, 
 // multiply-adds on (some 220 us) every form runs at the power cap, and the staged one, whose tiles have the full width, comes
 // out the same or better: 4096 x 8192 x 8192 464 against 474, 8192 x 8192 x 28672 bf16 2950 against 3098.
 // Among forms within the fit's error the configuration of a call without RMSNorm is kept.
-LaunchPlan plan_launch(const GemmOperands& g, int ctas) {
-  LaunchPlan plan{plan_algo(g, ctas), 0, 0};
+static LaunchPlan find_plan(const GemmOperands& g, int ctas) {
+  LaunchPlan plan{plan_algo(g, ctas), 0, 0, 1};
   plan.bn = kAlgoTable[plan.algo].bn;
-  if (!g.any_tile || !g.may_keep || static_cast<double>(g.M) * g.N * g.K >= 1.5e11) return plan;
+  if (!g.any_tile) return plan;
+  if (!g.normed) return plan_plain(g, plan.algo, ctas);
+  if (!g.may_keep || static_cast<double>(g.M) * g.N * g.K >= 1.5e11) return plan;
   const int plain = plan.algo;
   const double staged = 0.95 * staged_ns(g, plain, ctas);
   double best = staged;
@@ -192,11 +253,29 @@ LaunchPlan plan_launch(const GemmOperands& g, int ctas) {
       if (algo == plain) ns *= 0.92;
       if (ns < best) {
         best = ns;
-        plan = LaunchPlan{algo, bn, rows};
+        plan = LaunchPlan{algo, bn, rows, 1};
       }
     }
   }
   return plan;
+}
+
+// Comparing the forms takes some 3 us of host time, as long as a launch: each thread remembers the plans of its last shapes.
+LaunchPlan plan_launch(const GemmOperands& g, int ctas) {
+  struct Entry {
+    int key[6];
+    LaunchPlan plan;
+  };
+  static thread_local Entry seen[64] = {};
+  if (!g.any_tile) return find_plan(g, ctas);
+  const int key[6] = {g.M, g.N, g.K, g.algo, ctas, g.glu | g.normed << 1 | g.may_keep << 2};
+  const uint32_t slot = (static_cast<uint32_t>(g.M / 32) * 31u + static_cast<uint32_t>(g.N / 32)) * 31u + static_cast<uint32_t>(g.K / 8) * 7u + key[5];
+  Entry& e = seen[slot % 64];
+  if (!std::equal(key, key + 6, e.key)) {  // (no shape has M = 0)
+    e.plan = find_plan(g, ctas);
+    std::copy(key, key + 6, e.key);
+  }
+  return e.plan;
 }
 
 cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t stream, const char** why) {
@@ -234,6 +313,7 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
   const int algo = plan.algo;
   p.algo = algo;
   p.bn = plan.bn;
+  p.split = plan.split;
   p.trace_cols = tc.bn;
   tc = kAlgoTable[algo];
   // every CTA stages 128 rows of A and (for a CTA pair) half of the B tile, 64 K-values per box
@@ -286,6 +366,7 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
     return cudaErrorInvalidValue;
   }
   if (!p.reduce && !p.force_full_grid && grid > p.TM * p.TN * tc.ctas) grid = p.TM * p.TN * tc.ctas;
+  if (p.split > 1) grid = p.TM * p.TN * p.split;  // one tile per cluster
   if (tc.ctas == 2 && grid < 2) grid = 2;
   if (tc.ctas == 2) grid &= ~1;
   return kLaunchTable[algo][g.dtype == DT_BF16 ? 1 : 0](p, grid, stream);

@@ -41,14 +41,16 @@ struct GemmOperands {
   int any_tile;
   // 1 = GEMM + RMSNorm of one rank whose product nobody asks for: it may stay on the chip (FusedParams::resident).
   int may_keep;
+  // 1 = a reduce phase with RMSNorm follows (one rank): the plain plans do not apply.
+  int normed;
   // 1 = gated form (see FusedParams::glu): the result has N / 2 columns.  CTA-pair tiles of at least 128 columns.
   int glu;
 };
 
-// What a launch runs: the tile configuration (index of the table), the width of its tiles, and for a resident RMSNorm the
-// tile rows of a wave (0: not resident).
+// What a launch runs: the tile configuration (index of the table), the width of its tiles, for a resident RMSNorm the tile
+// rows of a wave (0: not resident), and over how many CTAs the K of a tile is split.
 struct LaunchPlan {
-  int algo, bn, rows;
+  int algo, bn, rows, split;
 };
 // The plan with which a GEMM on `ctas` CTAs is expected to take least time.
 LaunchPlan plan_launch(const GemmOperands& g, int ctas);

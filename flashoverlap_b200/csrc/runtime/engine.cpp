@@ -269,6 +269,7 @@ void FusedEngine::gemm_rmsnorm(const GemmOperands& g_in, void* scratch, void* ou
   p.stage = scratch;
   p.ssq = ssq;
   g.any_tile = tile_is_free() ? 1 : 0;
+  g.normed = 1;
   p.flag_target = static_cast<uint32_t>(g.N / tc.bn);
   p.norm = norm.gamma != nullptr;
   p.gamma = norm.gamma;
@@ -352,6 +353,7 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
     p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
     p.drop_stage = drop_stage(g) ? 1 : 0;
     g.any_tile = tile_is_free() ? 1 : 0;
+    g.normed = 1;
     // (the traces record the phases of the staged form)
     g.may_keep = p.phase_trace == nullptr && p.row_trace == nullptr ? 1 : 0;
     p.readers = exchange_;
@@ -439,6 +441,7 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
     p.ssq = static_cast<float*>(heap_.local(ws_.stage[set ^ 1]));  // idle in this call
     p.drop_stage = drop_stage(g) ? 1 : 0;
     g.any_tile = tile_is_free() ? 1 : 0;
+    g.normed = 1;
     // (the traces record the phases of the staged form)
     g.may_keep = p.phase_trace == nullptr && p.row_trace == nullptr ? 1 : 0;
     p.readers = exchange_;

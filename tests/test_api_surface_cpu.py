@@ -84,9 +84,9 @@ def test_resident_plans_fit_the_chip():
         algo = rng.randrange(len(ALGO_TILES))
         m, n = rng.randrange(1, 65) * ALGO_TILES[algo][0], rng.randrange(1, 40) * ALGO_TILES[algo][1]
         k = rng.randrange(1, 1024) * 8
-        a, bn, rows = plan(m, n, k, algo, ctas, False, True)
+        a, bn, rows, split = plan(m, n, k, algo, ctas, False, True)
         bm, width, _ = ALGO_TILES[a]
-        assert plan(m, n, k, algo, ctas, False, False)[2] == 0
+        assert split == 1
         if rows:
             seen += 1
             tiles = -(-n // bn)
@@ -95,3 +95,31 @@ def test_resident_plans_fit_the_chip():
         else:
             assert bn == width
     assert seen > 100
+
+
+def test_plain_plans_fit_the_chip():
+    # widths of whole chunks inside their configuration; a split over single CTAs that all run together, each with K to work
+    # on; of the gated form two halves of whole chunks
+    import random
+
+    from flashoverlap_b200.utils.config import ALGO_TILES
+
+    rng = random.Random(4)
+    plan, narrow, splits = torch.ops.flashoverlap_op.planned_tile, 0, 0
+    for i in range(600):
+        ctas = rng.choice([1, 2, 37, 100, 148, 148, 148])
+        glu = i % 4 == 0
+        algo = rng.choice([3, 4, 8, 9]) if glu else rng.randrange(len(ALGO_TILES))
+        m, n = rng.randrange(1, 17) * ALGO_TILES[algo][0], rng.randrange(1, 40) * ALGO_TILES[algo][1]
+        k = rng.randrange(1, 3500) * 8
+        a, bn, rows, split = plan(m, n, k, algo, ctas, glu, False)
+        bm, width, bk = ALGO_TILES[a]
+        assert rows == 0 and 0 < bn <= width and bn % (64 if glu else 32) == 0
+        assert bm // 128 <= ctas or a == algo       # no pair on a single CTA that was not asked for
+        assert not glu or (bm == 256 and bn >= 128)
+        narrow += bn < width
+        if split > 1:
+            splits += 1
+            assert not glu and bm == 128 and split <= 8
+            assert -(-m // bm) * -(-n // bn) * split <= ctas and -(-k // bk) >= 3 * split
+    assert narrow > 50 and splits > 30

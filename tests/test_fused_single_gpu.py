@@ -698,7 +698,7 @@ def test_resident_norm_matches_the_staged_form(dtype, M, N, K, algo, plan):
     # rows that stay on the chip between the product and its RMSNorm, call after call with another shape in between (the
     # exchange has to be left clean), results on a 32-byte boundary and on a 16-byte one; the same call with the named tile
     # kept goes through the staging buffer
-    assert tuple(torch.ops.flashoverlap_op.planned_tile(M, N, K, algo, 0, False, True)) == plan
+    assert tuple(torch.ops.flashoverlap_op.planned_tile(M, N, K, algo, 0, False, True))[:3] == plan
     A, B, W = make_inputs(M, N, K, dtype, seed=N)
     A2, B2, W2 = make_inputs(256, 1024, 264, dtype, seed=1)
     impl = make_impl()

@@ -162,3 +162,51 @@ def test_gemm_result_on_16_and_32_byte_boundaries(offset, algo, M, N, glu):
     # one rounding to 11 bits of fp32 sums
     assert ((C.double() - want).abs() <= 2 ** -10.9 * want.abs() + 1e-5).all()
     assert bool((buf[:offset] == 5).all()) and bool((buf[offset + M * n:] == 5).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K,algo", [
+    # K split over clusters of several sizes, some CTA without a column of its own, a last tile that is partly empty, K tails
+    (128, 64, 4096, 2), (128, 1024, 28672, 2), (128, 1152, 20416, 1), (256, 1024, 15640, 1), (256, 1088, 8192, 2),
+    (128, 2112, 6152, 2), (128, 10240, 8192, 6), (640, 640, 12296, 1),
+    # tiles of 96, 160, 192 and 224 columns in pairs and single CTAs, one wave and several, last columns of all sorts
+    (1152, 5120, 1720, 6), (3584, 2048, 4096, 8), (2048, 8192, 1024, 8), (1152, 1408, 2048, 6), (1024, 2560, 1128, 8),
+    (896, 4672, 1040, 2)])
+def test_gemm_in_tiles_of_any_width_and_split(dtype, M, N, K, algo):
+    plan = torch.ops.flashoverlap_op.planned_tile(M, N, K, algo, 0, False, False)
+    assert plan[3] > 1 or plan[1] < ALGO_TILES[plan[0]][1]      # a shape that is here for its plan
+    torch.manual_seed(K)
+    A = torch.randn(M, K, device="cuda", dtype=dtype)
+    B = (torch.randn(N, K, device="cuda") / K ** 0.5).to(dtype)
+    impl = _impl()
+    want = A.double() @ B.double().t()
+    bits = 10.9 if dtype == torch.float16 else 7.9
+    tiles = (M // ALGO_TILES[algo][0], N // ALGO_TILES[algo][1])
+    count = tiles[0] * tiles[1]
+    RA = torch.arange(count, dtype=torch.int32, device="cuda").flip(0).reshape(tiles)
+    cseg = torch.tensor([count], dtype=torch.int32)
+    MM = torch.zeros(tiles[0] + 1, tiles[1], dtype=torch.int32, device="cuda")
+    over = torch.classes.flashoverlap_class.OverlapImpl()
+    over.nccl_init(0, 1, [0] * 16)
+    over.cutlass_init()
+    over.overlap_init()
+    over.set_timeout_ms(2000)
+    first = None
+    for offset in (0, 8, 0):
+        buf = torch.full((M * N + 32,), 5.0, device="cuda", dtype=dtype)
+        C = buf[offset:offset + M * N].view(M, N)
+        impl.cutlass_gemm(A, B, C, algo)
+        assert impl.last_algo() == plan[0]
+        torch.cuda.synchronize()
+        impl.check_status()
+        # one rounding of fp32 sums
+        assert ((C.double() - want).abs() <= 2 ** -bits * want.abs() + 4e-6 * K ** 0.5).all()
+        assert bool((buf[:offset] == 5).all()) and bool((buf[offset + M * N:] == 5).all())
+        assert first is None or torch.equal(C, first)          # the same bits every time
+        first = C.clone()
+    T = torch.full((M, N), float("nan"), device="cuda", dtype=dtype)
+    over.gemm_allreduce_overlap(A, B, T, MM, RA, 1, cseg, cseg.cuda(), algo, False)
+    torch.cuda.synchronize()
+    over.check_status()
+    from flashoverlap_b200.utils.reorder import from_tile_order
+    assert torch.equal(from_tile_order(T, *ALGO_TILES[algo][:2], RA), first)
