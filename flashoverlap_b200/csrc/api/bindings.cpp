@@ -86,6 +86,20 @@ static void rmsnorm_op(at::Tensor X, at::Tensor O, at::Tensor RW, double eps) {
   check_norm_launch(e, "rmsnorm");
 }
 
+// The same with a result of their own: one call from Python in place of two.  37 x 8000, whose kernel runs 2 us: 6.4 -> 6.0 us
+// a call.
+static at::Tensor rmsnorm_new_op(at::Tensor X, at::Tensor RW, double eps) {
+  at::Tensor O = at::empty_like(X);
+  rmsnorm_op(X, O, RW, eps);
+  return O;
+}
+static at::Tensor reorder_rmsnorm_new_op(at::Tensor X, at::Tensor RW, int64_t BM, int64_t BN, int64_t rldn, at::Tensor RA,
+                                         double eps) {
+  at::Tensor RX = at::empty_like(X);
+  reorder_rmsnorm_eps(X, RX, RW, BM, BN, rldn, RA, eps);
+  return RX;
+}
+
 // add_rmsnorm(X, R, S, O, RW, eps): S = X + R (rounded to the 16-bit type), O = rmsnorm(S); one pass over the rows.
 static void add_rmsnorm_op(at::Tensor X, at::Tensor R, at::Tensor S, at::Tensor O, at::Tensor RW, double eps) {
   check_matrix(X, "X");
@@ -212,6 +226,7 @@ TORCH_LIBRARY(flashoverlap_class, m) {
       .def("gemm_rmsnorm", &OverlapImpl::GemmRmsNorm)
       .def("allgather_gemm", &OverlapImpl::AllGatherGemm)
       .def("a2a_dispatch_gemm", &OverlapImpl::A2aDispatchGemm)
+      .def("a2a_dispatch_gemm_new", &OverlapImpl::A2aDispatchGemmNew)
       .def("a2a_padded_rows", &OverlapImpl::A2aPaddedRows)
       .def("attach_symmetric", &OverlapImpl::AttachSymmetric)
       .def("detach_symmetric", &OverlapImpl::DetachSymmetric)
@@ -248,6 +263,8 @@ TORCH_LIBRARY(flashoverlap_op, m) {
   m.def("reorder_rmsnorm", &fo::reorder_rmsnorm_op);
   m.def("reorder_rmsnorm_eps", &fo::reorder_rmsnorm_eps);
   m.def("rmsnorm", &fo::rmsnorm_op);
+  m.def("rmsnorm_new", &fo::rmsnorm_new_op);
+  m.def("reorder_rmsnorm_new", &fo::reorder_rmsnorm_new_op);
   m.def("add_rmsnorm", &fo::add_rmsnorm_op);
   m.def("tile_walk", &fo::tile_walk_op);
   m.def("planned_algo", &fo::planned_algo_op);

@@ -7,6 +7,7 @@
 #include <nvtx3/nvToolsExt.h>
 #include <unistd.h>
 
+#include <algorithm>
 #include <functional>
 
 #include "../kernels/comm_kernels.h"
@@ -608,6 +609,20 @@ void OverlapImpl::A2aDispatchGemm(at::Tensor A_send, at::Tensor B, at::Tensor C,
   c10::cuda::CUDAGuard guard(A_send.device());
   engine_.a2a_gemm(A_send.data_ptr(), B.data_ptr(), C.data_ptr(), len, static_cast<int>(N), static_cast<int>(K),
                    dtype_of(A_send), static_cast<int>(algo), current_stream());
+}
+
+at::Tensor OverlapImpl::A2aDispatchGemmNew(at::Tensor A_send, at::Tensor B, at::Tensor mLen_CPU, int64_t rank,
+                                           int64_t algo) {
+  check_matrix(A_send, "A_send");
+  check_matrix(B, "B");
+  at::Tensor C = at::empty({A2aPaddedRows(mLen_CPU, algo), B.size(0)}, A_send.options());
+  A2aDispatchGemm(A_send, B, C, mLen_CPU, algo);
+  const int ws = comm_.world();
+  TORCH_CHECK(rank >= -ws && rank < ws, "rank out of range");
+  const int* len = mLen_CPU.data_ptr<int>();
+  int64_t rows = 0;
+  for (int i = 0; i < ws; ++i) rows += len[i * ws + (rank < 0 ? rank + ws : rank)];
+  return C.narrow(0, 0, std::min<int64_t>(rows, C.size(0)));
 }
 
 void OverlapImpl::GemmRmsNorm(at::Tensor A, at::Tensor B, at::Tensor C, at::Tensor O, at::Tensor weight, double eps,

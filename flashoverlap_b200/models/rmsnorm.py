@@ -39,9 +39,7 @@ class KernelRMSNorm(RMSNorm):
             return super().forward(x)
         shape = x.shape
         x2 = x.reshape(-1, shape[-1]).contiguous()
-        out = torch.empty_like(x2)
-        torch.ops.flashoverlap_op.rmsnorm(x2, out, self.weight, float(self.eps))
-        return out.reshape(shape)
+        return torch.ops.flashoverlap_op.rmsnorm_new.default(x2, self.weight, float(self.eps)).reshape(shape)
 
 
 class ReorderRMSNorm(nn.Module):
@@ -62,7 +60,5 @@ class ReorderRMSNorm(nn.Module):
                              persistent=False)
 
     def forward(self, x):
-        out = torch.empty_like(x)
-        torch.ops.flashoverlap_op.reorder_rmsnorm_eps(x, out, self.weight, self.bm, self.bn, 1, self.reorder_array,
-                                                      float(self.eps))
-        return out
+        return torch.ops.flashoverlap_op.reorder_rmsnorm_new.default(x, self.weight, self.bm, self.bn, 1,
+                                                                     self.reorder_array, float(self.eps))

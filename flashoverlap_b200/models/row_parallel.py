@@ -85,12 +85,12 @@ class OverlapRowParallelLayer(nn.Module):
     def forward(self, x):
         n = self.weight.size(0)
         if self.comm_op == "all_reduce":
-            out = torch.empty((x.size(0), n), dtype=x.dtype, device=x.device)
+            out = x.new_empty((x.size(0), n))
             self.overlap_class.gemm_allreduce_overlap(x, self.weight, out, self.counter, self.reorder_array, 1,
                                                       self.cseg_cpu, self.cseg_gpu, self.algo, False)
             return out
-        tmp = torch.empty((x.size(0), n), dtype=x.dtype, device=x.device)
-        out = torch.empty((x.size(0) // self.world_size, n), dtype=x.dtype, device=x.device)
+        tmp = x.new_empty((x.size(0), n))
+        out = x.new_empty((x.size(0) // self.world_size, n))
         self.overlap_class.gemm_reducescatter_overlap(x, self.weight, tmp, out, self.counter, self.reorder_array,
                                                       self.row_array, 1, self.cseg_cpu, self.cseg_gpu, self.algo,
                                                       False)
@@ -146,7 +146,7 @@ class FusedRowParallelLinear(nn.Module):
         try:
             if self.comm_op == "all_reduce":
                 return self.impl.gemm_allreduce_fused(x, self.weight, self.norm_weight, self.eps, self.algo)
-            out = torch.empty((x.size(0) // self.world_size, self.weight.size(0)), dtype=x.dtype, device=x.device)
+            out = x.new_empty((x.size(0) // self.world_size, self.weight.size(0)))
             self.impl.gemm_reducescatter_fused(x, self.weight, out, self.norm_weight, self.eps, self.algo,
                                                self.interleave)
             return out

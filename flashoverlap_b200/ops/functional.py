@@ -16,7 +16,7 @@ def gemm(impl, a: torch.Tensor, b: torch.Tensor, algo: int = 0, out: Optional[to
     """``a[M,K] @ b[N,K]^T`` on the tcgen05 kernel (reference: cutlass_gemm)."""
     _check(a)
     if out is None:
-        out = torch.empty((a.size(0), b.size(0)), dtype=a.dtype, device=a.device)
+        out = a.new_empty((a.size(0), b.size(0)))
     impl.cutlass_gemm(a, b, out, algo)
     return out
 
@@ -52,7 +52,7 @@ def allgather_gemm(impl, a_shard, b, world_size: int, algo: int = 0, out: Option
     gather pushed over NVLink by the same kernel that computes the product."""
     _check(a_shard)
     if out is None:
-        out = torch.empty((a_shard.size(0) * world_size, b.size(0)), dtype=a_shard.dtype, device=a_shard.device)
+        out = a_shard.new_empty((a_shard.size(0) * world_size, b.size(0)))
     impl.allgather_gemm(a_shard, b, out, algo)
     return out
 
@@ -62,21 +62,14 @@ def a2a_dispatch_gemm(impl, a_send, b, mlen_cpu: torch.Tensor, rank: int, algo: 
     to rank j (``a_send`` holds this rank's rows in destination order); returns
     the product of the rows received here, in source order, with ``b^T``."""
     _check(a_send)
-    m_pad = impl.a2a_padded_rows(mlen_cpu, algo)
-    out = torch.empty((m_pad, b.size(0)), dtype=a_send.dtype, device=a_send.device)
-    impl.a2a_dispatch_gemm(a_send, b, out, mlen_cpu, algo)
-    return out[: int(mlen_cpu[:, rank].sum())]
+    return impl.a2a_dispatch_gemm_new(a_send, b, mlen_cpu, rank, algo)
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
     _check(x)
-    out = torch.empty_like(x)
-    torch.ops.flashoverlap_op.rmsnorm(x, out, weight, eps)
-    return out
+    return torch.ops.flashoverlap_op.rmsnorm_new.default(x, weight, eps)
 
 
 def reorder_rmsnorm(x, weight, bm: int, bn: int, ra: torch.Tensor, rldn: int = 1, eps: float = 1e-5):
     _check(x)
-    out = torch.empty_like(x)
-    torch.ops.flashoverlap_op.reorder_rmsnorm_eps(x, out, weight, bm, bn, rldn, ra, eps)
-    return out
+    return torch.ops.flashoverlap_op.reorder_rmsnorm_new.default(x, weight, bm, bn, rldn, ra, eps)

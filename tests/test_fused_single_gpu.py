@@ -762,3 +762,36 @@ def test_resident_norm_in_a_graph():
         # the product, its scaling and the weight are each rounded to 11 bits
         assert ((D.double() - want).abs() <= 2 ** -9.3 * want.abs() + 1e-4).all()
         assert ((E.double() - y).abs() <= 2 ** -10.9 * y.abs() + 1e-5).all()
+
+
+def test_wrappers_that_make_their_result_natively():
+    # the same bits as the forms that write into a given tensor, rows of any count, and the same refusals
+    M, N, K, algo = 300, 512, 136, 8
+    A, B, W = make_inputs(M, N, K, torch.float16)
+    impl = make_impl()
+    from flashoverlap_b200 import ops
+
+    x = torch.randn(37, 520, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(520, device="cuda", dtype=torch.bfloat16)
+    out = torch.empty_like(x)
+    torch.ops.flashoverlap_op.rmsnorm(x, out, w, 1e-5)
+    assert torch.equal(ops.rmsnorm(x, w), out)
+    RA = torch.arange(8, dtype=torch.int32, device="cuda").flip(0).reshape(2, 4)
+    y = torch.randn(256, 512, device="cuda", dtype=torch.float16)
+    out = torch.empty_like(y)
+    torch.ops.flashoverlap_op.reorder_rmsnorm_eps(y, out, W, 128, 128, 2, RA, 1e-5)
+    assert torch.equal(ops.reorder_rmsnorm(y, W, 128, 128, RA, 2), out)
+    mlen = torch.tensor([[M]], dtype=torch.int32)
+    C = torch.empty(512, N, device="cuda", dtype=torch.float16)
+    impl.a2a_dispatch_gemm(A, B, C, mlen, algo)
+    got = ops.a2a_dispatch_gemm(impl, A, B, mlen, 0, algo)
+    assert got.shape == (M, N) and torch.equal(got, C[:M])
+    assert torch.equal(ops.a2a_dispatch_gemm(impl, A, B, mlen, -1, algo), C[:M])
+    assert ops.a2a_dispatch_gemm(impl, A, B, torch.tensor([[0]], dtype=torch.int32), 0, algo).shape == (0, N)
+    for bad in (lambda: ops.rmsnorm(x[:, ::2], w[:260]), lambda: ops.rmsnorm(x, w[:512]), lambda: ops.rmsnorm(x.float(), w),
+                lambda: ops.reorder_rmsnorm(y, W, 96, 128, RA, 2), lambda: ops.a2a_dispatch_gemm(impl, A, B, mlen + 1, 0, algo),
+                lambda: ops.a2a_dispatch_gemm(impl, A, B, mlen, 1, algo)):
+        with pytest.raises(RuntimeError):
+            bad()
+    torch.cuda.synchronize()
+    impl.check_status()
