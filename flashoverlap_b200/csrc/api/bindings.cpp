@@ -171,7 +171,7 @@ static int64_t planned_algo_op(int64_t M, int64_t N, int64_t K, int64_t algo, in
 static std::vector<int64_t> planned_tile_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu,
                                             bool norm) {
   const LaunchPlan p = plan_op(M, N, K, algo, ctas, glu, norm);
-  return {p.algo, p.bn, p.rows, p.split};
+  return {p.algo, p.bn, p.rows, p.split, p.norm_after};
 }
 
 }  // namespace fo

@@ -172,6 +172,8 @@ struct alignas(64) FusedParams {
   // chip and there is no reduce phase (resident_norm).  exchange: one word per row and tile column, [M / 128][TN][128],
   // all zero between launches; readers: tiles that have read a row block's entries, zero between launches.
   int resident;
+  // Set by the launch: the product goes to the staging buffer as a plain GEMM's, the caller launches the RMSNorm behind it.
+  int norm_after;
   uint32_t* exchange;
   uint32_t* readers;
   int drop_stage;  // norm_stream: the staged product is scratch, its lines need not reach memory once they are read

@@ -48,9 +48,9 @@ struct GemmOperands {
 };
 
 // What a launch runs: the tile configuration (index of the table), the width of its tiles, for a resident RMSNorm the tile
-// rows of a wave (0: not resident), and over how many CTAs the K of a tile is split.
+// rows of a wave (0: not resident), over how many CTAs the K of a tile is split, and whether the RMSNorm is a kernel of its own.
 struct LaunchPlan {
-  int algo, bn, rows, split;
+  int algo, bn, rows, split, norm_after;
 };
 // The plan with which a GEMM on `ctas` CTAs is expected to take least time.
 LaunchPlan plan_launch(const GemmOperands& g, int ctas);

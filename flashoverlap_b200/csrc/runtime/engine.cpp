@@ -1,5 +1,7 @@
 #include "engine.h"
 
+#include "../kernels/rmsnorm.h"
+
 #include <nvtx3/nvToolsExt.h>
 
 #include <cstdlib>
@@ -31,6 +33,9 @@ void FusedEngine::launch(const GemmOperands& g, FusedParams& p, cudaStream_t str
     throw std::runtime_error(cuda_error_string(e, msg.c_str()));
   }
   last_algo_ = p.algo;
+  if (p.norm_after) {
+    check(launch_rmsnorm(p.epi_base[0], p.out[p.me], p.gamma, g.M, g.N, p.eps, g.dtype, stream), op);
+  }
 }
 
 FusedEngine::~FusedEngine() {

@@ -795,3 +795,34 @@ def test_wrappers_that_make_their_result_natively():
             bad()
     torch.cuda.synchronize()
     impl.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K,algo", [(256, 1664, 11904, 1), (128, 1024, 28672, 2), (384, 1280, 22256, 2), (2176, 4096, 4096, 0)])
+def test_norm_behind_a_plain_gemm(dtype, M, N, K, algo):
+    # few tiles and a long K: a GEMM whose K is split, then the RMSNorm kernel; also where a plain GEMM has the better tiles;
+    # a call without RMSNorm and a resident one in between
+    plan = torch.ops.flashoverlap_op.planned_tile(M, N, K, algo, 0, False, True)
+    assert plan[4] == 1 and plan[2] == 0
+    A, B, W = make_inputs(M, N, K, dtype, seed=N)
+    impl = make_impl()
+    y = A.double() @ B.double().t()
+    want = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * W.double()
+    # the product, its scaling and the weight are each rounded to 11 or 8 bits
+    rel = 2 ** -9.3 if dtype == torch.float16 else 2 ** -6.3
+    first = None
+    for offset in (0, 8):
+        buf = torch.full((M * N + 32,), 9.0, device="cuda", dtype=dtype)
+        D = buf[offset:offset + M * N].view(M, N)
+        impl.gemm_reducescatter_fused(A, B, D, W, 1e-5, algo, False)
+        assert impl.last_algo() == plan[0]
+        out = impl.gemm_allreduce_fused(A, B, W, 1e-5, algo)
+        plain = impl.gemm_allreduce_fused(A[:, :264].contiguous(), B[:, :264].contiguous(), None, 1e-5, algo)
+        torch.cuda.synchronize()
+        impl.check_status()
+        assert torch.isfinite(plain.float()).all()
+        for got in (D, out):
+            assert ((got.double() - want).abs() <= rel * want.abs() + 1e-4).all()
+        assert bool((buf[:offset] == 9).all()) and bool((buf[offset + M * N:] == 9).all())
+        assert first is None or torch.equal(D, first)
+        first = D.clone()
