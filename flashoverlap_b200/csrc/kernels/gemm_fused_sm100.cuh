@@ -117,8 +117,10 @@ __device__ __forceinline__ void report_error(const FusedParams& p, uint32_t code
 template <bool BF16>
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   if constexpr (BF16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
+    // (as one 32-bit register from the start: through a pair of 16-bit values every bf16 instance spilled)
+    uint32_t v;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(b), "f"(a));
+    return v;
   } else {
     __half2 v = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -128,7 +130,7 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 template <bool BF16>
 __device__ __forceinline__ float2 unpack2(uint32_t u) {
   if constexpr (BF16) {
-    return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
+    return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));  // the upper half of an fp32
   } else {
     return __half22float2(*reinterpret_cast<__half2*>(&u));
   }
@@ -139,8 +141,8 @@ __device__ __forceinline__ float2 unpack2(uint32_t u) {
 template <bool BF16>
 __device__ __forceinline__ uint32_t norm_pack2(float a, float b, float rstd, uint32_t w2) {
   if constexpr (BF16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a * rstd, b * rstd);
-    __nv_bfloat162 r = __hmul2(v, *reinterpret_cast<__nv_bfloat162*>(&w2));
+    uint32_t v = pack2<true>(a * rstd, b * rstd);
+    __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&v), *reinterpret_cast<__nv_bfloat162*>(&w2));
     return *reinterpret_cast<uint32_t*>(&r);
   } else {
     __half2 v = __floats2half2_rn(a * rstd, b * rstd);
@@ -786,19 +788,17 @@ __device__ __forceinline__ void resident_norm(const FusedParams& p, uint32_t tme
     // ---- this warp's part of the tile, rounded; the accumulator goes back to the MMA warp ----
     uint32_t v[CHUNKS][16];
     float ssq = 0.f;
-    // sixteen columns are on their way while the sixteen before them are rounded (there are no registers for 32)
-    uint32_t r[2][16];
-    if (mine > 0) ptx::tmem_ld_32x32b_x16(t_row, r[0]);
+    {
+      // 32 columns are on their way while the 32 before them are rounded.  The loads are unconditional (columns past the
+      // share are read and dropped): in branches the two sets of registers did not fit.
+      uint32_t r[2][32];
+      ptx::tmem_ld_32x32b_x32(t_row, r[0]);
 #pragma unroll
-    for (int i = 0; i < 2 * CHUNKS; ++i) {
-      if (i < 2 * mine) {
-        ptx::tmem_ld_wait_for(r[i & 1]);
-        if (i + 1 < 2 * mine) ptx::tmem_ld_32x32b_x16(t_row + (i + 1) * 16, r[(i + 1) & 1]);
-        uint32_t* const o = v[i / 2] + 8 * (i & 1);
-        const uint32_t* const a = r[i & 1];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = pack2<BF16>(__uint_as_float(a[2 * e]), __uint_as_float(a[2 * e + 1]));
-        ssq += sum_squares<BF16>(make_uint4(o[0], o[1], o[2], o[3])) + sum_squares<BF16>(make_uint4(o[4], o[5], o[6], o[7]));
+      for (int c = 0; c < CHUNKS; ++c) {
+        ptx::tmem_ld_wait_for(r[c & 1]);
+        if (c + 1 < CHUNKS) ptx::tmem_ld_32x32b_x32(t_row + (c + 1) * 32, r[(c + 1) & 1]);
+        pack_row32<BF16>(v[c], r[c & 1]);
+        if (c < mine) ssq += sum_squares32<BF16>(v[c]);
       }
     }
     ptx::tc_fence_before_sync();

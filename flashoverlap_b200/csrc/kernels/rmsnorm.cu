@@ -4,7 +4,7 @@
 // (8 values each) of every row, so that the weights can stay in registers, and the next row is on its way from memory
 // while the current one is reduced, scaled and stored (one barrier per row).  Wide rows of matrices beyond the L2 take one
 // CTA each (rmsnorm_row_kernel), rows of more than 32768 values (of a sum: 16384) are read twice.  Bound by HBM: 16384 x
-// 4096 bf16 takes 45.1 us (5.95 TB/s) where one CTA per row, with nothing in flight while it reduced, took 63.0; 37 x
+// 4096 bf16 takes 43.5 us (6.17 TB/s) where one CTA per row, with nothing in flight while it reduced, took 63.0; 37 x
 // 8000 fp16 takes 2.2 us where it took 3.1; a single launch of 4096 x 8192 bf16 on a cold L2 28.7 where it took 30.7.
 // Tile order reads at 2048 x 8192 behind its GEMM: 54.3 us for the pair against 57.2 with the tile found anew for every
 // load.  With a sum (two rows in, two out) 2048 x 4096 bf16 takes 9.8 us.  Unlike the reference kernels (reference: src/rmsnorm/rmsnorm.cuh:12-115, block size dim/16, eps fixed to
@@ -32,6 +32,19 @@ __device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {
 template <bool BF16>
 __device__ __forceinline__ uint4 add_chunk(const uint4& a, const uint4& b) {
   return make_uint4(add2<BF16>(a.x, b.x), add2<BF16>(a.y, b.y), add2<BF16>(a.z, b.z), add2<BF16>(a.w, b.w));
+}
+
+// Eight values as floats that stay in registers (the compiler would rather unpack them again).
+template <bool BF16>
+__device__ __forceinline__ void unpack_chunk(float (&f)[8], const uint4& v) {
+  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 p = unpack2<BF16>(u[i]);
+    f[2 * i] = p.x;
+    f[2 * i + 1] = p.y;
+    asm volatile("" : "+f"(f[2 * i]), "+f"(f[2 * i + 1]));
+  }
 }
 
 // `r` and `sum`: NORM_SUM only.
@@ -110,9 +123,23 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t
         if (c < n_chunks) dst[c] = v[k];
       }
     }
+    // Up to two chunks (one of a sum, whose two would not fit) stay unpacked between the statistics and the scaling: less
+    // follows the barrier, and with these registers no CTA of the next grid finds a place before one of this grid has ended
+    // (with five of them on some SMs the grid ended later).  Launch after launch, fp16: 16384 x 4096 49.0 -> 43.5 us, 2048 x
+    // 4096 7.5 -> 5.2, 1000 x 1024 2.5 -> 2.1; in tile order 4096 x 9216 39.9 -> 36.7, 2048 x 8192 12.9 -> 12.3.
+    constexpr bool UNPACKED = INPUT == NORM_SUM ? CPT == 1 : CPT <= 2;
+    float f[UNPACKED ? CPT : 1][8];
 #pragma unroll
     for (int k = 0; k < CPT; ++k) {
-      ssq += static_cast<int>(threadIdx.x + k * blockDim.x) < n_chunks ? sum_squares<BF16>(v[k]) : 0.f;
+      if constexpr (UNPACKED) {
+        unpack_chunk<BF16>(f[k], v[k]);
+        float q = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) q += f[k][e] * f[k][e];
+        ssq += static_cast<int>(threadIdx.x + k * blockDim.x) < n_chunks ? q : 0.f;
+      } else {
+        ssq += static_cast<int>(threadIdx.x + k * blockDim.x) < n_chunks ? sum_squares<BF16>(v[k]) : 0.f;
+      }
     }
     const unsigned next = row + gridDim.x;
     uint4 nv[CPT];
@@ -131,7 +158,15 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t
 #pragma unroll
     for (int k = 0; k < CPT; ++k) {
       const int c = threadIdx.x + k * blockDim.x;
-      if (c < n_chunks) dst[c] = scale_chunk<BF16>(v[k], rstd, KEEP ? g[KEEP ? k : 0] : __ldg(weights + c));
+      const uint4 w4 = KEEP ? g[KEEP ? k : 0] : __ldg(weights + min(c, n_chunks - 1));
+      if constexpr (UNPACKED) {
+        if (c < n_chunks) {
+          dst[c] = make_uint4(norm_pack2<BF16>(f[k][0], f[k][1], rstd, w4.x), norm_pack2<BF16>(f[k][2], f[k][3], rstd, w4.y),
+                              norm_pack2<BF16>(f[k][4], f[k][5], rstd, w4.z), norm_pack2<BF16>(f[k][6], f[k][7], rstd, w4.w));
+        }
+      } else {
+        if (c < n_chunks) dst[c] = scale_chunk<BF16>(v[k], rstd, w4);
+      }
     }
 #pragma unroll
     for (int k = 0; k < CPT; ++k) v[k] = nv[k];
