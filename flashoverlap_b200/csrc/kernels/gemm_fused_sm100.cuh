@@ -75,6 +75,7 @@ struct TileTraits {
 
 constexpr int kThreads = kFusedThreads;  // 8 GEMM warps + 4 communication warps
 constexpr int kGemmThreads = 32 * kGemmWarps;
+constexpr uint64_t kPartnerGraceNs = 1000000000ull;  // how much longer than for anything else a CTA waits for its partner's end
 
 // ---------------------------------------------------------------------------
 // helpers
@@ -1226,11 +1227,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
           }
         }
       }
-      if (!ok) {
-        // Give copies that are still in flight time to land before the CTA
-        // releases its shared memory.
-        for (int i = 0; i < 64; ++i) __nanosleep(20000);
-      }
     }
   } else if (warp == 1) {
     // ===================== MMA issuer =====================
@@ -1599,23 +1595,29 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     const int gemm_threads = p.epi_halves == 2 ? kThreads : kGemmThreads;
     __syncwarp();
     ptx::tc_fence_before_sync();
+    // One answer for all GEMM warps: the communication warps may raise the flag at this very moment, and the warps of a
+    // row group must either all join the reduce phase, whose barriers have no deadline, or none.  (A warp that gave up
+    // above sees its own store, so a failure of the GEMM phase is always in the answer.)
+    bool gave_up = ptx::named_barrier_or(8, gemm_threads, *abort_flag != 0);
+    if (gave_up) {
+      // Whichever warp gave up, copies and MMAs of this CTA may be in flight: they land (in microseconds) before its shared
+      // memory and its TMEM go back.
+      for (int i = 0; i < 64; ++i) __nanosleep(20000);
+    }
     if constexpr (CTAS == 2) {
-      ptx::named_barrier_sync(8, gemm_threads);
       // The partner may still read this CTA's operands or signal its barriers:
       // each CTA tells the other that its GEMM warps are done and waits (bounded)
-      // to hear the same.
+      // to hear the same.  The partner's own waits end by its deadline, after which it may look at the clock a little later
+      // than this CTA and let its copies land: a CTA that left at its own deadline would not be there to be told.
       if (threadIdx.x == 0) {
         ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(pair_bar), cta_rank ^ 1u));
-        if (!ptx::mbar_wait_cluster(pair_bar, 0u, deadline)) {
+        if (!ptx::mbar_wait_cluster(pair_bar, 0u, deadline + kPartnerGraceNs)) {
           report_error(p, ST_TIMEOUT_PIPE, 0x700u, 0, 0);
           *abort_flag = 1;
         }
       }
+      gave_up = ptx::named_barrier_or(8, gemm_threads, *abort_flag != 0);
     }
-    // One answer for all GEMM warps: the communication warps may raise the flag at this very moment, and the warps of a
-    // row group must either all join the reduce phase, whose barriers have no deadline, or none.  (A warp that gave up
-    // above sees its own store, so a failure of the GEMM phase is always in the answer.)
-    const bool gave_up = ptx::named_barrier_or(8, gemm_threads, *abort_flag != 0);
     if (warp == 2) {
       ptx::tc_fence_after_sync();
       if constexpr (CTAS == 2) ptx::tmem_dealloc_pair(tmem_base, T::TMEM_COLS);

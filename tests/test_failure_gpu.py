@@ -39,6 +39,35 @@ def test_wait_that_nothing_satisfies_times_out_with_status():
     assert (C.float() - A.float() @ B.float().t()).abs().max().item() < 0.1
 
 
+# M, N, Algo: one CTA, pairs of CTAs, a pair with a second tile to come
+SLOW = {"one": (128, 64, 2), "pair": (256, 64, 5), "wide pair": (256, 128, 4), "second tile": (512, 64, 5)}
+
+
+@pytest.mark.parametrize("M,N,algo", list(SLOW.values()), ids=list(SLOW))
+def test_gemm_that_runs_out_of_time_returns_a_status(M, N, algo):
+    # a main loop of 9 ms or more under a deadline of 1 ms (which a wait notices some milliseconds late): the epilogue gives
+    # up while operands and products of its CTA are in flight; the kernel ends with a status, the context stays usable
+    K = 2_000_000
+    impl = torch.classes.flashoverlap_class.OverlapImpl()
+    impl.cutlass_init()
+    impl.set_keep_tile(True)
+    impl.set_sm_count(2)
+    A = torch.full((M, K), 2.0 ** -10, device="cuda", dtype=torch.float16)
+    B = torch.full((N, K), 2.0 ** -11, device="cuda", dtype=torch.float16)
+    C = torch.empty(M, N, device="cuda", dtype=torch.float16)
+    impl.set_timeout_ms(1)
+    impl.cutlass_gemm(A, B, C, algo)
+    torch.cuda.synchronize()
+    assert impl.status()[0] == 1, impl.status_string()  # ST_TIMEOUT_PIPE
+    impl.reset()
+    impl.set_timeout_ms(2000)
+    impl.cutlass_gemm(A, B, C, algo)
+    torch.cuda.synchronize()
+    impl.check_status()
+    # K products of 2^-21: sums of fewer than 2^24 equal steps are exact in fp32
+    assert bool((C == torch.tensor(K * 2.0 ** -21).half().cuda()).all())
+
+
 @pytest.mark.timeout(300)
 def test_late_rank_trips_short_deadline_and_reset_recovers():
     if torch.cuda.device_count() < 2:
