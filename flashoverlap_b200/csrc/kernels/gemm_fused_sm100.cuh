@@ -932,7 +932,8 @@ __device__ __forceinline__ void resident_clear(const FusedParams& p, uint32_t ct
 // Epilogue of a tile whose K is split over the CTAs of a cluster (one tile per cluster): every CTA owns a stretch of the
 // tile's columns, gets the other parts' sums for it through distributed shared memory (in place of the operands, which
 // everybody has read by then), adds them up in the order of the parts and stores.  Two warps to a quarter of the rows share
-// the chunks of 32 columns.
+// the chunks of 32 columns.  The warp arrives at the cluster's last barrier as soon as it has nothing left to do in the other
+// parts' memory, also when it gives up: no part leaves while another may still write there (see the teardown).
 template <bool BF16>
 __device__ __forceinline__ void split_epilogue(const FusedParams& p, uint32_t tmem_base, uint64_t* tfull_bar,
                                                uint64_t* split_bar, uint32_t inbox, int part, int q, int half, int lane,
@@ -946,12 +947,16 @@ __device__ __forceinline__ void split_epilogue(const FusedParams& p, uint32_t tm
   const int chunks = min(p.bn, p.N - col0) / 32;
   const int most = (chunks + p.split - 1) / p.split;  // chunks of an owner, at most
   auto first_of = [&](int owner) { return chunks * owner / p.split; };
-  auto give_up = [&](uint32_t where) {
+  auto report = [&](uint32_t where) {
     if (lane == 0) {
       report_error(p, ST_TIMEOUT_PIPE, where, part, blockIdx.x);
       *abort_flag = 1;
     }
     __syncwarp();
+  };
+  auto give_up = [&](uint32_t where) {
+    report(where);
+    ptx::cluster_arrive();
   };
   if (!__all_sync(0xffffffffu, ptx::mbar_wait(tfull_bar, 0u, deadline))) return give_up(0x400u);
   ptx::tc_fence_after_sync();
@@ -979,7 +984,8 @@ __device__ __forceinline__ void split_epilogue(const FusedParams& p, uint32_t tm
     __syncwarp();  // every lane's stores before the release
     if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&split_bar[1]), owner));
   }
-  if (!__all_sync(0xffffffffu, ptx::mbar_wait_cluster(&split_bar[1], 0u, deadline))) return give_up(0x900u);
+  ptx::cluster_arrive();
+  if (!__all_sync(0xffffffffu, ptx::mbar_wait_cluster(&split_bar[1], 0u, deadline))) return report(0x900u);
   const OutLayout& L = p.epi_layout;
   const long long pitch = L.tiled ? static_cast<long long>(L.rldn) * L.bn : L.ld;
   uint16_t* const base = reinterpret_cast<uint16_t*>(p.epi_base[0]) + lane * pitch;
@@ -1595,6 +1601,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     const int gemm_threads = p.epi_halves == 2 ? kThreads : kGemmThreads;
     __syncwarp();
     ptx::tc_fence_before_sync();
+    if constexpr (CTAS == 1) {
+      if (split > 1) {
+        // The parts of a tile leave together: a late one may still send sums to one that has given up, whose memory has to be
+        // there.  Every wait on the way to an arrival has a deadline, so all of them come.
+        if (warp < 4) ptx::cluster_arrive();
+        ptx::cluster_wait();
+      }
+    }
     // One answer for all GEMM warps: the communication warps may raise the flag at this very moment, and the warps of a
     // row group must either all join the reduce phase, whose barriers have no deadline, or none.  (A warp that gave up
     // above sees its own store, so a failure of the GEMM phase is always in the answer.)

@@ -380,6 +380,10 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
   // 3584 x 9472 x 256 fp16: 35.4 us with four epilogue warps and the transpose, 26.7 with eight and without; 4096 x 8192 x
   // 1024 74.5 -> 60.9; one wave of 512 x 9472 x 256 10.3 -> 8.6.
   p.epi_halves = p.epi_direct && !p.reduce && !p.ag_push ? 2 : 1;
+  if (p.split > 1 && p.epi_halves != 2) {
+    *why = "a split K needs the epilogue of eight warps";
+    return cudaErrorInvalidValue;
+  }
   if (p.raster_group <= 0) p.raster_group = 1;
   if (p.raster_group > p.TM) p.raster_group = p.TM;
   if (p.rot < 0 || p.rot >= p.TM) p.rot = 0;

@@ -293,6 +293,10 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same barrier in two steps: every thread of the cluster arrives once, then waits once.  The wait has no deadline: only
+// where every path to the arrivals is bounded.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // Address of this CTA's shared-memory object `smem_addr` as seen in CTA `rank`
 // of the cluster (shared::cluster window).
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t smem_addr, uint32_t rank) {

@@ -68,6 +68,29 @@ def test_gemm_that_runs_out_of_time_returns_a_status(M, N, algo):
     assert bool((C == torch.tensor(K * 2.0 ** -21).half().cuda()).all())
 
 
+def test_split_gemm_that_runs_out_of_time_returns_a_status():
+    # two parts of one tile, each with a main loop of 10 ms, under a deadline of 1 ms: both give up and leave together
+    M, N, K, algo = 128, 64, 4_000_000, 2
+    assert torch.ops.flashoverlap_op.planned_tile(M, N, K, algo, 2, False, False)[3] == 2
+    impl = torch.classes.flashoverlap_class.OverlapImpl()
+    impl.cutlass_init()
+    impl.set_sm_count(2)
+    A = torch.full((M, K), 2.0 ** -11, device="cuda", dtype=torch.float16)
+    B = torch.full((N, K), 2.0 ** -11, device="cuda", dtype=torch.float16)
+    C = torch.empty(M, N, device="cuda", dtype=torch.float16)
+    impl.set_timeout_ms(1)
+    impl.cutlass_gemm(A, B, C, algo)
+    torch.cuda.synchronize()
+    assert impl.status()[0] == 1, impl.status_string()  # ST_TIMEOUT_PIPE
+    impl.reset()
+    impl.set_timeout_ms(2000)
+    impl.cutlass_gemm(A, B, C, algo)
+    torch.cuda.synchronize()
+    impl.check_status()
+    # K products of 2^-22: sums of fewer than 2^24 equal steps are exact in fp32
+    assert bool((C == torch.tensor(K * 2.0 ** -22).half().cuda()).all())
+
+
 @pytest.mark.timeout(300)
 def test_late_rank_trips_short_deadline_and_reset_recovers():
     if torch.cuda.device_count() < 2:
