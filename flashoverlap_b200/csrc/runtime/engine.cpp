@@ -4,6 +4,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <sstream>
@@ -39,8 +40,6 @@ void FusedEngine::launch(const GemmOperands& g, FusedParams& p, cudaStream_t str
 }
 
 FusedEngine::~FusedEngine() {
-  if (exchange_ != nullptr) cudaFree(exchange_);
-  exchange_ = nullptr;
   if (status_dev_ != nullptr) cudaFree(status_dev_);
   if (status_host_ != nullptr) cudaFreeHost(status_host_);
   status_dev_ = nullptr;
@@ -85,6 +84,9 @@ uint32_t* FusedEngine::flag_ptr(int rank, int set) const {
 uint32_t* FusedEngine::done_ptr(int rank, int set) const { return flag_ptr(rank, set) + kFlagDone; }
 
 namespace {
+// Words of the row statistics that a resident RMSNorm exchanges: one per row and tile column, of 32 columns at least, behind
+// the counters of kMaxTileRows row blocks.
+size_t exchange_words(long long elems) { return kMaxTileRows + static_cast<size_t>(elems) / 32; }
 size_t workspace_bytes(long long elems) {
   const size_t mat = static_cast<size_t>(elems) * 2;
   return 4 * (mat + 4096) + 3 * (kFlagWords * 4 + 4096) + 8192 + (1 << 20);
@@ -92,19 +94,6 @@ size_t workspace_bytes(long long elems) {
 }  // namespace
 
 void FusedEngine::carve_workspace(long long elems) {
-  if (world_ == 1) {
-    // row statistics of tiles of 32 columns at least, and the counters of kMaxTileRows row blocks
-    const size_t bytes = (static_cast<size_t>(elems) / 32 + kMaxTileRows) * sizeof(uint32_t);
-    if (bytes > exchange_bytes_) {
-      if (exchange_ != nullptr) cudaFree(exchange_);
-      exchange_ = nullptr;
-      exchange_bytes_ = 0;
-      check(cudaMalloc(reinterpret_cast<void**>(&exchange_), bytes), "cudaMalloc(row statistics)");
-      exchange_bytes_ = bytes;
-    }
-    check(cudaMemset(exchange_, 0, exchange_bytes_), "cudaMemset(row statistics)");
-    check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
-  }
   const size_t mat = static_cast<size_t>(elems) * 2;
   heap_.reset_allocator();
   for (int s = 0; s < 2; ++s) ws_.stage[s] = heap_.alloc(mat, 1024);
@@ -113,17 +102,39 @@ void FusedEngine::carve_workspace(long long elems) {
   ws_.misc = heap_.alloc(4096, 1024);
   ws_.local_flags = heap_.alloc(kFlagWords * 4, 1024);
   ws_.capacity_elems = elems;
+  ws_.keep_elems = 0;
+  if (world_ == 1) {
+    // Memory of this engine's own has room for the largest problem's exchange; attached memory, whose size is somebody
+    // else's choice, perhaps for smaller problems only.  It is zero like all of a new workspace.
+    const size_t room = (heap_.size() - heap_.used()) / 4;
+    const size_t words = room < 256 ? 0 : std::min(exchange_words(elems), room - 256);  // (1024 bytes for the alignment)
+    if (words > kMaxTileRows) {
+      ws_.exchange = heap_.alloc(words * 4, 1024);
+      ws_.keep_elems = static_cast<long long>(words - kMaxTileRows) * 32;
+    }
+  }
   calls_ = 0;
   pushes_ = 0;
   mm_arrivals_ = 0;
 }
 
+bool FusedEngine::may_keep(const GemmOperands& g, FusedParams& p) const {
+  // (the traces record the phases of the staged form)
+  if (p.phase_trace != nullptr || p.row_trace != nullptr) return false;
+  if (static_cast<long long>(g.M) * g.N > ws_.keep_elems) return false;
+  p.readers = static_cast<uint32_t*>(heap_.local(ws_.exchange));
+  p.exchange = p.readers + kMaxTileRows;
+  return true;
+}
+
 void FusedEngine::attach_symmetric(size_t bytes, const std::vector<void*>& peer_ptrs, void* mc_ptr) {
   if (!initialized()) throw std::runtime_error("attach_symmetric: engine not initialised");
+  if (bytes < workspace_bytes(1)) throw std::runtime_error("attach_symmetric: buffer too small");
   if (heap_.valid()) {
     check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     heap_.destroy();
   }
+  ws_ = Workspace{};
   heap_.attach(rank_, world_, bytes, peer_ptrs, mc_ptr);
   check(cudaMemset(heap_.local(0), 0, bytes), "cudaMemset(symmetric memory)");
   check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
@@ -133,9 +144,7 @@ void FusedEngine::attach_symmetric(size_t bytes, const std::vector<void*>& peer_
     all_gather_(&t, 1, all.data());
   }
   // the largest problem the attached memory can hold
-  long long elems = static_cast<long long>((bytes - workspace_bytes(0)) / 8);
-  if (elems < 1) throw std::runtime_error("attach_symmetric: buffer too small");
-  carve_workspace(elems);
+  carve_workspace(static_cast<long long>((bytes - workspace_bytes(0)) / 8));
 }
 
 void FusedEngine::detach_symmetric() {
@@ -165,8 +174,11 @@ void FusedEngine::ensure_workspace(long long m, long long n) {
       all_gather_(&t, 1, all.data());
     }
     heap_.destroy();
+    ws_ = Workspace{};
   }
-  heap_.init(rank_, world_, workspace_bytes(elems), all_gather_);
+  // (several ranks keep nothing on the chip between a product and its RMSNorm)
+  const size_t exchange = world_ == 1 ? exchange_words(elems) * 4 : 0;
+  heap_.init(rank_, world_, workspace_bytes(elems) + exchange, all_gather_);
   carve_workspace(elems);
 }
 
@@ -359,10 +371,7 @@ void* FusedEngine::gemm_allreduce(const GemmOperands& g_in, void* out_user, cons
     p.drop_stage = drop_stage(g) ? 1 : 0;
     g.any_tile = tile_is_free() ? 1 : 0;
     g.normed = 1;
-    // (the traces record the phases of the staged form)
-    g.may_keep = p.phase_trace == nullptr && p.row_trace == nullptr ? 1 : 0;
-    p.readers = exchange_;
-    p.exchange = exchange_ + kMaxTileRows;
+    g.may_keep = may_keep(g, p) ? 1 : 0;
   }
   // with one rank there is nobody to deliver to: rows go to the result buffer like a reduce-scatter's
   p.bcast = world_ > 1 ? 1 : 0;
@@ -447,10 +456,7 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
     p.drop_stage = drop_stage(g) ? 1 : 0;
     g.any_tile = tile_is_free() ? 1 : 0;
     g.normed = 1;
-    // (the traces record the phases of the staged form)
-    g.may_keep = p.phase_trace == nullptr && p.row_trace == nullptr ? 1 : 0;
-    p.readers = exchange_;
-    p.exchange = exchange_ + kMaxTileRows;
+    g.may_keep = may_keep(g, p) ? 1 : 0;
   }
   p.bcast = 0;
   p.job_counter = flag_ptr(rank_, set) + kFlagJob;
@@ -747,7 +753,9 @@ void FusedEngine::reset_counters() {
   if (heap_.valid()) {
     for (int s = 0; s < 2; ++s) check(cudaMemset(flag_ptr(rank_, s), 0, kFlagWords * 4), "cudaMemset(counters)");
     check(cudaMemset(heap_.local(ws_.misc), 0, 4096), "cudaMemset(counters)");
-    if (exchange_ != nullptr) check(cudaMemset(exchange_, 0, exchange_bytes_), "cudaMemset(row statistics)");
+    if (ws_.keep_elems > 0) {
+      check(cudaMemset(heap_.local(ws_.exchange), 0, exchange_words(ws_.keep_elems) * 4), "cudaMemset(row statistics)");
+    }
     check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
   }
   if (world_ > 1 && all_gather_) {

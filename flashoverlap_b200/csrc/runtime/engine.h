@@ -201,6 +201,8 @@ class FusedEngine {
     size_t flags[2] = {0, 0};  // kMaxTileRows arrival counters + 1 delivery counter each
     size_t misc = 0;           // counters that the per-call clearing must not touch
     size_t local_flags = 0;    // arrival counters of single-GPU operations (never written by peers)
+    size_t exchange = 0;       // one rank: row statistics of a resident RMSNorm (FusedParams::readers, then ::exchange)
+    long long keep_elems = 0;  // values of the largest product that has room there
     long long capacity_elems = 0;
   };
   void base_params(FusedParams& p, const SignalArgs* sig);
@@ -214,10 +216,6 @@ class FusedEngine {
   AllGatherFn all_gather_;
   SymmHeap heap_;
   Workspace ws_;
-  // One rank: row statistics of a resident RMSNorm (FusedParams::readers, then FusedParams::exchange), as large as the
-  // workspace asks for and allocated with it.
-  uint32_t* exchange_ = nullptr;
-  size_t exchange_bytes_ = 0;
   StatusWord* status_dev_ = nullptr;
   StatusWord* status_host_ = nullptr;    // mirror of the status word in mapped host memory (host address)
   StatusWord* status_mirror_ = nullptr;  // the same memory as the device sees it
@@ -235,6 +233,8 @@ class FusedEngine {
   int nvls_auto_min_world_ = 0;
   int nvls_rs_ = -1;
   void carve_workspace(long long elems);
+  // May this product stay on the chip between the GEMM and its RMSNorm?  Points `p` to the exchange if so.
+  bool may_keep(const GemmOperands& g, FusedParams& p) const;
   static constexpr size_t kNoMulticast = ~size_t(0);
   void gathered_gemm(const void* const* src_for, const long long* bytes_for, const int* src_end, int M, int first_row,
                      const void* B, void* C, int N, int K, DType dtype, int algo, const char* op, cudaStream_t stream,

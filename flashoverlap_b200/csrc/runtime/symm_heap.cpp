@@ -11,7 +11,9 @@ std::string cuda_error_string(cudaError_t e, const char* what) {
 }
 
 static void check(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) throw std::runtime_error(cuda_error_string(e, what));
+  if (e == cudaSuccess) return;
+  cudaGetLastError();  // reported here: the next launch check must not find it again
+  throw std::runtime_error(cuda_error_string(e, what));
 }
 
 SymmHeap::~SymmHeap() {
@@ -30,7 +32,9 @@ void SymmHeap::init(int rank, int world, size_t bytes, const AllGatherFn& all_ga
   world_ = world;
   bytes_ = bytes;
   top_ = 0;
-  check(cudaMalloc(&base_, bytes), "cudaMalloc(symmetric slab)");
+  const cudaError_t e = cudaMalloc(&base_, bytes);
+  if (e != cudaSuccess) base_ = nullptr;
+  check(e, "cudaMalloc(symmetric slab)");
   check(cudaMemset(base_, 0, bytes), "cudaMemset(symmetric slab)");
   check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
   peer_base_.assign(world, nullptr);

@@ -764,6 +764,77 @@ def test_resident_norm_in_a_graph():
         assert ((E.double() - y).abs() <= 2 ** -10.9 * y.abs() + 1e-5).all()
 
 
+def norm_oracle(A, B, W):
+    y = A.double() @ B.double().t()
+    return y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * W.double()
+
+
+def small_resident_call(impl):
+    M, N, K = 128, 8192, 1024
+    assert torch.ops.flashoverlap_op.planned_tile(M, N, K, 7, 0, False, True)[2] == 1
+    A, B, W = make_inputs(M, N, K, torch.float16)
+    out = impl.gemm_allreduce_fused(A, B, W, 1e-5, 7)
+    torch.cuda.synchronize()
+    impl.check_status()
+    want = norm_oracle(A, B, W)
+    assert ((out.double() - want).abs() <= 2 ** -9.3 * want.abs() + 1e-4).all()   # three roundings to 11 bits
+
+
+def test_resident_norm_while_the_workspace_grows():
+    # the exchange of row statistics is part of the workspace: it moves with it and starts clean
+    impl = make_impl()
+    small_resident_call(impl)
+    for M, N, K in [(384, 4544, 200), (2048, 4096, 2048), (256, 1024, 264), (4096, 8192, 1024)]:
+        A, B, W = make_inputs(M, N, K, torch.float16, seed=M)
+        D = torch.empty(M, N, device="cuda", dtype=torch.float16)
+        impl.gemm_reducescatter_fused(A, B, D, W, 1e-5, 2, False)
+        torch.cuda.synchronize()
+        want = norm_oracle(A, B, W)
+        assert ((D.double() - want).abs() <= 2 ** -9.3 * want.abs() + 1e-4).all()
+        small_resident_call(impl)
+
+
+def test_workspace_that_cannot_grow_or_be_attached():
+    # an allocation that fails leaves an engine that works: room for the four buffers of a 16384 x 16384 problem, but for
+    # little more; then memory that is refused because it is too small
+    impl = make_impl()
+    small_resident_call(impl)
+    M = N = 16384
+    A, B, W = make_inputs(M, N, 8, torch.float16)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    spare = 8 * M * N + (16 << 20)
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - spare, dtype=torch.uint8, device="cuda")
+    with pytest.raises(RuntimeError, match="cudaMalloc"):
+        impl.gemm_allreduce_fused(A, B, W, 1e-5, 8)
+    del hold
+    torch.cuda.empty_cache()
+    small_resident_call(impl)
+    tiny = torch.empty(1 << 18, dtype=torch.uint8, device="cuda")
+    with pytest.raises(RuntimeError, match="too small"):
+        impl.attach_symmetric([tiny.data_ptr()], 0, tiny.numel())
+    small_resident_call(impl)
+
+
+def test_resident_norm_in_attached_memory():
+    # as large as the two products that the workspace is asked for: every call is accepted, also where the exchange has no room
+    M, N, K = 4096, 8192, 256
+    impl = make_impl()
+    buf = torch.empty(8 * M * N + (4 << 20), dtype=torch.uint8, device="cuda")
+    base = (buf.data_ptr() + 1023) // 1024 * 1024
+    impl.attach_symmetric([base], 0, buf.numel() - 1024)
+    A, B, W = make_inputs(M, N, K, torch.float16)
+    for _ in range(2):
+        out = impl.gemm_allreduce_fused(A, B, W, 1e-5, 8)
+        torch.cuda.synchronize()
+        impl.check_status()
+        want = norm_oracle(A, B, W)
+        assert ((out.double() - want).abs() <= 2 ** -9.3 * want.abs() + 1e-4).all()
+        small_resident_call(impl)
+    impl.detach_symmetric()
+    small_resident_call(impl)
+
+
 def test_wrappers_that_make_their_result_natively():
     # the same bits as the forms that write into a given tensor, rows of any count, and the same refusals
     M, N, K, algo = 300, 512, 136, 8
