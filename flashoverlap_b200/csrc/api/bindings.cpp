@@ -150,6 +150,7 @@ static std::vector<int64_t> tile_walk_op(int64_t TM, int64_t TN, int64_t raster_
 
 // The tile configuration that a one-rank GEMM which names `algo` runs on `ctas` CTAs (0 = all SMs of the device).  For
 // tests and for reasoning about a call's time; needs no GPU when `ctas` is given.
+constexpr int kB200Sms = 148;
 static LaunchPlan plan_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu, bool norm) {
   TORCH_CHECK(M > 0 && N > 0 && K > 0 && algo >= 0 && algo < kNumAlgos && ctas >= 0, "planned_algo: bad arguments");
   GemmOperands g{};
@@ -161,7 +162,9 @@ static LaunchPlan plan_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t
   g.may_keep = norm ? 1 : 0;
   g.normed = g.may_keep;
   g.glu = glu ? 1 : 0;
-  return plan_launch(g, ctas > 0 ? static_cast<int>(ctas) : device_sm_count());
+  const int sms = device_sm_count();
+  const int whole = sms > 0 ? sms : kB200Sms;  // (without a GPU: those of a B200)
+  return plan_launch(g, ctas > 0 ? static_cast<int>(ctas) : sms, ctas == 0 || ctas >= whole);
 }
 static int64_t planned_algo_op(int64_t M, int64_t N, int64_t K, int64_t algo, int64_t ctas, bool glu) {
   return plan_op(M, N, K, algo, ctas, glu, false).algo;

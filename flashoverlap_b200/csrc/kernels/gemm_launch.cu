@@ -233,7 +233,7 @@ double resident_ns(const GemmOperands& g, const TileConfig& tc, int bn, int tn, 
 // multiply-adds on (some 220 us) every form runs at the power cap, and the staged one, whose tiles have the full width, comes
 // out the same or better: 4096 x 8192 x 8192 464 against 474, 8192 x 8192 x 28672 bf16 2950 against 3098.
 // Among forms within the fit's error the configuration of a call without RMSNorm is kept.
-static LaunchPlan find_plan(const GemmOperands& g, int ctas) {
+static LaunchPlan find_plan(const GemmOperands& g, int ctas, bool whole_chip) {
   LaunchPlan plan{plan_algo(g, ctas), 0, 0, 1, 0};
   plan.bn = kAlgoTable[plan.algo].bn;
   if (!g.any_tile) return plan;
@@ -266,6 +266,8 @@ static LaunchPlan find_plan(const GemmOperands& g, int ctas) {
   // where it is expected to save 3 % (27 % of them; 1.56 times where K is split), nowhere slower by more than 3 %:
   // 256 x 1664 x 11904 53.3 -> 26.8 us, 9344 x 7040 x 17784 2351 -> 2130.  Not for calls of less than 14 us, which is what
   // the host takes for two launches and the way to them.
+  // Not for calls that leave SMs to other streams either: the RMSNorm kernel takes every SM.
+  if (!whole_chip) return plan;
   const LaunchPlan two = plan_plain(g, plain, ctas);
   const double two_ns = plain_ns(g, two.algo, two.bn, two.split, ctas) + 2280 + 0.76e-3 * g.M * static_cast<double>(g.N);
   if (two_ns < 0.97 * expected && two_ns >= 14000) {
@@ -276,18 +278,18 @@ static LaunchPlan find_plan(const GemmOperands& g, int ctas) {
 }
 
 // Comparing the forms takes some 3 us of host time, as long as a launch: each thread remembers the plans of its last shapes.
-LaunchPlan plan_launch(const GemmOperands& g, int ctas) {
+LaunchPlan plan_launch(const GemmOperands& g, int ctas, bool whole_chip) {
   struct Entry {
     int key[6];
     LaunchPlan plan;
   };
   static thread_local Entry seen[64] = {};
-  if (!g.any_tile) return find_plan(g, ctas);
-  const int key[6] = {g.M, g.N, g.K, g.algo, ctas, g.glu | g.normed << 1 | g.may_keep << 2};
+  if (!g.any_tile) return find_plan(g, ctas, whole_chip);
+  const int key[6] = {g.M, g.N, g.K, g.algo, ctas, g.glu | g.normed << 1 | g.may_keep << 2 | (whole_chip ? 8 : 0)};
   const uint32_t slot = (static_cast<uint32_t>(g.M / 32) * 31u + static_cast<uint32_t>(g.N / 32)) * 31u + static_cast<uint32_t>(g.K / 8) * 7u + key[5];
   Entry& e = seen[slot % 64];
   if (!std::equal(key, key + 6, e.key)) {  // (no shape has M = 0)
-    e.plan = find_plan(g, ctas);
+    e.plan = find_plan(g, ctas, whole_chip);
     std::copy(key, key + 6, e.key);
   }
   return e.plan;
@@ -324,7 +326,7 @@ cudaError_t launch_fused(const GemmOperands& g, FusedParams& p, cudaStream_t str
   int grid = g.sm_count > 0 ? g.sm_count : device_sm_count();
   const int sms = device_sm_count();
   if (grid > sms) grid = sms;  // every CTA must be resident: CTAs wait on one another's output
-  const LaunchPlan plan = plan_launch(g, grid);
+  const LaunchPlan plan = plan_launch(g, grid, grid == sms);
   const int algo = plan.algo;
   p.algo = algo;
   p.bn = plan.bn;

@@ -52,8 +52,9 @@ struct GemmOperands {
 struct LaunchPlan {
   int algo, bn, rows, split, norm_after;
 };
-// The plan with which a GEMM on `ctas` CTAs is expected to take least time.
-LaunchPlan plan_launch(const GemmOperands& g, int ctas);
+// The plan with which a GEMM on `ctas` CTAs is expected to take least time.  `whole_chip`: those are all SMs of the device,
+// so that a kernel behind the GEMM may take them as well.
+LaunchPlan plan_launch(const GemmOperands& g, int ctas, bool whole_chip);
 
 // Fills p.tmA / p.tmB / shape fields from `g`, validates shapes, launches.
 // Everything else in `p` must already be set by the caller; p.algo says

@@ -97,6 +97,15 @@ def test_resident_plans_fit_the_chip():
     assert seen > 100
 
 
+def test_rmsnorm_kernel_behind_the_gemm_only_on_the_whole_chip():
+    # a call that leaves SMs to other streams stays one kernel on the SMs it may use
+    plan = torch.ops.flashoverlap_op.planned_tile
+    for m, n, k, algo in [(256, 1664, 11904, 1), (128, 1024, 28672, 2), (384, 1280, 22256, 2), (2176, 4096, 4096, 0)]:
+        assert plan(m, n, k, algo, 148, False, True)[4] == 1
+        for ctas in (1, 2, 37, 100, 146, 147):
+            assert list(plan(m, n, k, algo, ctas, False, True))[3:] == [1, 0]     # K in one piece, no second kernel
+
+
 def test_plain_plans_fit_the_chip():
     # widths of whole chunks inside their configuration; a split over single CTAs that all run together, each with K to work
     # on; of the gated form two halves of whole chunks

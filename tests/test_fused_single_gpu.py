@@ -764,6 +764,24 @@ def test_resident_norm_in_a_graph():
         assert ((E.double() - y).abs() <= 2 ** -10.9 * y.abs() + 1e-5).all()
 
 
+@pytest.mark.parametrize("M,N,K,algo", [(256, 1664, 11904, 1), (2176, 4096, 4096, 0)])
+@pytest.mark.parametrize("sms", [2, 37, 100])
+def test_norm_on_some_of_the_sms(M, N, K, algo, sms):
+    # shapes whose RMSNorm is a kernel behind the GEMM on the whole chip: on some of its SMs they stay one kernel
+    plan = torch.ops.flashoverlap_op.planned_tile
+    assert plan(M, N, K, algo, 0, False, True)[4] == 1 and plan(M, N, K, algo, sms, False, True)[4] == 0
+    A, B, W = make_inputs(M, N, K, torch.bfloat16, seed=N)
+    impl = make_impl()
+    impl.set_sm_count(sms)
+    want = norm_oracle(A, B, W)
+    for _ in range(2):
+        out = impl.gemm_allreduce_fused(A, B, W, 1e-5, algo)
+        torch.cuda.synchronize()
+        impl.check_status()
+        assert impl.last_algo() == plan(M, N, K, algo, sms, False, True)[0]
+        assert ((out.double() - want).abs() <= 2 ** -6.3 * want.abs() + 1e-4).all()   # three roundings to 8 bits
+
+
 def norm_oracle(A, B, W):
     y = A.double() @ B.double().t()
     return y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * W.double()
