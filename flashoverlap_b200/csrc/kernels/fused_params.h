@@ -206,7 +206,7 @@ struct alignas(64) FusedParams {
   // ---- phase trace ----------------------------------------------------------
   // Optional, kTraceWords x uint64 per CTA, times as %globaltimer nanoseconds:
   // [0] kernel start, [1] end of the GEMM phase, [2] last row reduced by this
-  // CTA, [3] tiles computed, [4] first row reduced by this CTA (0 = none),
+  // CTA, [3] tiles computed (of a split K by its first part), [4] first row reduced by this CTA (0 = none),
   // [5] rows reduced by this CTA, [6] all rows delivered (CTA 0 of an
   // all-reduce only), [7] unused.
   unsigned long long* phase_trace;

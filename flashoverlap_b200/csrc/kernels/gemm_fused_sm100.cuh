@@ -1648,6 +1648,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
         const int n0 = n_blk * p.bn, n1 = min(n0 + p.bn, p.N);
         mine += (n1 + p.trace_cols - 1) / p.trace_cols - (n0 + p.trace_cols - 1) / p.trace_cols;  // tiles that begin here
       }
+      if (part != 0) mine = 0;  // a tile whose K is split counts once
       tr[3] = static_cast<unsigned long long>(mine);
     }
     if (!p.reduce || gave_up) return;

@@ -173,6 +173,25 @@ def test_phase_trace_records_every_row_once():
     assert bool((t[:, 1] >= t[:, 0]).all())   # GEMM phase ends after the start
 
 
+@pytest.mark.parametrize("M,N,K,algo", [(128, 1024, 28672, 2), (256, 1088, 8192, 2), (640, 640, 12296, 1), (2048, 2048, 256, 0)])
+def test_phase_trace_counts_every_tile_once(M, N, K, algo):
+    # tiles of the named configuration, also where the launch splits their K over several CTAs
+    A, B, _ = make_inputs(M, N, K, torch.float16)
+    C = torch.empty(M, N, device="cuda", dtype=torch.float16)
+    split = torch.ops.flashoverlap_op.planned_tile(M, N, K, algo, 0, False, False)[3]
+    assert (split > 1) == (K > 256)
+    impl = make_impl()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    trace = torch.zeros(8 * sms, dtype=torch.int64, device="cuda")
+    impl.set_phase_trace(trace)
+    impl.cutlass_gemm(A, B, C, algo)
+    torch.cuda.synchronize()
+    impl.set_phase_trace(torch.empty(0, dtype=torch.int64, device="cuda"))
+    t = trace.view(sms, 8).cpu()
+    assert int(t[:, 3].sum()) == (M // 128) * (N // ALGO_TILES[algo][1])     # pairs count 128 rows each
+    assert bool((t[:, 1] >= t[:, 0]).all())
+
+
 def test_row_trace_has_ordered_stamps_for_every_row():
     M, N, K = 1024, 2048, 256
     A, B, W = make_inputs(M, N, K, torch.float16, seed=5)
