@@ -10,8 +10,6 @@
 
 namespace fo {
 
-// Launches one CTA per requested SM (a cluster of two for CTA pairs), as a
-// cooperative launch when cooperative_launch_enabled().
 // Raises the kernel's dynamic shared-memory limit on the current device (once
 // per device and instance; a device index beyond the cache is set every time).
 template <int BN, int BK, bool BF16, int CTAS>
@@ -30,6 +28,9 @@ cudaError_t prepare_instance() {
   return cudaSuccess;
 }
 
+// Launches one CTA per requested SM (a cluster of two for CTA pairs, of p.split
+// CTAs for a split K), as a cooperative launch when cooperative_launch_enabled()
+// and CTAs of different clusters wait for one another.
 template <int BN, int BK, bool BF16, int CTAS>
 cudaError_t launch_instance(const FusedParams& p, int grid, cudaStream_t stream) {
   using T = TileTraits<BN, CTAS, BK>;
@@ -50,7 +51,9 @@ cudaError_t launch_instance(const FusedParams& p, int grid, cudaStream_t stream)
     attr[n].val.clusterDim.z = 1;
     ++n;
   }
-  if (cooperative_launch_enabled()) {
+  // The clusters of a split K wait for nobody outside themselves: they need not all be resident, and a chip on which fewer of
+  // them fit together than planned takes them one after the other.
+  if (cooperative_launch_enabled() && p.split == 1) {
     attr[n].id = cudaLaunchAttributeCooperative;
     attr[n].val.cooperative = 1;
     ++n;

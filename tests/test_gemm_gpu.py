@@ -1,4 +1,8 @@
 """Numerics of the sm_100a GEMM kernel against a plain PyTorch fp32 reference."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -210,3 +214,39 @@ def test_gemm_in_tiles_of_any_width_and_split(dtype, M, N, K, algo):
     over.check_status()
     from flashoverlap_b200.utils.reorder import from_tile_order
     assert torch.equal(from_tile_order(T, *ALGO_TILES[algo][:2], RA), first)
+
+
+COOPERATIVE = """
+import torch
+import flashoverlap_b200
+impl = torch.classes.flashoverlap_class.OverlapImpl()
+impl.nccl_init(0, 1, [0] * 16)
+impl.cutlass_init()
+impl.set_timeout_ms(2000)
+plan = torch.ops.flashoverlap_op.planned_tile
+for M, N, K, algo, norm in [(128, 1024, 28672, 2, False), (640, 640, 12296, 1, False), (128, 8192, 1024, 7, True),
+                            (256, 1664, 11904, 1, True), (2048, 2048, 256, 0, False)]:
+    A = torch.randn(M, K, device="cuda", dtype=torch.float16)
+    B = (torch.randn(N, K, device="cuda") / K ** 0.5).half()
+    want = A.double() @ B.double().t()
+    if norm:
+        C = impl.gemm_allreduce_fused(A, B, torch.ones(N, device="cuda", dtype=torch.float16), 1e-5, algo)
+        want = want * torch.rsqrt(want.pow(2).mean(-1, keepdim=True) + 1e-5)
+    else:
+        C = torch.empty(M, N, device="cuda", dtype=torch.float16)
+        impl.cutlass_gemm(A, B, C, algo)
+    torch.cuda.synchronize()
+    impl.check_status()
+    # two roundings to 11 bits of fp32 sums over K
+    assert ((C.double() - want).abs() <= 2 ** -9.9 * want.abs() + 1e-3).all(), (M, N, K)
+    print("split", plan(M, N, K, algo, 0, False, norm)[3])
+"""
+
+
+def test_calls_with_the_cooperative_attribute():
+    # every form of a launch, K split and not, where launches ask the driver for the residency of all CTAs
+    env = dict(os.environ, FLASHOVERLAP_COOPERATIVE="1")
+    res = subprocess.run([sys.executable, "-c", COOPERATIVE], env=env, capture_output=True, text=True, timeout=240,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert res.returncode == 0, res.stderr[-2000:]
+    assert "split 8" in res.stdout and "split 1" in res.stdout
