@@ -408,8 +408,15 @@ void FusedEngine::gemm_reducescatter(const GemmOperands& g_in, void* D, bool int
   const int set = static_cast<int>(calls_ & 1ull);
   uint32_t* const clear_words = clear_next_set(set, stream);
   if (world_ == 1 && norm.gamma == nullptr) {
-    gemm(g, D, out_layout, sig, stream, clear_words);  // one rank, no RMSNorm: the GEMM writes the rows where they belong
+    // One rank, no RMSNorm: the GEMM writes the rows where they belong.  A result that takes the place of an operand, which
+    // the GEMM still reads while it stores, goes through the buffer.
+    void* const result = overlaps_operand(g, D) ? heap_.local(ws_.result[set]) : D;
+    gemm(g, result, out_layout, sig, stream, clear_words);
     ++calls_;
+    if (result != D) {
+      check(cudaMemcpyAsync(D, result, static_cast<size_t>(g.M) * g.N * 2, cudaMemcpyDeviceToDevice, stream),
+            "cudaMemcpyAsync(result)");
+    }
     return;
   }
 

@@ -783,6 +783,26 @@ def test_resident_norm_in_a_graph():
         assert ((E.double() - y).abs() <= 2 ** -10.9 * y.abs() + 1e-5).all()
 
 
+@pytest.mark.parametrize("operand", ["A", "B"])
+@pytest.mark.parametrize("norm", [False, True])
+def test_reducescatter_into_an_operand(operand, norm):
+    # a result that takes the place of the rows (or, without RMSNorm, of the weights) that the GEMM reads while it stores tiles
+    if norm and operand == "B":
+        pytest.skip("rows are delivered while others are computed")
+    M = N = K = 2048
+    A, B, W = make_inputs(M, N, K, torch.float16)
+    impl = make_impl()
+    want = torch.empty(M, N, device="cuda", dtype=torch.float16)
+    weight = W if norm else None
+    impl.gemm_reducescatter_fused(A, B, want, weight, 1e-5, 3, False)
+    X, Y = A.clone(), B.clone()
+    D = X if operand == "A" else Y
+    impl.gemm_reducescatter_fused(X, Y, D, weight, 1e-5, 3, False)
+    torch.cuda.synchronize()
+    impl.check_status()
+    assert torch.equal(D, want)
+
+
 @pytest.mark.parametrize("M,N,K,algo", [(256, 1664, 11904, 1), (2176, 4096, 4096, 0)])
 @pytest.mark.parametrize("sms", [2, 37, 100])
 def test_norm_on_some_of_the_sms(M, N, K, algo, sms):
