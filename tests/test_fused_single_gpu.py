@@ -803,6 +803,36 @@ def test_reducescatter_into_an_operand(operand, norm):
     assert torch.equal(D, want)
 
 
+def test_resident_norm_of_rows_that_are_not_finite():
+    # a sum of squares that is infinite or not a number passes the exchange like any other, and stays in its row; the next call
+    # finds the exchange clean
+    M, N, K = 384, 4544, 200
+    assert torch.ops.flashoverlap_op.planned_tile(M, N, K, 2, 0, False, True)[2] > 0
+    A, B, W = make_inputs(M, N, K, torch.float16)
+    impl = make_impl()
+    clean = impl.gemm_allreduce_fused(A, B, W, 1e-5, 2).clone()
+    bad = {5: float("nan"), 130: float("inf"), 383: float("-inf"), 200: 60000.0, 201: 0.0}
+    A2 = A.clone()
+    for row, value in bad.items():
+        A2[row] = value
+    got = impl.gemm_allreduce_fused(A2, B, W, 1e-5, 2).clone()
+    again = impl.gemm_allreduce_fused(A, B, W, 1e-5, 2).clone()
+    torch.cuda.synchronize()
+    impl.check_status()
+    y = (A2.float() @ B.float().t()).half().float()       # as the 16-bit product holds it
+    want = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * W.float()
+    rest = torch.ones(M, dtype=torch.bool, device="cuda")
+    rest[list(bad)] = False
+    assert torch.equal(got[rest], clean[rest]) and torch.equal(again, clean)
+    assert bool(got[5].isnan().all()) and bool((got[201] == 0).all())
+    for row in (130, 200, 383):
+        # infinities of the product times a scale of zero, zeros (or a finite row's values) elsewhere
+        assert torch.equal(got[row].isnan(), want[row].isnan()), row
+        fine = ~want[row].isnan()
+        # a value of the product may round the other way (one unit of 11 bits), then two roundings
+        assert ((got[row][fine].float() - want[row][fine]).abs() <= 2 ** -9 * want[row][fine].abs() + 1e-4).all()
+
+
 @pytest.mark.parametrize("M,N,K,algo", [(256, 1664, 11904, 1), (2176, 4096, 4096, 0)])
 @pytest.mark.parametrize("sms", [2, 37, 100])
 def test_norm_on_some_of_the_sms(M, N, K, algo, sms):

@@ -110,12 +110,14 @@ def test_algo_table_matches_generated_python_copy():
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("algo,M,ffn", [(8, 256, 128), (3, 512, 1920), (9, 768, 64), (4, 256, 14336 // 8), (4, 256, 4800)])
+@pytest.mark.parametrize("algo,M,ffn", [(8, 256, 128), (3, 512, 1920), (9, 768, 64), (4, 256, 14336 // 8), (4, 256, 4800),
+                                        (4, 256, 4864)])
 @pytest.mark.parametrize("K", [8, 328])
 @pytest.mark.parametrize("keep", [True, False])
 def test_gemm_swiglu(dtype, algo, M, ffn, K, keep):
     # gate and up columns of one tile in the two CTAs of a pair, for each pair of at least 128 columns: one tile, many,
-    # the narrowest; in the tile that the launch chooses also a last tile that is half full (4800 of 38 x 128)
+    # the narrowest; in the tile that the launch chooses also a last tile that is partly full (64 columns of 96, the last of
+    # 4864)
     torch.manual_seed(ffn)
     impl = torch.classes.flashoverlap_class.OverlapImpl()
     impl.cutlass_init()
@@ -126,7 +128,9 @@ def test_gemm_swiglu(dtype, algo, M, ffn, K, keep):
     impl.gemm_swiglu(x, w, guard[:M], algo)
     torch.cuda.synchronize()
     assert impl.last_algo() == (algo if keep else torch.ops.flashoverlap_op.planned_algo(M, 2 * ffn, K, algo, 0, True))
-    assert (ffn, K) != (4800, 328) or keep or ALGO_TILES[impl.last_algo()][:2] == (256, 256)
+    if (ffn, K, keep) == (4864, 328, False):
+        half = torch.ops.flashoverlap_op.planned_tile(M, 2 * ffn, K, algo, 0, True, False)[1] // 2
+        assert ffn % half == 64 and half > 64
     gate, up = (x.double() @ w.double().t()).chunk(2, dim=-1)
     want = torch.nn.functional.silu(gate) * up
     # one rounding of the result (11 or 8 bits) on fp32 sums
@@ -214,6 +218,31 @@ def test_gemm_in_tiles_of_any_width_and_split(dtype, M, N, K, algo):
     over.check_status()
     from flashoverlap_b200.utils.reorder import from_tile_order
     assert torch.equal(from_tile_order(T, *ALGO_TILES[algo][:2], RA), first)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,N,K,algo", [(130, 1024, 4096, 1), (200, 2048, 4096, 2), (3, 1024, 28672, 2), (257, 1088, 8192, 2)])
+def test_dispatch_of_ragged_rows_with_a_split_k(dtype, rows, N, K, algo):
+    # rows that do not fill their tiles, few enough for the K of a tile to be split: the missing rows read as zero in every part
+    impl = torch.classes.flashoverlap_class.OverlapImpl()
+    impl.nccl_init(0, 1, [0] * 16)
+    impl.cutlass_init()
+    impl.set_timeout_ms(2000)
+    mlen = torch.tensor([[rows]], dtype=torch.int32)
+    padded = impl.a2a_padded_rows(mlen, algo)
+    assert padded > rows and torch.ops.flashoverlap_op.planned_tile(padded, N, K, algo, 0, False, False)[3] > 1
+    torch.manual_seed(rows)
+    A = torch.randn(rows + 1, K, device="cuda").to(dtype)      # one row more than is sent
+    B = (torch.randn(N, K, device="cuda") / K ** 0.5).to(dtype)
+    buf = torch.full((padded + 1, N), 5.0, device="cuda", dtype=dtype)
+    impl.a2a_dispatch_gemm(A, B, buf[:padded], mlen, algo)
+    torch.cuda.synchronize()
+    impl.check_status()
+    want = A[:rows].double() @ B.double().t()
+    # one rounding of fp32 sums
+    bits = 10.9 if dtype == torch.float16 else 7.9
+    assert ((buf[:rows].double() - want).abs() <= 2 ** -bits * want.abs() + 4e-6 * K ** 0.5).all()
+    assert bool((buf[padded:] == 5).all())
 
 
 COOPERATIVE = """
