@@ -4,7 +4,8 @@ The package offers the capabilities of FlashOverlap (fused GEMM+AllReduce /
 GEMM+ReduceScatter with tile-order-aware RMSNorm, a non-overlapped baseline,
 a wave-group tuner and its config files) on a different engine: every
 overlapped operation is one persistent tcgen05/TMEM kernel that pushes
-finished tiles to peer GPUs over NVLink and reduces them in a trailing phase.
+finished tiles to peer GPUs over NVLink and reduces them while later tiles are
+computed.
 
 Importing the package loads the native library and registers
 ``torch.classes.flashoverlap_class.{OverlapImpl, BaselineImpl}`` and

@@ -749,7 +749,9 @@ struct ResidentScratch {
 // own mark (the sign bit, a sum of squares has none), so that a value is seen as soon as it is written: counted behind a
 // release, with the accumulator read twice, a wave of 256 x 224 tiles took 9.2 us, of which 5.7 were the exchange.
 // A tile waits for tiles of its own wave only, and those for nothing but the epilogue of the wave before: with all CTAs
-// resident (as everywhere in this kernel) nobody waits in a circle.
+// resident (as everywhere in this kernel) nobody waits in a circle.  4096 x 8192 x 1024 fp16: 65 us on a cool chip, 77 after
+// seconds of load (staged: 81 and 88); DRAM takes 26 MB in and 19 MB out while it runs, the tensor pipe is active 56 % of
+// the time.
 template <int BN, int CTAS, bool BF16>
 __device__ __forceinline__ void resident_norm(const FusedParams& p, uint32_t tmem_base, uint64_t* tfull_bar,
                                               uint64_t* tempty_bar, uint32_t tempty_addr0, uint32_t cta_rank, int q, int half,
@@ -1457,8 +1459,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fused_sm100_kernel(const __g
     }
   } else if (warp == 3) {
     // ===================== signalling =====================
-    // One thread per CTA follows the epilogue warps tile by tile: when all four
-    // have stored their slabs it fences at system scope and bumps the arrival
+    // One thread per CTA follows the epilogue warps tile by tile: when all of
+    // them (four, or eight) have stored their part it fences at system scope and bumps the arrival
     // counter of the tile's 128-row block on the GPU(s) that own those rows,
     // and keeps the reference-compatible counters.
     if (p.resident) resident_clear<CTAS>(p, cta_rank, lane, epi_prog, deadline, abort_flag);

@@ -95,7 +95,8 @@ struct TileTime {
 };
 // From single waves (fp16, K from 2048 to 8192, all SMs busy).  A CTA takes in 110 to 125 GB/s of operands, which is what
 // the tiles of up to 128 columns wait for; only the 256-wide ones wait for the tensor cores.  A stage of 64 K-values costs
-// 290 ns at least, one of 128 K-values 430 ns.
+// 290 ns at least, one of 128 K-values 430 ns.  Like the table below taken while four warps stored every tile; what rests on
+// the two is the configuration that plan_plain and find_plan start from and weigh other forms against.
 constexpr TileTime kSingleWave[] = {{6.7, 300, 7000}, {4.6, 300, 7000},  {4.5, 300, 6000}, {6.1, 300, 9500},
                                     {4.7, 300, 8700}, {4.5, 300, 7700},  {4.1, 300, 6300}, {3.4, 300, 5500},
                                     {6.0, 300, 9000}, {3.75, 300, 8300}, {3.4, 300, 7300}};
@@ -120,7 +121,8 @@ double estimate_ns(const TileTime (&times)[kNumAlgos], const GemmOperands& g, in
 // Another tile than the named one runs when it is the fastest by the single waves, clearly, and no slower by the whole
 // calls.  On 700 shapes other than the fitted ones, the tile that runs is more than 3 % slower than the named one in 0.3 %
 // of the calls that name the first of gather_algo_candidates (5.1 % without the second condition) and in 1.4 % (4.1 %) of
-// those that name any other; it is 1.25 times as fast on average over all.
+// those that name any other; it is 1.25 times as fast on average over all (shares and average with the epilogue of that
+// time, four warps).
 static int plan_algo(const GemmOperands& g, int ctas) {
   if (!g.any_tile) return g.algo;
   int best = g.algo;
@@ -136,7 +138,8 @@ static int plan_algo(const GemmOperands& g, int ctas) {
 }
 
 namespace {
-// Clusters of so many CTAs that fit the chip together (148 SMs in groups of unequal size); the launch asks for no more.
+// Clusters of so many CTAs that fit the chip together (148 SMs in groups of unequal size); the plan asks for no more.  Counted
+// on one B200: where fewer fit, the others run in a second round.
 constexpr int kMaxSplit = 8;
 constexpr int kClusters[kMaxSplit + 1] = {0, 148, 73, 44, 32, 25, 21, 14, 14};
 
@@ -162,9 +165,9 @@ double plain_ns(const GemmOperands& g, int algo, int bn, int split, int ctas) {
 // The plan of a plain GEMM: the configuration that plan_algo finds, in the width that suits the wave, or another one where
 // that is clearly better.  Short K gives little to go by (rounds of the epilogue and of HBM writes), and a split pays where
 // the tiles leave SMs without work.  Over the fitted shapes 1.11 times as fast as plan_algo's tile alone (1.15 with the best
-// choice each time), slower by more than 3 % in 0.2 %.  1152 x 5120 x 1720 bf16 38 -> 28 us (256 x 192), 128 x 10240 x 8192
-// bf16 42 -> 37 (three CTAs per 128 x 256 tile), 128 x 1024 x 28672 113 -> 29 (eight per 128 x 128), 2048 x 8192 x 1024 38.7
-// -> 35.
+// choice each time), slower by more than 3 % in 0.2 %.  Against plan_algo's tile with the epilogue of four warps, two
+// libraries in turn: 1152 x 5120 x 1720 bf16 38.4 -> 26.5 us (256 x 192), 128 x 10240 x 8192 bf16 42.2 -> 37.6 (two CTAs per
+// 128 x 160 tile), 128 x 1024 x 28672 bf16 98 -> 27 (eight per 128 x 96), 2048 x 8192 x 1024 fp16 31.9 -> 30.7 (256 x 224).
 LaunchPlan plan_plain(const GemmOperands& g, int base, int ctas) {
   LaunchPlan plan{base, kAlgoTable[base].bn, 0, 1, 0};
   const TileConfig& named = kAlgoTable[base];
@@ -228,8 +231,9 @@ double resident_ns(const GemmOperands& g, const TileConfig& tc, int bn, int tn, 
 
 // A resident RMSNorm (see resident_norm) takes as many tile rows per wave as have all their tiles in it.  It runs where it
 // is expected to save 5 %: in 89 % of the fitted shapes, slower than the staged form by more than 3 % in 1.6 % of all, 1.17
-// times as fast over all (1.19 with the best choice each time).  4096 x 8192 x 1024 fp16 88 -> 74 us (one run in turn; the
-// chip warm), 2048 x 4096 x 2048 43.5 -> 35.8, 4096 x 4096 x 512 34.6 -> 28.9, 128 x 8192 x 1024 14.2 -> 12.2.  From 1.5e11
+// times as fast over all (1.19 with the best choice each time).  Against the best tile of the staged form, fp16, in turn on a
+// warm chip: 4096 x 8192 x 1024 83.5 -> 76.8 us, 2048 x 4096 x 2048 40.6 -> 34.2, 4096 x 4096 x 512 35.2 -> 29.1, 128 x 8192
+// x 1024 15.6 -> 12.2.  From 1.5e11
 // multiply-adds on (some 220 us) every form runs at the power cap, and the staged one, whose tiles have the full width, comes
 // out the same or better: 4096 x 8192 x 8192 464 against 474, 8192 x 8192 x 28672 bf16 2950 against 3098.
 // Among forms within the fit's error the configuration of a call without RMSNorm is kept.
@@ -263,9 +267,10 @@ static LaunchPlan find_plan(const GemmOperands& g, int ctas, bool whole_chip) {
   }
   // A plain GEMM, in a tile of any width and with its K split, and an RMSNorm kernel that reads the product from L2: 2.3 us
   // and 0.76 ns per 1000 values more than the GEMM.  Over 800 shapes 1.09 times as fast as the better of the other forms
-  // where it is expected to save 3 % (27 % of them; 1.56 times where K is split), nowhere slower by more than 3 %:
-  // 256 x 1664 x 11904 53.3 -> 26.8 us, 9344 x 7040 x 17784 2351 -> 2130.  Not for calls of less than 14 us, which is what
-  // the host takes for two launches and the way to them.
+  // where it is expected to save 3 % (27 % of them; 1.56 times where K is split), nowhere slower by more than 3 %.  Against
+  // the better of the other forms (the plan on 147 SMs), in turn: 256 x 1664 x 11904 bf16 47.6 -> 24.5 us, 384 x 1280 x 22256
+  // fp16 82 -> 35.5, 128 x 1024 x 28672 bf16 100 -> 27; without a split 2176 x 4096 x 4096 fp16 65 to 81 -> 61 to 65.  Not
+  // for calls of less than 14 us, which is what the host takes for two launches and the way to them.
   // Not for calls that leave SMs to other streams either: the RMSNorm kernel takes every SM.
   if (!whole_chip) return plan;
   const LaunchPlan two = plan_plain(g, plain, ctas);

@@ -125,7 +125,9 @@ __global__ void __launch_bounds__(kMaxNormThreads) rmsnorm_kernel(const uint16_t
     }
     // Up to two chunks (one of a sum, whose two would not fit) stay unpacked between the statistics and the scaling: less
     // follows the barrier, and with these registers no CTA of the next grid finds a place before one of this grid has ended
-    // (with five of them on some SMs the grid ended later).  Launch after launch, fp16: 16384 x 4096 49.0 -> 43.5 us, 2048 x
+    // (with five of them on some SMs the grid ended later).  That takes more than 48 registers a thread with two chunks (55 as
+    // compiled, 58 in tile order; a fifth CTA of 256 threads fits at 48): a build with fewer would be slower, not wrong.
+    // Launch after launch, fp16: 16384 x 4096 49.0 -> 43.5 us, 2048 x
     // 4096 7.5 -> 5.2, 1000 x 1024 2.5 -> 2.1; in tile order 4096 x 9216 39.9 -> 36.7, 2048 x 8192 12.9 -> 12.3.
     constexpr bool UNPACKED = INPUT == NORM_SUM ? CPT == 1 : CPT <= 2;
     float f[UNPACKED ? CPT : 1][8];

@@ -207,10 +207,11 @@ void FusedEngine::base_params(FusedParams& p, const SignalArgs* sig) {
 
 namespace {
 // Tile rows walked together on one GPU.  A group reads every B panel once for all of its rows; rows that are normalised
-// wait for their whole group, so operands that stay in L2 anyway (up to a third of it) take a narrower one.  Groups of 8
-// and 4 in turn, fp16: 2304 x 8192 x 1024 57.9 and 54.4 us, 4096 x 8192 x 1024 93.9 and 91.5, 4096 x 8192 x 1536 118 and
-// 112, 8192 x 8192 x 1024 181 and 177; the other way round at 4096 x 4096 x 2048, 74.0 and 76.2.  With 50 to 101 MB of
-// operands the two differ by 1 % either way (8192 x 8192 x 2048: 276 and 270).
+// wait for their whole group, so operands that stay in L2 anyway (up to a third of it) take a narrower one.  (Rows that stay
+// on the chip walk in groups of one wave.)  Groups of 8 and 4 in turn on a warm chip, calls that stage their product, fp16:
+// 2176 x 9600 x 944 67.6 and 59.1 us, 3328 x 9984 x 384 60.4 and 58.9, 3840 x 10496 x 280 76.7 and 74.3, 6528 x 10752 x 1128
+// 231 and 226, bf16 8704 x 10880 x 272 173 and 167; no difference at 1664 x 9856 x 760 and 2048 x 16384 x 512.  From 46 MB of
+// operands on none either, or the other way round (14080 x 11264 x 1024: 402 and 411).
 int local_group(const GemmOperands& g, bool norm) {
   const double operands = 2.0 * (static_cast<double>(g.M) + g.N) * g.K;
   return norm && operands <= 40e6 ? 4 : 8;
@@ -219,10 +220,11 @@ int local_group(const GemmOperands& g, bool norm) {
 
 namespace {
 // Staged products that crowd the L2 (with the result of the same size) are dropped line by line as they are read.  Of a
-// 4096 x 8192 x 1024 fp16 call 75 MB are written to HBM in place of 133 (67 MB are the product), and 28 read in place of
-// 44: 93.7 -> 91.5 us.  2048 x 8192 x 1024 50.6 -> 49.0, 4096 x 8192 x 512 74.7 -> 71.0; no difference beyond 1 % from K =
-// 1536 on, where the main loop hides the traffic.  Small products only pay for the instruction: 128 x 8192 16.1 -> 16.5,
-// 1024 x 4096 27.7 both ways.
+// 4096 x 8192 x 1024 fp16 call that stages its product 75 MB are written to HBM in place of 133 (67 MB are the product), and
+// 28 read in place of 44.  In turn on a warm chip, fp16: 2176 x 9600 x 944 62.4 -> 59.1 us, 3840 x 10496 x 280 79.2 -> 74.3,
+// 2048 x 16384 x 512 70.8 -> 66.9, 6016 x 10368 x 504 136 -> 134, bf16 8704 x 10880 x 272 170 -> 167.  From K = 1100 on the
+// main loop hides the traffic and the drop costs up to 1.5 % (6528 x 10752 x 1128 223 -> 226, 8448 x 10752 x 1904 372 -> 373),
+// as it does for products just above the line (1664 x 9856 x 760 47.4 -> 48.2).  Small ones only pay for the instruction.
 bool drop_stage(const GemmOperands& g) { return 2.0 * g.M * g.N >= 32e6; }
 }  // namespace
 

@@ -4,8 +4,9 @@
 // buffers for all-reduce, arrival counters), the device status word and the
 // per-call bookkeeping (which of the two staging/counter sets a call uses).
 // It plays the role of the reference's OverlapImpl host code
-// (reference: src/overlap_impl.cu:221-328) but issues exactly one kernel per
-// operation: no second stream, no wait kernels, no NCCL calls.
+// (reference: src/overlap_impl.cu:221-328) but issues one kernel per operation
+// (on one rank with RMSNorm: two where that is faster): no second stream, no
+// wait kernels, no NCCL calls.
 //
 // Why two sets of staging buffers and counters are enough: a rank can finish
 // call i only after every rank has pushed its share of call i, hence after

@@ -98,7 +98,8 @@ class OverlapRowParallelLayer(nn.Module):
 
 
 class FusedRowParallelLinear(nn.Module):
-    """``y = collective(x @ W^T)`` with an optional RMSNorm, as one kernel.
+    """``y = collective(x @ W^T)`` with an optional RMSNorm, as one kernel (on
+    one rank with RMSNorm: two where that is faster).
 
     ``impl`` is an initialised ``OverlapImpl`` (see
     :func:`flashoverlap_b200.parallel.make_overlap_impl`); ``norm_weight`` turns

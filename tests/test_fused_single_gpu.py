@@ -783,12 +783,9 @@ def test_resident_norm_in_a_graph():
         assert ((E.double() - y).abs() <= 2 ** -10.9 * y.abs() + 1e-5).all()
 
 
-@pytest.mark.parametrize("operand", ["A", "B"])
-@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("operand,norm", [("A", False), ("A", True), ("B", False)])
 def test_reducescatter_into_an_operand(operand, norm):
     # a result that takes the place of the rows (or, without RMSNorm, of the weights) that the GEMM reads while it stores tiles
-    if norm and operand == "B":
-        pytest.skip("rows are delivered while others are computed")
     M = N = K = 2048
     A, B, W = make_inputs(M, N, K, torch.float16)
     impl = make_impl()

@@ -2,6 +2,7 @@
 
     python tool/profile_case.py gemm 4096 8192 8192 --algo 3
     python tool/profile_case.py gemm_rmsnorm 4096 8192 1024 --algo 3 --dtype float16
+    python tool/profile_case.py allreduce_norm 4096 8192 1024 --algo 8 --dtype float16   # the product may stay on the chip
     python tool/profile_case.py rmsnorm 4096 8192
 
     ncu --set full --clock-control none -k regex:gemm_fused -s 2 -c 1 -o out python tool/profile_case.py gemm ...
@@ -23,7 +24,7 @@ from flashoverlap_b200.cli import DTYPES  # noqa: E402
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("op", choices=["gemm", "gemm_rmsnorm", "rmsnorm"])
+    ap.add_argument("op", choices=["gemm", "gemm_rmsnorm", "allreduce_norm", "rmsnorm"])
     ap.add_argument("m", type=int)
     ap.add_argument("n", type=int)
     ap.add_argument("k", type=int, nargs="?", default=1024)
@@ -52,6 +53,8 @@ def main():
             impl.cutlass_gemm(A, B, C, args.algo)
         elif args.op == "gemm_rmsnorm":
             impl.gemm_rmsnorm(A, B, C, O, W, 1e-5, args.algo)
+        elif args.op == "allreduce_norm":
+            impl.gemm_allreduce_fused(A, B, W, 1e-5, args.algo)
         else:
             torch.ops.flashoverlap_op.rmsnorm(C, O, W, 1e-5)
     torch.cuda.synchronize()
